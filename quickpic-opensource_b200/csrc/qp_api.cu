@@ -94,6 +94,9 @@ struct qp_species {
   float* q3 = nullptr;         // (nz+1) real planes
   float* q3_first = nullptr;   // slice-1 plane after renew (pristine)
   int regrowths = 0;
+  // q holds the charge of A's particles, as the fused step's slices hand it
+  // on; a class-level call that changes either clears it
+  bool q_live = false;
   PlasmaProfile prof;          // the loader's profile, lengths in cells
 };
 
@@ -392,15 +395,15 @@ static bool parity_of(int dim, int kind, int c, int* px, int* py) {
   return false;
 }
 
-static int fft_rk(qp_ctx* ctx, float* const* rs, float* const* ks, const float* const* add,
-                  int dim, const int* px, const int* py) {
+static int fft_rk(qp_ctx* ctx, float* const* rs, float* const* ks, int dim, const int* px,
+                  const int* py) {
   const GridDims& g = ctx->g;
   XJob xj{};
   YJob yj{};
   xj.ncomp = yj.ncomp = dim;
   const float norm = 0.25f / ((float)g.nx * (float)g.ny);
   for (int c = 0; c < dim; ++c) {
-    xj.c[c] = XComp{rs[c], add ? add[c] : nullptr, ks[c], 1.0f, px[c], 0};
+    xj.c[c] = XComp{rs[c], nullptr, ks[c], 1.0f, px[c], 0};
     yj.c[c] = YComp{ks[c], norm, py[c]};
   }
   launch_xfwd(xj, g, ctx->tx.t, ctx->st, ctx->stream);
@@ -430,7 +433,7 @@ extern "C" int qp_field2d_fftrk(qp_field2d* f, int kind) {
   for (int c = 0; c < f->dim; ++c)
     if (!parity_of(f->dim, kind, c, &px[c], &py[c]))
       return fail(ctx, __LINE__, "fftrk_field2d: wrong fft kind");
-  fft_rk(ctx, f->rs, f->ks, nullptr, f->dim, px, py);
+  fft_rk(ctx, f->rs, f->ks, f->dim, px, py);
   CK(cudaGetLastError());
   f->state = 1;
   return 0;
@@ -499,8 +502,10 @@ static long long plane_n(qp_ctx* ctx, int state) {
 
 extern "C" int qp_field2d_as(qp_field2d* f, float value) {
   qp_ctx* ctx = f->ctx;
+  LinList l(ctx->st, ctx->stream);
   for (int c = 0; c < f->dim; ++c)
-    launch_lin(ctx->g.rplane, f->rs[c], nullptr, nullptr, value, LIN_FILL, ctx->st, ctx->stream);
+    l.add(LIN_FILL, ctx->g.rplane, f->rs[c], nullptr, nullptr, value);
+  l.flush();
   f->state = 0;
   CK(cudaGetLastError());
   return 0;
@@ -509,9 +514,10 @@ extern "C" int qp_field2d_as(qp_field2d* f, float value) {
 extern "C" int qp_field2d_copy(qp_field2d* d, qp_field2d* s) {
   qp_ctx* ctx = d->ctx;
   const int st = s->state;
+  LinList l(ctx->st, ctx->stream);
   for (int c = 0; c < std::min(d->dim, s->dim); ++c)
-    launch_lin(plane_n(ctx, st), planes(d, st)[c], planes(s, st)[c], nullptr, 0.f, LIN_COPY,
-               ctx->st, ctx->stream);
+    l.add(LIN_COPY, plane_n(ctx, st), planes(d, st)[c], planes(s, st)[c]);
+  l.flush();
   d->state = st;
   CK(cudaGetLastError());
   return 0;
@@ -521,9 +527,10 @@ static int binop(qp_field2d* d, qp_field2d* a, qp_field2d* b, int op) {
   qp_ctx* ctx = d->ctx;
   if (a->state != b->state) return fail(ctx, __LINE__, "states are different");
   const int st = a->state;
+  LinList l(ctx->st, ctx->stream);
   for (int c = 0; c < d->dim; ++c)
-    launch_lin(plane_n(ctx, st), planes(d, st)[c], planes(a, st)[c], planes(b, st)[c], 0.f, op,
-               ctx->st, ctx->stream);
+    l.add(op, plane_n(ctx, st), planes(d, st)[c], planes(a, st)[c], planes(b, st)[c]);
+  l.flush();
   d->state = st;
   CK(cudaGetLastError());
   return 0;
@@ -535,9 +542,10 @@ extern "C" int qp_field2d_sub(qp_field2d* d, qp_field2d* a, qp_field2d* b) { ret
 extern "C" int qp_field2d_mult(qp_field2d* d, qp_field2d* a, float value) {
   qp_ctx* ctx = d->ctx;
   const int st = a->state;
+  LinList l(ctx->st, ctx->stream);
   for (int c = 0; c < d->dim; ++c)
-    launch_lin(plane_n(ctx, st), planes(d, st)[c], planes(a, st)[c], nullptr, value, LIN_SCALE,
-               ctx->st, ctx->stream);
+    l.add(LIN_SCALE, plane_n(ctx, st), planes(d, st)[c], planes(a, st)[c], nullptr, value);
+  l.flush();
   d->state = st;
   CK(cudaGetLastError());
   return 0;
@@ -548,13 +556,17 @@ static int binop_comp(qp_field2d* d, qp_field2d* a, qp_field2d* b, const int* di
   qp_ctx* ctx = d->ctx;
   if (a->state != b->state) return fail(ctx, __LINE__, "states are different");
   const int st = a->state;
+  LinList l(ctx->st, ctx->stream);
   for (int i = 0; i < n; ++i) {
     if (dim[i] < 1 || dim[i] > d->dim || dim1[i] < 1 || dim1[i] > a->dim || dim2[i] < 1 ||
-        dim2[i] > b->dim)
+        dim2[i] > b->dim) {
+      l.flush();  // the components before the bad one are done, as one by one
       return fail(ctx, __LINE__, "component index out of range");
-    launch_lin(plane_n(ctx, st), planes(d, st)[dim[i] - 1], planes(a, st)[dim1[i] - 1],
-               planes(b, st)[dim2[i] - 1], 0.f, op, ctx->st, ctx->stream);
+    }
+    l.add(op, plane_n(ctx, st), planes(d, st)[dim[i] - 1], planes(a, st)[dim1[i] - 1],
+          planes(b, st)[dim2[i] - 1]);
   }
+  l.flush();
   d->state = st;
   CK(cudaGetLastError());
   return 0;
@@ -573,16 +585,19 @@ extern "C" int qp_field2d_mult_comp(qp_field2d* d, qp_field2d* a, const int* dim
                                     const float* value, int n) {
   qp_ctx* ctx = d->ctx;
   const int st = a->state;
-  // multiply2 reads a1 and writes this element by element; when this == a1 and
-  // the component lists overlap, compute into scratch first so that every
-  // product uses the input value (the reference's loop order gives the same
-  // result for the lists QuickPIC uses).
+  // multiply2 reads a1 and writes this one component after another, as the
+  // reference's loop does: a component that reads an earlier one's result waits
+  // for it (LinList)
+  LinList l(ctx->st, ctx->stream);
   for (int i = 0; i < n; ++i) {
-    if (dim[i] < 1 || dim[i] > d->dim || dim1[i] < 1 || dim1[i] > a->dim)
+    if (dim[i] < 1 || dim[i] > d->dim || dim1[i] < 1 || dim1[i] > a->dim) {
+      l.flush();  // the components before the bad one are done, as one by one
       return fail(ctx, __LINE__, "component index out of range");
-    launch_lin(plane_n(ctx, st), planes(d, st)[dim[i] - 1], planes(a, st)[dim1[i] - 1], nullptr,
-               value[i], LIN_SCALE, ctx->st, ctx->stream);
+    }
+    l.add(LIN_SCALE, plane_n(ctx, st), planes(d, st)[dim[i] - 1], planes(a, st)[dim1[i] - 1],
+          nullptr, value[i]);
   }
+  l.flush();
   d->state = st;
   CK(cudaGetLastError());
   return 0;
@@ -591,7 +606,7 @@ extern "C" int qp_field2d_mult_comp(qp_field2d* d, qp_field2d* a, const int* dim
 extern "C" int qp_field2d_cg(qp_field2d* f) {
   qp_ctx* ctx = f->ctx;
   if (f->state != 0) return fail(ctx, __LINE__, "copyguard_field2d: data is in ks");
-  for (int c = 0; c < f->dim; ++c) launch_guard_copy(f->rs[c], ctx->g, ctx->st, ctx->stream);
+  launch_guard_copy(f->rs, f->dim, ctx->g, ctx->st, ctx->stream);
   CK(cudaGetLastError());
   return 0;
 }
@@ -599,7 +614,7 @@ extern "C" int qp_field2d_cg(qp_field2d* f) {
 extern "C" int qp_field2d_ag(qp_field2d* f) {
   qp_ctx* ctx = f->ctx;
   if (f->state != 0) return fail(ctx, __LINE__, "acopyguard_field2d: data is in ks");
-  for (int c = 0; c < f->dim; ++c) launch_guard_add(f->rs[c], ctx->g, ctx->st, ctx->stream);
+  launch_guard_add(f->rs, f->dim, ctx->g, ctx->st, ctx->stream);
   CK(cudaGetLastError());
   return 0;
 }
@@ -657,6 +672,23 @@ static int part_copy(qp_ctx* ctx, PartBuf& dst, const PartBuf& src) {
   return 0;
 }
 
+// q_s = the smoothed a + b (b may be null): x pass, smoothing between the y
+// passes, x pass back into the species' real-space charge
+static void smooth_charge(qp_species* sp, const float* a, const float* b) {
+  qp_ctx* ctx = sp->ctx;
+  sp->q_live = false;
+  const GridDims& g = ctx->g;
+  XJob xj{};
+  YJob yj{};
+  xj.ncomp = yj.ncomp = 1;
+  xj.c[0] = XComp{a, b, sp->q->ks[0], 1.0f, 0, 0};
+  yj.c[0] = YComp{sp->q->ks[0], 0.25f / ((float)g.nx * (float)g.ny), 0};
+  launch_xfwd(xj, g, ctx->tx.t, ctx->st, ctx->stream);
+  launch_ysmooth(yj, g, ctx->kc, ctx->ty.t, ctx->st, ctx->stream);
+  xj.c[0] = XComp{sp->q->ks[0], nullptr, sp->q->rs[0], 1.0f, 0, 0};
+  launch_xinv(xj, g, ctx->tx.t, ctx->st, ctx->stream);
+}
+
 // species q / qn / q3 bookkeeping after (re)loading: qn = -(deposit + guard
 // add); q = qn; smoothed q -> q3 slice 1 (species2d_class.f03:104-115).
 static int species_background(qp_species* sp) {
@@ -664,14 +696,8 @@ static int species_background(qp_species* sp) {
   const GridDims& g = ctx->g;
   launch_lin(g.rplane, sp->qn->rs[0], nullptr, nullptr, 0.f, LIN_FILL, ctx->st, ctx->stream);
   launch_deposit_rho(sp->A, ctx->tg, sp->qn->rs[0], ctx->st, ctx->stream);
-  launch_lin(g.rplane, sp->q->rs[0], sp->qn->rs[0], nullptr, 0.f, LIN_COPY, ctx->st, ctx->stream);
   sp->q->state = 0;
-  int px = 0, py = 0;
-  fft_rk(ctx, sp->q->rs, sp->q->ks, nullptr, 1, &px, &py);
-  float* in[8] = {sp->q->ks[0]};
-  float* out[8] = {sp->q->ks[0]};
-  launch_kpoint(KOP_SMOOTH, g, ctx->kc, in, out, 0.f, 1.f, ctx->st, ctx->stream);
-  fft_kr(ctx, sp->q->rs, sp->q->ks, 1, &px, &py);
+  smooth_charge(sp, sp->qn->rs[0], nullptr);
   if (sp->q3)
     CK(cudaMemcpyAsync(sp->q3, sp->q->rs[0], sizeof(float) * g.rplane, cudaMemcpyDeviceToDevice,
                        ctx->stream));
@@ -733,11 +759,8 @@ static int species_renew_device(qp_species* sp, float s) {
   std::string err;
   if (!plasma_qm(sp->prof, s, &qm, &err)) return fail(ctx, __LINE__, "plasma loader: " + err);
   if (sp->A.cap < sp->P0.cap) return fail(ctx, __LINE__, "renew: capacity shrank");
-  const long long n = (long long)tg.ntiles * sp->A.cap;
-  for (int k = 0; k < NCOMP; ++k)
-    launch_lin(n, sp->A.c[k], nullptr, nullptr, 0.f, LIN_FILL, ctx->st, ctx->stream);
-  if (part_copy(ctx, sp->A, sp->P0)) return -1;
-  launch_lin(n, sp->A.c[7], sp->A.c[7], nullptr, qm, LIN_SCALE, ctx->st, ctx->stream);
+  sp->q_live = false;
+  launch_renew(sp->P0, sp->A, tg.ntiles, qm, ctx->stream);
   CK(cudaGetLastError());
   return 0;
 }
@@ -866,11 +889,13 @@ extern "C" int qp_species_qdp(qp_species* sp, qp_field2d* qe) {
   if (qe->state != 0) return fail(ctx, __LINE__, "sum: states are different");
   const GridDims& g = ctx->g;
   float* q = sp->q->rs[0];
+  sp->q_live = false;
   launch_lin(g.rplane, q, nullptr, nullptr, 0.f, LIN_FILL, ctx->st, ctx->stream);
   launch_deposit_rho(sp->A, ctx->tg, q, ctx->st, ctx->stream);
   sp->q->state = 0;
-  launch_lin(g.rplane, qe->rs[0], q, qe->rs[0], 0.f, LIN_ADD, ctx->st, ctx->stream);
-  launch_lin(g.rplane, qe->rs[0], sp->qn->rs[0], qe->rs[0], 0.f, LIN_ADD, ctx->st, ctx->stream);
+  LinList l(ctx->st, ctx->stream);
+  l.add(LinPlane{qe->rs[0], q, qe->rs[0], sp->qn->rs[0], nullptr, g.rplane, 0.f, LIN_ADD3});
+  l.flush();
   CK(cudaGetLastError());
   return 0;
 }
@@ -915,21 +940,17 @@ extern "C" int qp_species_amjdp(qp_species* sp, qp_field2d* fxy, qp_field2d* bxy
     return fail(ctx, __LINE__, "amjdp: invalid vector size");
   float* acc[8] = {sp->cusp->rs[0], sp->cusp->rs[1], sp->cusp->rs[2], sp->dcusp->rs[0],
                    sp->dcusp->rs[1], sp->amusp->rs[0], sp->amusp->rs[1], sp->amusp->rs[2]};
-  for (int i = 0; i < 8; ++i)
-    launch_lin(g.rplane, acc[i], nullptr, nullptr, 0.f, LIN_FILL, ctx->st, ctx->stream);
+  LinList l(ctx->st, ctx->stream);
+  for (int i = 0; i < 8; ++i) l.add(LIN_FILL, g.rplane, acc[i]);
+  l.flush();
   launch_amjdp(sp->A, ctx->tg, gplanes(fxy, bxyz, psit, 0), acc, sp->qbm, sp->dt, dex, 1.0f,
                ctx->st, ctx->stream);
-  for (int c = 0; c < 3; ++c)
-    launch_lin(g.rplane, cu->rs[c], sp->cusp->rs[c], cu->rs[c], 0.f, LIN_ADD, ctx->st, ctx->stream);
-  for (int c = 0; c < 2; ++c)
-    launch_lin(g.rplane, dcu->rs[c], sp->dcusp->rs[c], dcu->rs[c], 0.f, LIN_ADD, ctx->st,
-               ctx->stream);
-  for (int c = 0; c < 3; ++c)
-    launch_lin(g.rplane, amu->rs[c], sp->amusp->rs[c], amu->rs[c], 0.f, LIN_ADD, ctx->st,
-               ctx->stream);
-  for (int c = 0; c < 3; ++c)
-    launch_lin(g.rplane, sp->cusp->rs[c], sp->cusp->rs[c], nullptr, dex, LIN_SCALE, ctx->st,
-               ctx->stream);
+  float* out[8] = {cu->rs[0], cu->rs[1], cu->rs[2], dcu->rs[0],
+                   dcu->rs[1], amu->rs[0], amu->rs[1], amu->rs[2]};
+  for (int i = 0; i < 8; ++i)
+    l.add(LinPlane{out[i], acc[i], out[i], nullptr, i < 3 ? acc[i] : nullptr, g.rplane, dex,
+                   i < 3 ? LIN_ADDSC : LIN_ADD});
+  l.flush();
   cu->state = dcu->state = amu->state = 0;
   CK(cudaGetLastError());
   return check_particles(ctx, "amjdp");
@@ -940,6 +961,7 @@ extern "C" int qp_species_amjdp(qp_species* sp, qp_field2d* fxy, qp_field2d* bxy
 static int push_rebin(qp_species* sp, int mode, const GatherPlanes& f, float dex) {
   qp_ctx* ctx = sp->ctx;
   const int nt = ctx->tg.ntiles;
+  sp->q_live = false;
   for (int attempt = 0; attempt < 12; ++attempt) {
     if (sp->B.cap < sp->A.cap) {
       part_free(&sp->B);
@@ -988,6 +1010,7 @@ extern "C" int qp_species_push(qp_species* sp, qp_field2d* fxy, qp_field2d* bxyz
 extern "C" int qp_species_partpush(qp_species* sp, qp_field2d* fxy, qp_field2d* bxyz,
                                    qp_field2d* psit, float dex) {
   qp_ctx* ctx = sp->ctx;
+  sp->q_live = false;
   launch_push(0, sp->A, sp->A, sp->ib, ctx->tg, gplanes(fxy, bxyz, psit, 0), sp->qbm, sp->dt, dex,
               ctx->st, ctx->stream);
   CK(cudaGetLastError());
@@ -1003,12 +1026,7 @@ extern "C" int qp_species_cbq(qp_species* sp, int pos) {
   qp_ctx* ctx = sp->ctx;
   const GridDims& g = ctx->g;
   if (pos < 1 || pos > ctx->nz + 1) return fail(ctx, __LINE__, "cbq: slice out of range");
-  int px = 0, py = 0;
-  const float* add[1] = {sp->cusp->rs[2]};
-  fft_rk(ctx, sp->q->rs, sp->q->ks, add, 1, &px, &py);
-  float* in[8] = {sp->q->ks[0]};
-  launch_kpoint(KOP_SMOOTH, g, ctx->kc, in, in, 0.f, 1.f, ctx->st, ctx->stream);
-  fft_kr(ctx, sp->q->rs, sp->q->ks, 1, &px, &py);
+  smooth_charge(sp, sp->q->rs[0], sp->cusp->rs[2]);
   CK(cudaMemcpyAsync(sp->q3 + (size_t)(pos - 1) * g.rplane, sp->q->rs[0],
                      sizeof(float) * g.rplane, cudaMemcpyDeviceToDevice, ctx->stream));
   sp->q->state = 0;
@@ -1059,6 +1077,7 @@ extern "C" int qp_species_upload(qp_species* sp, const float* ppart, const int* 
   const int nt = ctx->tg.ntiles;
   int mx = 0;
   for (int t = 0; t < nt; ++t) mx = std::max(mx, kpic[t]);
+  sp->q_live = false;
   if (mx > sp->A.cap) {
     part_free(&sp->A);
     if (part_alloc(&sp->A, nt, mx)) return fail(ctx, __LINE__, "out of device memory");

@@ -219,30 +219,38 @@ __global__ void __launch_bounds__(256) k_xinv(XJob job, GridDims g, LineTables t
 }
 
 // ------------------------------------------------------------------ y pass
-// In-place y transform of the columns kx of every component, times scale_c.
-template <int P>
-__global__ void __launch_bounds__(256) k_ycol(YJob job, GridDims g, LineTables ty,
-                                              const DevStatus* st) {
-  grid_dep_sync();
+// In-place y transform of the columns kx of component blockIdx.y, times
+// scale_c; with SMOOTH the smoothing operator is applied to the transformed
+// column and the column is transformed back (sine lines: parity_c of the
+// inverse is that of the forward transform).  One warp per column and
+// component: a launch is one latency chain (load, transform, store), so the
+// components of a vector run side by side instead of one after another.
+template <int P, bool SMOOTH>
+__global__ void __launch_bounds__(256) k_ycol(const __grid_constant__ YJob job, GridDims g,
+                                              KCoef K, LineTables ty, const DevStatus* st) {
   extern __shared__ __align__(16) float smem[];
-  if (st && st->error) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = g.ny, pitch = line_pitch(n);
   float* L = smem + warp * pitch;
   float* S = smem + (8 + warp) * pitch;
   float* T = smem + line_count(g.indy) * pitch;
-  if (P > 0) {
-    stage_lane_table(T, ty);
-    __syncthreads();
-  }
+  if (P > 0) stage_lane_table(T, ty);  // constant tables: staged before the wait
+  grid_dep_sync();
+  if (st && st->error) return;
+  if (P > 0) __syncthreads();
   const int kx = blockIdx.x * 8 + warp;
   if (kx > g.nx) return;
-  for (int ci = 0; ci < job.ncomp; ++ci) {
-    float* col = job.c[ci].plane + (long long)kx * g.kp;
-    line_transform<P>(col, nullptr, 1.f, L, S, g.indy, job.c[ci].parity, ty, T, lane);
-    line_store(col, L, n, job.c[ci].scale, lane);
+  const YComp c = job.c[blockIdx.y];
+  float* col = c.plane + (long long)kx * g.kp;
+  line_transform<P>(col, nullptr, 1.f, L, S, g.indy, c.parity, ty, T, lane);
+  float scale = c.scale;
+  if (SMOOTH) {
+    for (int ky = lane; ky <= n; ky += 32) L[ky] = k_smooth(K, kx, ky, QM(L[ky], scale));
     __syncwarp();
+    line_transform<P>(L, nullptr, 1.f, L, S, g.indy, c.parity, ty, T, lane);
+    scale = 1.f;
   }
+  line_store(col, L, n, scale, lane);
 }
 
 size_t xpass_smem(const GridDims& g) {
@@ -258,7 +266,9 @@ static int set_smem_limits(int big) {
           cudaSuccess ||
       cudaFuncSetAttribute(k_xinv<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) !=
           cudaSuccess ||
-      cudaFuncSetAttribute(k_ycol<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) !=
+      cudaFuncSetAttribute(k_ycol<P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_ycol<P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) !=
           cudaSuccess)
     return -2;
   return 0;
@@ -289,8 +299,16 @@ void launch_xinv(const XJob& job, const GridDims& g, const LineTables& tx, const
 
 void launch_ycol(const YJob& job, const GridDims& g, const LineTables& ty, const DevStatus* st,
                  cudaStream_t s) {
-  dim3 grid((g.nx + 1 + 7) / 8);
-  QP_LINE_SWITCH(g.indy, (launch_pdl(k_ycol<P_>, grid, 256, ypass_smem(g), s, job, g, ty, st)));
+  dim3 grid((g.nx + 1 + 7) / 8, job.ncomp);
+  QP_LINE_SWITCH(g.indy, (launch_pdl(k_ycol<P_, false>, grid, 256, ypass_smem(g), s, job, g,
+                                     KCoef{}, ty, st)));
+}
+
+void launch_ysmooth(const YJob& job, const GridDims& g, const KCoef& K, const LineTables& ty,
+                    const DevStatus* st, cudaStream_t s) {
+  dim3 grid((g.nx + 1 + 7) / 8, job.ncomp);
+  QP_LINE_SWITCH(g.indy, (launch_pdl(k_ycol<P_, true>, grid, 256, ypass_smem(g), s, job, g, K, ty,
+                                     st)));
 }
 
 }  // namespace qp

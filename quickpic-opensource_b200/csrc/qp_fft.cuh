@@ -2,6 +2,7 @@
 #pragma once
 
 #include "qp_common.cuh"
+#include "qp_solve.cuh"
 
 namespace qp {
 
@@ -34,7 +35,7 @@ struct XJob {
   int ncomp;
   // xinv only: real-space planes whose rows this launch clears (plane i is
   // cleared by the CTAs of component i % ncomp)
-  float* zero[8];
+  float* zero[16];
   int nzero;
   int pass;  // predictor-corrector pass of the launch (pass_skipped), 0 = none
 };
@@ -58,5 +59,10 @@ void launch_xinv(const XJob& job, const GridDims& g, const LineTables& tx, const
                  cudaStream_t s);
 void launch_ycol(const YJob& job, const GridDims& g, const LineTables& ty, const DevStatus* st,
                  cudaStream_t s);
+
+// species2d%cbq between the two x passes: y forward (times scale), the
+// smoothing of every mode, y inverse, in one pass over the columns
+void launch_ysmooth(const YJob& job, const GridDims& g, const KCoef& K, const LineTables& ty,
+                    const DevStatus* st, cudaStream_t s);
 
 }  // namespace qp

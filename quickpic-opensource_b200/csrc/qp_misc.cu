@@ -2,6 +2,8 @@
 // and the small per-slice kernels of the fused 3D step.
 #include "qp_misc.cuh"
 
+#include <algorithm>
+
 namespace qp {
 
 namespace {
@@ -77,96 +79,92 @@ __global__ void k_kpoint(int op, GridDims g, KCoef K, KPtrs in, KPtrs out, float
   }
 }
 
-__global__ void k_lin(long long n, float* d, const float* a, const float* b, float v, int op,
-                      const DevStatus* st) {
+__device__ __forceinline__ float lin1(int op, float a, float b, float c, float v) {
+  switch (op) {
+    case LIN_FILL: return v;
+    case LIN_SCALE: return a * v;
+    case LIN_SUB: return a - b;
+    case LIN_COPY: return a;
+    case LIN_ADD3: return c + (a + b);
+    default: return a + b;  // LIN_ADD, LIN_ADDSC
+  }
+}
+
+// One row of CTAs per plane, four nodes per thread and step.  Bound by launch
+// latency: a plane is 0.02 - 4.2 MB and stays in L2, so a launch costs about
+// 4 us in a stream whatever it moves.  What counts is the number of launches
+// (the class interface's amjdp: 20 with one plane each, 3 with a job's).
+__global__ void __launch_bounds__(256) k_lin(const __grid_constant__ LinJob job, const DevStatus* st) {
   grid_dep_sync();
   if (st && st->error) return;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    switch (op) {
-      case LIN_FILL:
-        d[i] = v;
-        break;
-      case LIN_SCALE:
-        d[i] = a[i] * v;
-        break;
-      case LIN_ADD:
-        d[i] = a[i] + b[i];
-        break;
-      case LIN_SUB:
-        d[i] = a[i] - b[i];
-        break;
-      case LIN_COPY:
-        d[i] = a[i];
-        break;
+  const LinPlane& p = job.p[blockIdx.y];
+  const int op = p.op;
+  const float v = p.v;
+  const bool ra = op != LIN_FILL, rb = op != LIN_FILL && op != LIN_SCALE && op != LIN_COPY;
+  const bool rc = op == LIN_ADD3;
+  const long long n4 = p.n >> 2;
+  const long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  for (long long i = i0; i < n4; i += step) {
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 a = ra ? reinterpret_cast<const float4*>(p.a)[i] : z;
+    const float4 b = rb ? reinterpret_cast<const float4*>(p.b)[i] : z;
+    const float4 c = rc ? reinterpret_cast<const float4*>(p.c)[i] : z;
+    reinterpret_cast<float4*>(p.d)[i] =
+        make_float4(lin1(op, a.x, b.x, c.x, v), lin1(op, a.y, b.y, c.y, v),
+                    lin1(op, a.z, b.z, c.z, v), lin1(op, a.w, b.w, c.w, v));
+    if (op == LIN_ADDSC)
+      reinterpret_cast<float4*>(p.s)[i] = make_float4(a.x * v, a.y * v, a.z * v, a.w * v);
+  }
+  for (long long i = 4 * n4 + i0; i < p.n; i += step) {  // a length that is not a multiple of 4
+    const float a = ra ? p.a[i] : 0.f;
+    p.d[i] = lin1(op, a, rb ? p.b[i] : 0.f, rc ? p.c[i] : 0.f, v);
+    if (op == LIN_ADDSC) p.s[i] = a * v;
+  }
+}
+
+__global__ void __launch_bounds__(256) k_sum(const __grid_constant__ SumJob job, long long n,
+                                             float* d, const DevStatus* st) {
+  grid_dep_sync();
+  if (st && st->error) return;
+  const long long n4 = n >> 2;
+  const long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  for (long long i = i0; i < n4; i += step) {
+    float4 v = job.onto ? reinterpret_cast<const float4*>(d)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = 0; k < job.count; ++k) {
+      const float4 a = reinterpret_cast<const float4*>(job.src[k])[i];
+      v = make_float4(a.x + v.x, a.y + v.y, a.z + v.z, a.w + v.w);
     }
+    reinterpret_cast<float4*>(d)[i] = v;
+  }
+  for (long long i = 4 * n4 + i0; i < n; i += step) {
+    float v = job.onto ? d[i] : 0.f;
+    for (int k = 0; k < job.count; ++k) v = job.src[k][i] + v;
+    d[i] = v;
   }
 }
 
 // copyguard: row ny = row 0, every column (ufield2d_lib.f03:37-42)
-__global__ void k_guard_copy(float* p, GridDims g, const DevStatus* st) {
+__global__ void k_guard_copy(Planes3 pl, GridDims g, const DevStatus* st) {
   grid_dep_sync();
   if (st && st->error) return;
+  float* p = pl.p[blockIdx.y];
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j <= g.nx + 1) p[(long long)g.ny * g.rp + j] = p[j];
 }
 
 // acopyguard: row 0 += row ny, row ny = 0 for columns 0..nx (ufield2d_lib.f03:90-97)
-__global__ void k_guard_add(float* p, GridDims g, const DevStatus* st) {
+__global__ void k_guard_add(Planes3 pl, GridDims g, const DevStatus* st) {
   grid_dep_sync();
   if (st && st->error) return;
+  float* p = pl.p[blockIdx.y];
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j <= g.nx) {
     float* top = p + (long long)g.ny * g.rp + j;
     p[j] = p[j] + *top;
     *top = 0.f;
   }
-}
-
-// bxyz assembly in Fourier space (simulation_class.f03:677-680 and 717-720):
-//   bx = -dex*epw(2) - epwb(2); by = dex*epw(1) + epwb(1); bz = dex*bz
-__global__ void k_assemble(GridDims g, float* bx, float* by, float* bz, const float* ex,
-                           const float* ey, const float* ebx, const float* eby, float dex,
-                           const DevStatus* st) {
-  grid_dep_sync();
-  if (st->error) return;
-  int kx, ky;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (!kidx(g, i, &kx, &ky)) return;
-  const long long o = (long long)kx * g.kp + ky;
-  const float b1 = ey[o] * (-dex);
-  const float b2 = ex[o] * dex;
-  bz[o] = bz[o] * dex;
-  bx[o] = b1 - eby[o];
-  by[o] = b2 + ebx[o];
-}
-
-// end-of-slice extrapolation of the current in Fourier space
-// (simulation_class.f03:725-726): dcu = dcu*dxi; cu(1:2) = cu(1:2) - dcu(1:2)
-__global__ void k_extrap(GridDims g, float* cx, float* cy, float* dx, float* dy, float dxi,
-                         const DevStatus* st) {
-  grid_dep_sync();
-  if (st->error) return;
-  int kx, ky;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (!kidx(g, i, &kx, &ky)) return;
-  const long long o = (long long)kx * g.kp + ky;
-  const float a = dx[o] * dxi, b = dy[o] * dxi;
-  dx[o] = a;
-  dy[o] = b;
-  cx[o] = cx[o] - a;
-  cy[o] = cy[o] - b;
-}
-
-// Fourier-space scale of one plane, skipped after an error
-__global__ void k_kscale(GridDims g, float* p, float v, const DevStatus* st) {
-  grid_dep_sync();
-  if (st->error) return;
-  int kx, ky;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (!kidx(g, i, &kx, &ky)) return;
-  const long long o = (long long)kx * g.kp + ky;
-  p[o] = p[o] * v;
 }
 
 // End of a slice (simulation_class.f03:722-735): the final force
@@ -259,38 +257,61 @@ int launch_kpoint(int op, const GridDims& g, const KCoef& K, float* const* in, f
   return 0;
 }
 
+bool lin_conflict(const LinJob& job, const LinPlane& q) {
+  auto overlap = [](const float* x, long long nx, const float* y, long long ny) {
+    return x && y && x < y + ny && y < x + nx;
+  };
+  for (int i = 0; i < job.count; ++i) {
+    const LinPlane& p = job.p[i];
+    for (const float* w : {(const float*)p.d, (const float*)p.s})
+      for (const float* r : {(const float*)q.d, (const float*)q.s, q.a, q.b, q.c})
+        if (overlap(w, p.n, r, q.n)) return true;
+    for (const float* w : {(const float*)q.d, (const float*)q.s})
+      for (const float* r : {p.a, p.b, p.c})
+        if (overlap(w, q.n, r, p.n)) return true;
+  }
+  return false;
+}
+
+static int lin_blocks(long long n, int rows) {
+  const long long want = ((n >> 2) + 255) / 256, most = std::max(1, 148 * 16 / rows);
+  return (int)std::max(1LL, std::min(want, most));
+}
+
+void launch_lin_job(const LinJob& job, const DevStatus* st, cudaStream_t s) {
+  long long n = 1;
+  for (int i = 0; i < job.count; ++i) n = std::max(n, job.p[i].n);
+  launch_pdl(k_lin, dim3(lin_blocks(n, job.count), job.count), 256, 0, s, job, st);
+}
+
 void launch_lin(long long n, float* d, const float* a, const float* b, float v, int op,
                 const DevStatus* st, cudaStream_t s) {
-  long long blocks = (n + 255) / 256;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  if (blocks < 1) blocks = 1;
-  launch_pdl(k_lin, (int)blocks, 256, 0, s, n, d, a, b, v, op, st);
+  LinJob job{};
+  job.p[0] = LinPlane{d, a, b, nullptr, nullptr, n, v, op};
+  job.count = 1;
+  launch_lin_job(job, st, s);
 }
 
-void launch_guard_copy(float* p, const GridDims& g, const DevStatus* st, cudaStream_t s) {
-  launch_pdl(k_guard_copy, (g.nx + 2 + 255) / 256, 256, 0, s, p, g, st);
+void launch_sum(const SumJob& job, long long n, float* d, const DevStatus* st, cudaStream_t s) {
+  launch_pdl(k_sum, lin_blocks(n, 1), 256, 0, s, job, n, d, st);
 }
 
-void launch_guard_add(float* p, const GridDims& g, const DevStatus* st, cudaStream_t s) {
-  launch_pdl(k_guard_add, (g.nx + 1 + 255) / 256, 256, 0, s, p, g, st);
+static Planes3 planes3(float* const* p, int count) {
+  Planes3 r{};
+  for (int i = 0; i < count; ++i) r.p[i] = p[i];
+  return r;
 }
 
-void launch_assemble(const GridDims& g, float* const* bxyz, float* const* epw,
-                     float* const* epwb, float dex, const DevStatus* st, cudaStream_t s) {
-  const int n = (g.nx + 1) * (g.ny + 1);
-  launch_pdl(k_assemble, (n + 255) / 256, 256, 0, s, g, bxyz[0], bxyz[1], bxyz[2], epw[0], epw[1],
-                                             epwb[0], epwb[1], dex, st);
+void launch_guard_copy(float* const* p, int count, const GridDims& g, const DevStatus* st,
+                       cudaStream_t s) {
+  launch_pdl(k_guard_copy, dim3((g.nx + 2 + 255) / 256, count), 256, 0, s, planes3(p, count), g,
+             st);
 }
 
-void launch_extrap(const GridDims& g, float* const* cu, float* const* dcu, float dxi,
-                   const DevStatus* st, cudaStream_t s) {
-  const int n = (g.nx + 1) * (g.ny + 1);
-  launch_pdl(k_extrap, (n + 255) / 256, 256, 0, s, g, cu[0], cu[1], dcu[0], dcu[1], dxi, st);
-}
-
-void launch_kscale(const GridDims& g, float* p, float v, const DevStatus* st, cudaStream_t s) {
-  const int n = (g.nx + 1) * (g.ny + 1);
-  launch_pdl(k_kscale, (n + 255) / 256, 256, 0, s, g, p, v, st);
+void launch_guard_add(float* const* p, int count, const GridDims& g, const DevStatus* st,
+                      cudaStream_t s) {
+  launch_pdl(k_guard_add, dim3((g.nx + 1 + 255) / 256, count), 256, 0, s, planes3(p, count), g,
+             st);
 }
 
 void launch_cursor(DevStatus* st, int v, cudaStream_t s) {

@@ -13,17 +13,76 @@ struct Planes3 {
   float* p[3];
 };
 
-enum { LIN_FILL = 0, LIN_SCALE, LIN_ADD, LIN_SUB, LIN_COPY };
+// Element-wise operations on planes, several planes per launch (grid row i =
+// plane i).  Every plane starts on a 16-byte boundary; the planes of one job
+// must not depend on one another (lin_conflict).
+//   FILL d = v   SCALE d = a v   ADD d = a + b   SUB d = a - b   COPY d = a
+//   ADD3 d = c + (a + b)         ADDSC d = a + b, then s = a v (s may be a)
+enum { LIN_FILL = 0, LIN_SCALE, LIN_ADD, LIN_SUB, LIN_COPY, LIN_ADD3, LIN_ADDSC };
+constexpr int LIN_MAX = 24;
+struct LinPlane {
+  float* d;
+  const float* a;
+  const float* b;
+  const float* c;
+  float* s;
+  long long n;
+  float v;
+  int op;
+};
+struct LinJob {
+  LinPlane p[LIN_MAX];
+  int count;
+};
+// whether plane `q` reads or writes what a plane of the job writes, or writes
+// what one of them reads: then it has to wait for them
+bool lin_conflict(const LinJob& job, const LinPlane& q);
+void launch_lin_job(const LinJob& job, const DevStatus* st, cudaStream_t s);
+
+// A list of element-wise operations in the caller's order, launched in as few
+// jobs as their dependences allow.  flush() returns the launches made so far.
+class LinList {
+ public:
+  LinList(const DevStatus* st, cudaStream_t s) : st_(st), s_(s) {}
+  void add(const LinPlane& q) {
+    if (job_.count == LIN_MAX || lin_conflict(job_, q)) flush();
+    job_.p[job_.count++] = q;
+  }
+  void add(int op, long long n, float* d, const float* a = nullptr, const float* b = nullptr,
+           float v = 0.f) {
+    add(LinPlane{d, a, b, nullptr, nullptr, n, v, op});
+  }
+  int flush() {
+    if (job_.count) {
+      launch_lin_job(job_, st_, s_);
+      ++launches_;
+    }
+    job_.count = 0;
+    return launches_;
+  }
+
+ private:
+  LinJob job_{};
+  int launches_ = 0;
+  const DevStatus* st_;
+  cudaStream_t s_;
+};
 
 void launch_lin(long long n, float* d, const float* a, const float* b, float v, int op,
                 const DevStatus* st, cudaStream_t s);
-void launch_guard_copy(float* p, const GridDims& g, const DevStatus* st, cudaStream_t s);
-void launch_guard_add(float* p, const GridDims& g, const DevStatus* st, cudaStream_t s);
-void launch_assemble(const GridDims& g, float* const* bxyz, float* const* epw,
-                     float* const* epwb, float dex, const DevStatus* st, cudaStream_t s);
-void launch_extrap(const GridDims& g, float* const* cu, float* const* dcu, float dxi,
-                   const DevStatus* st, cudaStream_t s);
-void launch_kscale(const GridDims& g, float* p, float v, const DevStatus* st, cudaStream_t s);
+
+// d = src[n-1] + (... + (src[0] + 0)), or on top of d when `onto` is set
+constexpr int SUM_MAX = 16;
+struct SumJob {
+  const float* src[SUM_MAX];
+  int count, onto;
+};
+void launch_sum(const SumJob& job, long long n, float* d, const DevStatus* st, cudaStream_t s);
+// of `count` (1..3) planes in one launch
+void launch_guard_copy(float* const* p, int count, const GridDims& g, const DevStatus* st,
+                       cudaStream_t s);
+void launch_guard_add(float* const* p, int count, const GridDims& g, const DevStatus* st,
+                      cudaStream_t s);
 void launch_cursor(DevStatus* st, int v, cudaStream_t s);
 // also clears zero_q (if not null) and advances the slice cursor
 void launch_store3d(const GridDims& g, float* const* fxy, float* const* bxyz, const float* psit,

@@ -19,6 +19,8 @@
 // memory or a plane; a particle outside its tile raises a status error instead.
 #include "qp_part.cuh"
 
+#include <algorithm>
+
 namespace qp {
 
 namespace {
@@ -805,6 +807,29 @@ __global__ void __launch_bounds__(256) k_insert(PartBuf B, Inbox ib, TileGeom tg
   if (dq) deposit_tile(B, tg, t, stay + nin, dq, st);
 }
 
+// species2d%renew on the device: one read of the pristine particles and one
+// write of the live buffer, component blockIdx.y, four slots per thread (in
+// place of a fill, a strided copy per component and a scaling pass over q).
+// Both capacities are multiples of 4, so a float4 never spans two tiles.
+__global__ void __launch_bounds__(256) k_renew(PartBuf P0, PartBuf A, int ntiles, float qm) {
+  grid_dep_sync();
+  const int c = blockIdx.y;
+  const int na = A.cap >> 2, np = P0.cap >> 2;
+  const long long n4 = (long long)ntiles * na;
+  const long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  for (long long i = i0; i < n4; i += (long long)gridDim.x * blockDim.x) {
+    const long long t = i / na;
+    const int k = (int)(i - t * na);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (k < np) v = reinterpret_cast<const float4*>(P0.c[c])[t * np + k];
+    if (c == 7) v = make_float4(v.x * qm, v.y * qm, v.z * qm, v.w * qm);
+    reinterpret_cast<float4*>(A.c[c])[i] = v;
+  }
+  if (c == 0)
+    for (long long t = i0; t < ntiles; t += (long long)gridDim.x * blockDim.x)
+      A.count[t] = P0.count[t];
+}
+
 }  // namespace
 
 int part_kernels_init() {
@@ -821,6 +846,12 @@ void launch_insert(const PartBuf& B, const Inbox& ib, const TileGeom& tg, DevSta
   while (p2 < ib.cap) p2 <<= 1;
   const size_t smem = (size_t)p2 * (sizeof(unsigned long long) + sizeof(int));
   launch_pdl(k_insert, tg.ntiles, 256, smem, s, B, ib, tg, p2, st, deposit_q);
+}
+
+void launch_renew(const PartBuf& P0, const PartBuf& A, int ntiles, float qm, cudaStream_t s) {
+  const long long n4 = (long long)ntiles * (A.cap >> 2);
+  const long long blocks = std::max(1LL, std::min((n4 + 255) / 256, 148LL * 8));
+  launch_pdl(k_renew, dim3((unsigned)blocks, NCOMP), 256, 0, s, P0, A, ntiles, qm);
 }
 
 void launch_deposit_rho(const PartBuf& P, const TileGeom& tg, float* q, const DevStatus* st,

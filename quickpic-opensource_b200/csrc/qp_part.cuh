@@ -60,6 +60,8 @@ void launch_amjdp(const PartBuf& P, const TileGeom& tg, const GatherPlanes& f, f
 void launch_push(int mode, const PartBuf& A, const PartBuf& B, const Inbox& ib,
                  const TileGeom& tg, const GatherPlanes& f, float qbm, float dt, float dex,
                  DevStatus* st, cudaStream_t s);
+// A = the particles of P0 (rest of A's slots zero) with charge q P0's times qm
+void launch_renew(const PartBuf& P0, const PartBuf& A, int ntiles, float qm, cudaStream_t s);
 // deposit_q (optional): after the re-bin, deposit the charge of every
 // particle of the tile into deposit_q (zero on entry), as k_deposit_rho does
 void launch_insert(const PartBuf& B, const Inbox& ib, const TileGeom& tg, DevStatus* st,

@@ -45,3 +45,67 @@ def test_two_half_density_species_are_one_plasma(qp, ind, iter, graphs):
     assert rel_l2(two["epw"], one["epw"]) < 1e-4
     assert rel_l2(two["q3"], one["q3"]) < 1e-4
     assert np.isfinite(two["bb"]).all()
+
+
+@pytest.mark.parametrize("nspecies", [1, 3])
+def test_particles_restored_between_slices_give_the_same_slices(qp, nspecies):
+    """A caller that puts a species' particles back between two slices (here the
+    ones it has just read, in another order) gets the slices it would have got
+    without: the charge of the next slice is formed from what it put there."""
+    def run(restore):
+        c = qp.Context(6, 6, 5, BOX)
+        sp = [qp.Species2d(c, ppc=(2, 2), density=1.0 / nspecies) for _ in range(nspecies)]
+        bm = qp.Beam3d(c, (16, 16, 32), gamma=20000.0, peak_density=2.0, center=(0.0, 0.0, 2.5),
+                       sigma=(0.5, 0.5, 0.5))
+        sim = qp.Simulation(c, sp, [bm], iter=1)
+        sim.begin3d()
+        sim.slices(15)
+        if restore:
+            for s in sp:
+                pp, kp = s.get_particles()
+                pp[7] *= 0.5  # wrong charges, which must be gone again below
+                s.set_particles(pp, kp)
+                pp[7] *= 2.0
+                for t in range(s.ntiles):
+                    pp[:, : kp[t], t] = pp[:, : kp[t], t][:, ::-1]
+                s.set_particles(pp, kp)
+        sim.slices(17)
+        sim.end3d()
+        be = sim.get_3d("bexyz")
+        for h in [sim, bm, *sp, c]:
+            h.close()
+        return be
+
+    assert rel_l2(run(True), run(False)) < 1e-5  # FP32 sums in another order
+
+
+@pytest.mark.parametrize("ind", [(4, 4), (6, 5), (5, 9)])
+def test_field_algebra_runs_components_in_the_lists_order(qp, ind):
+    """mult / add / sub over component lists, several of them in one launch: the
+    same as one component after another, also where a component reads what an
+    earlier one of the list wrote, and for planes whose length is no multiple of
+    the launch."""
+    c = qp.Context(ind[0], ind[1], 1, BOX)
+    rng = np.random.default_rng(3)
+    a, b = qp.Field2d(c, 3), qp.Field2d(c, 3)
+    va, vb = (rng.standard_normal(c.ks_shape(3)).astype(np.float32) for _ in range(2))
+    cases = [("mult", a, None, [1, 2], [2, 1], [2.0, 3.0]), ("mult", b, None, [1, 3], [3, 1], [0.5, -1.0]),
+             ("add", a, b, [1, 2, 3], [2, 1, 3], [1, 3, 2]), ("sub", a, b, [2, 1], [1, 2], [2, 2])]
+    for op, x, y, d, d1, third in cases:
+        a.set_ks(va)
+        b.set_ks(vb)
+        ref = {id(a): va.copy(), id(b): vb.copy()}
+        for i in range(len(d)):
+            src = ref[id(x)][d1[i] - 1]
+            if op == "mult":
+                ref[id(a)][d[i] - 1] = src * np.float32(third[i])
+            else:
+                o = ref[id(y)][third[i] - 1]
+                ref[id(a)][d[i] - 1] = src + o if op == "add" else src - o
+        if op == "mult":
+            a.mult(x, third, dim=d, dim1=d1)
+        else:
+            getattr(a, op)(x, y, dim=d, dim1=d1, dim2=third)
+        assert np.array_equal(a.get_ks(), ref[id(a)])
+    for h in (a, b, c):
+        h.close()
