@@ -6,6 +6,10 @@
 //   k-space plane     K[kx][ky], kx = 0..nx, ky = 0..ny, pitch kp = ny + 4;
 //                     the same array holds the half-transformed data between
 //                     the x pass and the y pass ([kx][y])
+//   the fused step's force fields are node-major instead: real space
+//                     [y][x][4], k space [kx][ky][4], in two groups of four --
+//                     (psit, bx, by, bz) and (fx, fy, psi, unused) -- so that a
+//                     node is one 16-byte access
 //   particles         structure of arrays: 8 planes (x, y, px, py, pz, p6, p7, q)
 //                     of ntiles * cap floats; tile t owns [t*cap, t*cap+count[t])
 // Grid nodes, tile size and the particle slots follow QuickPIC's part2d/ufield2d
@@ -76,10 +80,10 @@ struct __align__(16) DevStatus {
   int fail_slice;     // slice index at which the first error was raised
   int need_cap;       // particles a tile must hold
   int need_inbox;     // movers a tile must accept
-  int cursor;         // slice cursor of the fused 3D step
+  int cursor;         // slice cursor of the fused 3D step (moved on by k_slice_a)
   int pass_done;      // convergence-controlled B loop: the pass of this slice
                       // whose residual met the tolerance (0 = none yet)
-  int store_ctas;     // CTA completion counter of the 3D store kernel
+  int unused0;
   int beam_drops;     // beam particles dropped at the conducting boundary
   float resid_num;    // residual of the current pass: sum |epw - epw_old|^2
   float resid_den;    //                               sum |epw|^2

@@ -109,7 +109,7 @@ void line_tables_free(LineTablesHost* t) {
 // The slice cursor must name one of the planes of the 3D array a component
 // reads or writes; otherwise the launch raises an error and does nothing.
 __device__ __forceinline__ bool cursor_ok(const XComp& c, const DevStatus* st) {
-  const int cur = st->cursor;
+  const int cur = st->cursor + c.cursor_next;
   if (cur >= 0 && cur < c.cursor_planes) return true;
   if (threadIdx.x == 0) atomicCAS(const_cast<int*>(&st->error), 0, -7);
   return false;
@@ -124,27 +124,18 @@ static __host__ __device__ int line_count(int logn) { return logn < 6 ? 16 : 8; 
 // Forward x pass: for every component c and row y, the line
 //   x[j] = scale_c * (src_c[y][j] + src2_c[y][j]),  j = 0..nx
 // is transformed with parity_c and stored transposed into dst_c[kx][y].
+// The 8 rows y0 .. y0 + 7 of component c (the CTA's 8 warps).
 template <int P>
-__global__ void __launch_bounds__(256) k_xfwd(XJob job, GridDims g, LineTables tx,
-                                              const DevStatus* st) {
-  extern __shared__ __align__(16) float smem[];
+__device__ __forceinline__ void xfwd_rows(const XComp& c, int y0, const GridDims& g,
+                                          const LineTables& tx, float* smem, float* T,
+                                          const DevStatus* st) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = g.nx, pitch = line_pitch(n);
   float* L = smem + warp * pitch;
   float* S = smem + (8 + warp) * pitch;
-  float* T = smem + line_count(g.indx) * pitch;
-  if (P > 0) stage_lane_table(T, tx);  // constant tables: staged before the wait
-  grid_dep_sync();
-  if (st && st->error) return;
-  if (pass_skipped(st, job.pass)) return;
-  const XComp c = job.c[blockIdx.y];
-  const int y0 = blockIdx.x * 8;
   const int y = y0 + warp;
-  long long cur = 0;
-  if (c.cursor_stride) {
-    if (!cursor_ok(c, st)) return;
-    cur = (long long)st->cursor * c.cursor_stride;
-  }
+  const long long cur =
+      c.cursor_stride ? (long long)(st->cursor + c.cursor_next) * c.cursor_stride : 0;
   if (P > 0) __syncthreads();
   if (y <= g.ny) {
     const float* s1 = c.src + cur + (long long)y * g.rp;
@@ -159,24 +150,30 @@ __global__ void __launch_bounds__(256) k_xfwd(XJob job, GridDims g, LineTables t
   }
 }
 
-// Inverse x pass: rows y of the [kx][y] array are gathered, transformed with
-// parity_c, scaled and written as real-space rows; row 0 is also written to the
-// guard row ny (copyguard), and the line computed for row ny is discarded.
 template <int P>
-__global__ void __launch_bounds__(256) k_xinv(XJob job, GridDims g, LineTables tx,
+__global__ void __launch_bounds__(256) k_xfwd(XJob job, GridDims g, LineTables tx,
                                               const DevStatus* st) {
   extern __shared__ __align__(16) float smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n = g.nx, pitch = line_pitch(n);
-  float* T = smem + line_count(g.indx) * pitch;
-  // constant tables, staged before the wait; the barrier after the gather covers them
-  if (P > 0) stage_lane_table(T, tx);
+  float* T = smem + line_count(g.indx) * line_pitch(g.nx);
+  if (P > 0) stage_lane_table(T, tx);  // constant tables: staged before the wait
   grid_dep_sync();
   if (st && st->error) return;
   if (pass_skipped(st, job.pass)) return;
   const XComp c = job.c[blockIdx.y];
   if (c.cursor_stride && !cursor_ok(c, st)) return;
-  const int y0 = blockIdx.x * 8;
+  xfwd_rows<P>(c, blockIdx.x * 8, g, tx, smem, T, st);
+}
+
+// Inverse x pass: rows y of the [kx][y] array are gathered, transformed with
+// parity_c, scaled and written as real-space rows; row 0 is also written to the
+// guard row ny (copyguard), and the line computed for row ny is discarded.
+// The 8 rows y0 .. y0 + 7 of component c (the CTA's 8 warps).
+template <int P>
+__device__ __forceinline__ void xinv_rows(const XComp& c, int y0, const GridDims& g,
+                                          const LineTables& tx, float* smem, float* T,
+                                          const DevStatus* st) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n = g.nx, pitch = line_pitch(n);
   // the 8 rows' [kx][y] entries, 32 bytes per kx: batches of 8 loads per
   // thread are all issued before their shared-memory stores, so a thread waits
   // for L2 twice per 16 loads instead of once per load
@@ -202,7 +199,7 @@ __global__ void __launch_bounds__(256) k_xinv(XJob job, GridDims g, LineTables t
   if (y < g.ny) {
     line_transform<P>(L, nullptr, 1.f, L, S, g.indx, c.parity, tx, T, lane);
     long long cur = 0;
-    if (c.cursor_stride) cur = (long long)st->cursor * c.cursor_stride;
+    if (c.cursor_stride) cur = (long long)(st->cursor + c.cursor_next) * c.cursor_stride;
     float* d = c.dst + cur + (long long)y * g.rp;
     line_store(d, L, n, c.scale, lane);
     if (y == 0) {
@@ -211,11 +208,137 @@ __global__ void __launch_bounds__(256) k_xinv(XJob job, GridDims g, LineTables t
       if (lane == 0) dg[n + 1] = d[n + 1];
     }
   }
+}
+
+template <int P>
+__global__ void __launch_bounds__(256) k_xinv(XJob job, GridDims g, LineTables tx,
+                                              const DevStatus* st) {
+  extern __shared__ __align__(16) float smem[];
+  const int pitch = line_pitch(g.nx);
+  float* T = smem + line_count(g.indx) * pitch;
+  // constant tables, staged before the wait; the barrier after the gather covers them
+  if (P > 0) stage_lane_table(T, tx);
+  grid_dep_sync();
+  if (st && st->error) return;
+  if (pass_skipped(st, job.pass)) return;
+  const XComp c = job.c[blockIdx.y];
+  if (c.cursor_stride && !cursor_ok(c, st)) return;
+  const int y0 = blockIdx.x * 8;
+  xinv_rows<P>(c, y0, g, tx, smem, T, st);
   for (int z = blockIdx.y; z < job.nzero; z += job.ncomp) {
     float* p = job.zero[z] + (long long)y0 * g.rp;
     const int rows = min(8, g.ny + 1 - y0);
     for (int i = threadIdx.x; i < rows * g.rp; i += 256) p[i] = 0.f;
   }
+}
+
+// Inverse x pass of node-major fields.  A CTA takes two rows of one group of
+// four components, its warps one line each: a (kx, y) pair of rows is one
+// 32-byte sector of the [kx][y][4] array, read as two float4, and a node of the
+// result is one float4 of the [y][x][4] array -- 5 loads and 5 stores of 16
+// bytes per thread at 512 points, where the planar form makes 17 of 4 bytes
+// each.  The remaining CTAs transform planar components, 8 rows each.
+template <int P>
+__global__ void __launch_bounds__(256) k_xinv4(const __grid_constant__ X4Job job, GridDims g,
+                                               LineTables tx, const DevStatus* st) {
+  extern __shared__ __align__(16) float smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n = g.nx, pitch = line_pitch(n);
+  float* T = smem + line_count(g.indx) * pitch;
+  if (P > 0) stage_lane_table(T, tx);  // constant tables: staged before the wait
+  grid_dep_sync();
+  if (st && st->error) return;
+  if (pass_skipped(st, job.x.pass)) return;
+  float* L = smem + warp * pitch;
+  float* S = smem + (8 + warp) * pitch;
+  const int pairs = g.ny >> 1;
+  if ((int)blockIdx.x < job.ngroup * pairs) {
+    const int gi = (int)blockIdx.x >= pairs ? 1 : 0;
+    const int y0 = 2 * ((int)blockIdx.x - gi * pairs);
+    const float4* src = job.src[gi] + y0;
+    // node (kx, row r) -> lines 4 r .. 4 r + 3; every load before the stores
+    constexpr int U = P == 8 ? 5 : 4;
+    const int total = 2 * (n + 1);
+    for (int b0 = threadIdx.x; b0 < total; b0 += U * 256) {
+      float4 v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = b0 + u * 256;
+        if (i < total) v[u] = src[(long long)(i >> 1) * g.kp + (i & 1)];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = b0 + u * 256;
+        if (i < total) {
+          float* d = smem + 4 * (i & 1) * pitch + (i >> 1);
+          d[0] = v[u].x;
+          d[pitch] = v[u].y;
+          d[2 * pitch] = v[u].z;
+          d[3 * pitch] = v[u].w;
+        }
+      }
+    }
+    __syncthreads();
+    line_transform<P>(L, nullptr, 1.f, L, S, g.indx, job.par[gi][warp & 3], tx, T, lane);
+    __syncthreads();
+    for (int r = 0; r < 2; ++r) {
+      float4* d = job.dst[gi] + (long long)(y0 + r) * g.rp;
+      const float* l = smem + 4 * r * pitch;
+      for (int i = threadIdx.x; i <= n; i += 256) {
+        const float4 v = node4(l, pitch, i);
+        d[i] = v;
+        if (y0 + r == 0) job.dst[gi][(long long)g.ny * g.rp + i] = v;  // copyguard
+      }
+    }
+  } else {
+    const int b = (int)blockIdx.x - job.ngroup * pairs, per = g.ny >> 3;
+    const XComp c = job.x.c[b / per];
+    if (c.cursor_stride && !cursor_ok(c, st)) return;
+    xinv_rows<P>(c, 8 * (b % per), g, tx, smem, T, st);
+  }
+  // the zero planes, a share per CTA (planes are multiples of 16 bytes)
+  const long long n4 = g.rplane >> 2, share = (n4 + gridDim.x - 1) / gridDim.x;
+  const long long lo = share * blockIdx.x, hi = min(n4, lo + share);
+  for (int z = 0; z < job.x.nzero; ++z)
+    for (long long i = lo + threadIdx.x; i < hi; i += 256)
+      reinterpret_cast<float4*>(job.x.zero[z])[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// Forward x pass of node-major densities.  A CTA takes one row, its 8 warps
+// the 8 components: the row is one run of 16-byte loads, which the warps
+// spread over 8 shared lines (lane pairs take a node: component 4 h + k of
+// node i goes to bank 16 h + 4 k + i, so no two lanes of a store collide), and
+// a node of the transposed result is one full 32-byte sector -- 5 loads and 5
+// stores of 16 bytes per thread at 512 points, where the planar form loads 8
+// bytes and stores 4 at a time.  Planar components follow, 8 rows per CTA.
+template <int P>
+__global__ void __launch_bounds__(256) k_xfwd8(const __grid_constant__ X8Job job, GridDims g,
+                                               LineTables tx, const DevStatus* st) {
+  extern __shared__ __align__(16) float smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n = g.nx, pitch = line_pitch(n);
+  float* T = smem + line_count(g.indx) * pitch;
+  if (P > 0) stage_lane_table(T, tx);  // constant tables: staged before the wait
+  grid_dep_sync();
+  if (st && st->error) return;
+  if (pass_skipped(st, job.x.pass)) return;
+  if ((int)blockIdx.x >= g.ny) {
+    const int b = (int)blockIdx.x - g.ny, per = (g.ny + 8) >> 3;
+    const XComp c = job.x.c[b / per];
+    if (c.cursor_stride && !cursor_ok(c, st)) return;
+    xfwd_rows<P>(c, 8 * (b % per), g, tx, smem, T, st);
+    return;
+  }
+  const int y = blockIdx.x;
+  stage_lines8<P>(job.src + 2LL * y * g.rp, n, pitch, smem, 256);
+  __syncthreads();
+  float* L = smem + warp * pitch;
+  float* S = smem + (8 + warp) * pitch;
+  line_transform<P>(L, nullptr, 1.f, L, S, g.indx, job.par[warp], tx, T, lane);
+  __syncthreads();
+  float4* d = job.dst + 2LL * y;
+  for (int i = threadIdx.x; i < 2 * (n + 1); i += 256)
+    d[2LL * (i >> 1) * g.kp + (i & 1)] = node4(smem + 4 * (i & 1) * pitch, pitch, i >> 1);
 }
 
 // ------------------------------------------------------------------ y pass
@@ -266,6 +389,10 @@ static int set_smem_limits(int big) {
           cudaSuccess ||
       cudaFuncSetAttribute(k_xinv<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) !=
           cudaSuccess ||
+      cudaFuncSetAttribute(k_xfwd8<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_xinv4<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) !=
+          cudaSuccess ||
       cudaFuncSetAttribute(k_ycol<P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) !=
           cudaSuccess ||
       cudaFuncSetAttribute(k_ycol<P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big) !=
@@ -295,6 +422,18 @@ void launch_xinv(const XJob& job, const GridDims& g, const LineTables& tx, const
                  cudaStream_t s) {
   dim3 grid((g.ny + 1 + 7) / 8, job.ncomp);
   QP_LINE_SWITCH(g.indx, (launch_pdl(k_xinv<P_>, grid, 256, xpass_smem(g), s, job, g, tx, st)));
+}
+
+void launch_xfwd8(const X8Job& job, const GridDims& g, const LineTables& tx, const DevStatus* st,
+                  cudaStream_t s) {
+  const int grid = g.ny + job.x.ncomp * ((g.ny + 8) >> 3);
+  QP_LINE_SWITCH(g.indx, (launch_pdl(k_xfwd8<P_>, grid, 256, xpass_smem(g), s, job, g, tx, st)));
+}
+
+void launch_xinv4(const X4Job& job, const GridDims& g, const LineTables& tx, const DevStatus* st,
+                  cudaStream_t s) {
+  const int grid = job.ngroup * (g.ny >> 1) + job.x.ncomp * (g.ny >> 3);
+  QP_LINE_SWITCH(g.indx, (launch_pdl(k_xinv4<P_>, grid, 256, xpass_smem(g), s, job, g, tx, st)));
 }
 
 void launch_ycol(const YJob& job, const GridDims& g, const LineTables& ty, const DevStatus* st,

@@ -29,6 +29,7 @@ struct XComp {
   int parity;  // 0 sine, 1 cosine
   long long cursor_stride;
   int cursor_planes;  // planes of that 3D array: a cursor outside them raises an error
+  int cursor_next;    // 1: the plane after the cursor (before k_slice_a has moved it on)
 };
 struct XJob {
   XComp c[QP_MAX_JOB];
@@ -57,6 +58,30 @@ void launch_xfwd(const XJob& job, const GridDims& g, const LineTables& tx, const
                  cudaStream_t s);
 void launch_xinv(const XJob& job, const GridDims& g, const LineTables& tx, const DevStatus* st,
                  cudaStream_t s);
+// Inverse x pass of the fused step's node-major fields: group g is
+// src [kx][y][4] -> dst [y][x][4] with the x parities par[g]; planar components
+// (c[0..ncomp), as launch_xinv) ride along, and the launch clears the zero
+// planes of the job.
+struct X4Job {
+  const float4* src[2];
+  float4* dst[2];
+  int par[2][4];
+  int ngroup;
+  XJob x;
+};
+void launch_xinv4(const X4Job& job, const GridDims& g, const LineTables& tx, const DevStatus* st,
+                  cudaStream_t s);
+// Forward x pass of the fused step's node-major densities: src [y][x][8] ->
+// dst [kx][y][8] with the x parities par, rows y < ny (row ny of both stays
+// zero: the deposits fold it onto row 0); planar components ride along.
+struct X8Job {
+  const float4* src;  // two per node
+  float4* dst;
+  int par[8];
+  XJob x;
+};
+void launch_xfwd8(const X8Job& job, const GridDims& g, const LineTables& tx, const DevStatus* st,
+                  cudaStream_t s);
 void launch_ycol(const YJob& job, const GridDims& g, const LineTables& ty, const DevStatus* st,
                  cudaStream_t s);
 

@@ -637,4 +637,38 @@ __device__ __forceinline__ void line_store(float* dst, const float* sline, int n
   if (lane == 0) dst[n] = sline[n] * sc;
 }
 
+// One float4 per node from four shared lines (pitch `pitch`): consecutive
+// threads read consecutive nodes of one line, so no two hit the same bank.
+__device__ __forceinline__ float4 node4(const float* L, int pitch, int i) {
+  return make_float4(L[i], L[pitch + i], L[2 * pitch + i], L[3 * pitch + i]);
+}
+
+// n + 1 nodes of 8 components (two float4 each) into 8 shared lines: every
+// load of a thread before its stores, in batches that cover a 512-point line.
+template <int P>
+__device__ __forceinline__ void stage_lines8(const float4* src, int n, int pitch, float* lines,
+                                             int threads) {
+  constexpr int U = P >= 8 ? 5 : (P == 4 ? 3 : 2);
+  const int total = 2 * (n + 1);
+  for (int b0 = threadIdx.x; b0 < total; b0 += U * threads) {
+    float4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = b0 + u * threads;
+      if (i < total) v[u] = src[i];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = b0 + u * threads;
+      if (i < total) {
+        float* d = lines + 4 * (i & 1) * pitch + (i >> 1);
+        d[0] = v[u].x;
+        d[pitch] = v[u].y;
+        d[2 * pitch] = v[u].z;
+        d[3 * pitch] = v[u].w;
+      }
+    }
+  }
+}
+
 }  // namespace qp

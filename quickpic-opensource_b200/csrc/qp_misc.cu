@@ -167,76 +167,6 @@ __global__ void k_guard_add(Planes3 pl, GridDims g, const DevStatus* st) {
   }
 }
 
-// End of a slice (simulation_class.f03:722-735): the final force
-// fxy = -fxy + (by, -bx), then fxy *= dex -> bexyz(1:2), psit -> bexyz(3),
-// bxyz(1:2) *= dex -> bbxyz, stored at 3D plane `cursor` (0-based; the
-// reference's 1-based slice j+1 for slice j); fxy and bxyz are
-// updated in place as in the reference.
-__global__ void k_store3d(GridDims g, float* fx, float* fy, float* bx, float* by, const float* bz,
-                          const float* psit, Planes3 be, Planes3 bb, float dex, int store,
-                          int nplanes, float* zero_q, DevStatus* st) {
-  grid_dep_sync();
-  if (st->error) return;
-  const int cur = st->cursor;
-  if (store && (cur < 0 || cur >= nplanes)) {  // never store outside the 3D arrays
-    if (threadIdx.x == 0) atomicCAS(&st->error, 0, -7);
-    return;
-  }
-  // four nodes per thread: planes and rows are 16-byte aligned (rp = nx + 4)
-  const long long n4 = g.rplane >> 2;
-  const long long pl4 = (long long)cur * n4;
-  float4* fx4 = reinterpret_cast<float4*>(fx);
-  float4* fy4 = reinterpret_cast<float4*>(fy);
-  float4* bx4 = reinterpret_cast<float4*>(bx);
-  float4* by4 = reinterpret_cast<float4*>(by);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4;
-       i += (long long)gridDim.x * blockDim.x) {
-    // every load of the iteration first, so the thread waits for L2 once
-    const float4 vfx = fx4[i], vfy = fy4[i], vbx = bx4[i], vby = by4[i];
-    float4 vpt = make_float4(0.f, 0.f, 0.f, 0.f), vbz = vpt;
-    if (store) {
-      vpt = reinterpret_cast<const float4*>(psit)[i];
-      vbz = reinterpret_cast<const float4*>(bz)[i];
-    }
-    float4 f1, f2, b1, b2;
-    // f1 = (-fx + by) * dex, f2 = (-fy - bx) * dex; b1 = bx * dex, b2 = by * dex
-    f1.x = (-1.f * vfx.x + vby.x) * dex;
-    f1.y = (-1.f * vfx.y + vby.y) * dex;
-    f1.z = (-1.f * vfx.z + vby.z) * dex;
-    f1.w = (-1.f * vfx.w + vby.w) * dex;
-    f2.x = (-1.f * vfy.x - vbx.x) * dex;
-    f2.y = (-1.f * vfy.y - vbx.y) * dex;
-    f2.z = (-1.f * vfy.z - vbx.z) * dex;
-    f2.w = (-1.f * vfy.w - vbx.w) * dex;
-    b1 = make_float4(vbx.x * dex, vbx.y * dex, vbx.z * dex, vbx.w * dex);
-    b2 = make_float4(vby.x * dex, vby.y * dex, vby.z * dex, vby.w * dex);
-    fx4[i] = f1;
-    fy4[i] = f2;
-    bx4[i] = b1;
-    by4[i] = b2;
-    if (store) {
-      reinterpret_cast<float4*>(be.p[0])[pl4 + i] = f1;
-      reinterpret_cast<float4*>(be.p[1])[pl4 + i] = f2;
-      reinterpret_cast<float4*>(be.p[2])[pl4 + i] = vpt;
-      reinterpret_cast<float4*>(bb.p[0])[pl4 + i] = b1;
-      reinterpret_cast<float4*>(bb.p[1])[pl4 + i] = b2;
-      reinterpret_cast<float4*>(bb.p[2])[pl4 + i] = vbz;
-    }
-    if (zero_q) reinterpret_cast<float4*>(zero_q)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  // the last CTA to finish advances the slice cursor
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    const int done = atomicAdd(&st->store_ctas, 1);
-    if (done == (int)gridDim.x - 1) {
-      st->store_ctas = 0;
-      st->cursor = st->cursor + 1;
-      __threadfence();
-    }
-  }
-}
-
 __global__ void k_cursor(DevStatus* st, int v) {
   grid_dep_sync();
   if (st->error) return;
@@ -316,15 +246,6 @@ void launch_guard_add(float* const* p, int count, const GridDims& g, const DevSt
 
 void launch_cursor(DevStatus* st, int v, cudaStream_t s) {
   launch_pdl(k_cursor, 1, 1, 0, s, st, v);
-}
-
-void launch_store3d(const GridDims& g, float* const* fxy, float* const* bxyz, const float* psit,
-                    const Planes3& be, const Planes3& bb, float dex, int store, int nplanes,
-                    float* zero_q, DevStatus* st, cudaStream_t s) {
-  long long blocks = ((g.rplane >> 2) + 255) / 256;
-  if (blocks > 148 * 8) blocks = 148 * 8;
-  launch_pdl(k_store3d, (int)blocks, 256, 0, s, g, fxy[0], fxy[1], bxyz[0], bxyz[1], bxyz[2],
-             psit, be, bb, dex, store, nplanes, zero_q, st);
 }
 
 }  // namespace qp

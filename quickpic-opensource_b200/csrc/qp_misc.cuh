@@ -84,9 +84,4 @@ void launch_guard_copy(float* const* p, int count, const GridDims& g, const DevS
 void launch_guard_add(float* const* p, int count, const GridDims& g, const DevStatus* st,
                       cudaStream_t s);
 void launch_cursor(DevStatus* st, int v, cudaStream_t s);
-// also clears zero_q (if not null) and advances the slice cursor
-void launch_store3d(const GridDims& g, float* const* fxy, float* const* bxyz, const float* psit,
-                    const Planes3& be, const Planes3& bb, float dex, int store, int nplanes,
-                    float* zero_q, DevStatus* st, cudaStream_t s);
-
 }  // namespace qp

@@ -60,6 +60,81 @@ __device__ __forceinline__ void stage_planes(float (*s)[TN * TN], const float* c
   }
 }
 
+// The force fields of a tile's 17 x 17 nodes in shared memory, interleaved so
+// that a particle reads a corner with one 16-byte and one 8-byte access:
+// consecutive nodes are distinct banks for a warp of cell-ordered particles,
+// and the 6 gathers of 4 corners take 8 load instructions instead of 24.
+struct FieldTile {
+  float4 b[TN * TN];  // psit, bx, by, bz
+  float2 f[TN * TN];  // fx, fy
+};
+
+// All loads of a thread before its first shared-memory store (one wait for L2).
+// psi (optional) is staged beside them.
+template <bool NODE>
+__device__ __forceinline__ void stage_fields(FieldTile& s, float* spsi, const GatherPlanes& f,
+                                             const TileGeom& tg, int noffp, int moffp) {
+  constexpr int PER = (TN * TN + 255) / 256;
+  float4 vb[PER], vf[PER];
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int i = threadIdx.x + 256 * k;
+    const int a = i % TN, b = i / TN;
+    const long long o = (long long)(moffp + b) * tg.rp + noffp + a;
+    vb[k] = vf[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < TN * TN) {
+      if constexpr (NODE) {
+        vb[k] = f.fb[o];
+        vf[k] = f.ff[o];
+      } else {
+        vb[k] = make_float4(f.psit[o], f.bx[o], f.by[o], f.bz[o]);
+        vf[k].x = f.fx[o];
+        vf[k].y = f.fy[o];
+        if (f.psi) vf[k].z = f.psi[o];
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int i = threadIdx.x + 256 * k;
+    if (i < TN * TN) {
+      s.b[i] = vb[k];
+      s.f[i] = make_float2(vf[k].x, vf[k].y);
+      if (spsi) spsi[i] = vf[k].z;
+    }
+  }
+}
+
+// bilinear interpolation of one component from its 4 corner values, in the
+// reference's order of operations
+__device__ __forceinline__ float lerp4(float p00, float p01, float p10, float p11, float amx,
+                                       float amy, float dxp, float dyp) {
+  float d = amx * p00;
+  d = amy * (dxp * p01 + d);
+  const float ac = amx * p10;
+  return d + dyp * (dxp * p11 + ac);
+}
+
+struct Gathered {
+  float psit, bx, by, bz, fx, fy;
+};
+__device__ __forceinline__ Gathered gather6(const FieldTile& s, int nn, int mm, float amx,
+                                            float amy, float dxp, float dyp) {
+  const int o = mm * TN + nn;
+  Gathered g;
+  {
+    const float2 a = s.f[o], b = s.f[o + 1], c = s.f[o + TN], d = s.f[o + TN + 1];
+    g.fx = lerp4(a.x, b.x, c.x, d.x, amx, amy, dxp, dyp);
+    g.fy = lerp4(a.y, b.y, c.y, d.y, amx, amy, dxp, dyp);
+  }
+  const float4 a = s.b[o], b = s.b[o + 1], c = s.b[o + TN], d = s.b[o + TN + 1];
+  g.psit = lerp4(a.x, b.x, c.x, d.x, amx, amy, dxp, dyp);
+  g.bx = lerp4(a.y, b.y, c.y, d.y, amx, amy, dxp, dyp);
+  g.by = lerp4(a.z, b.z, c.z, d.z, amx, amy, dxp, dyp);
+  g.bz = lerp4(a.w, b.w, c.w, d.w, amx, amy, dxp, dyp);
+  return g;
+}
+
 // Add a run's 4 corner charges to the global plane q with L2 reductions
 // (red.global.add.f32), folding the top edge of the top tile row onto row 0.
 __device__ __forceinline__ void deposit_q(float* q, const TileGeom& tg, int noffp, int moffp,
@@ -215,7 +290,7 @@ struct AmjOut {
   float p6;
 };
 
-__device__ __forceinline__ void amjdp_one(float (*sf)[TN * TN], int nn, int mm, float dxp,
+__device__ __forceinline__ void amjdp_one(const FieldTile& sf, int nn, int mm, float dxp,
                                           float dyp, float vx, float vy, float p6, float p7,
                                           float qm, float qbm, float qtmh, float dti, float dex,
                                           float idex, AmjOut* o) {
@@ -225,12 +300,9 @@ __device__ __forceinline__ void amjdp_one(float (*sf)[TN * TN], int nn, int mm, 
   const float inv_part_7 = __frcp_rn(p7);
   const float qtmh1 = qtmh * inv_part_7;
   const float qtmh2 = qtmh1 * p6;
-  float dx = gather(sf[0], nn, mm, amx, amy, dxp, dyp);
-  float dy = gather(sf[1], nn, mm, amx, amy, dxp, dyp);
-  float dz = gather(sf[5], nn, mm, amx, amy, dxp, dyp);
-  float ox = gather(sf[2], nn, mm, amx, amy, dxp, dyp);
-  float oy = gather(sf[3], nn, mm, amx, amy, dxp, dyp);
-  float oz = gather(sf[4], nn, mm, amx, amy, dxp, dyp);
+  const Gathered g = gather6(sf, nn, mm, amx, amy, dxp, dyp);
+  const float dx = g.fx, dy = g.fy;
+  float dz = g.psit, ox = g.bx, oy = g.by, oz = g.bz;
   const float ddx = -1.f * qtmh2 * dx + qtmh * oy;
   const float ddy = -1.f * qtmh2 * dy - qtmh * ox;
   const float acx = vx + ddx, acy = vy + ddy;
@@ -271,23 +343,58 @@ __device__ __forceinline__ void amjdp_one(float (*sf)[TN * TN], int nn, int mm, 
   o->v[7] = v3;
 }
 
-// Add a run's 8 x 4 corner sums to the global planes: fire-and-forget
-// reductions in L2 (red.global.add.f32), native for FP32, where a
-// shared-memory float atomic is a compare-and-swap loop.  The top edge of the
-// top tile row folds onto row 0 (the single-rank guard add, PPNACGUARD2L).
-__device__ __forceinline__ void deposit_run(float* const* pl, const TileGeom& tg, int noffp,
-                                            int moffp, int cell, const float (*acc)[4]) {
-  const int nn = cell % TN, mm = cell / TN;
-  const long long o0 = (long long)(moffp + mm) * tg.rp + noffp + nn;
-  const int y1 = moffp + mm + 1;
-  const long long o2 = (long long)(y1 == tg.ny ? 0 : y1) * tg.rp + noffp + nn;
+// Where amjdp adds its 8 densities: node-major [y][x][8] (node, the fused
+// step) or one plane each.  cz (node form only, optional): the z current also
+// goes to this plane.
+struct Densities {
+  float* node;
+  float* cz;
+  float* pl[8];
+};
+
+__device__ __forceinline__ void red4(float* p, float a, float b, float c, float d) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a),
+               "f"(b), "f"(c), "f"(d)
+               : "memory");
+}
+
+// Add the 8 sums v of one corner to node o: fire-and-forget reductions in L2,
+// native for FP32, where a shared-memory float atomic is a compare-and-swap
+// loop.  A node's 8 densities are one 32-byte sector: two vector reductions
+// from one address in place of eight from eight.
+template <bool NODE>
+__device__ __forceinline__ void add_node(const Densities& d, long long o, const float (&v)[8]) {
+  if constexpr (NODE) {
+    float* p = d.node + 8 * o;
+    red4(p, v[0], v[1], v[2], v[3]);
+    red4(p + 4, v[4], v[5], v[6], v[7]);
+    if (d.cz) atomicAdd(d.cz + o, v[2]);
+  } else {
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    atomicAdd(pl[q] + o0, acc[q][0]);
-    atomicAdd(pl[q] + o0 + 1, acc[q][1]);
-    atomicAdd(pl[q] + o2, acc[q][2]);
-    atomicAdd(pl[q] + o2 + 1, acc[q][3]);
+    for (int q = 0; q < 8; ++q) atomicAdd(d.pl[q] + o, v[q]);
   }
+}
+
+// The left corners' nodes of a cell in the two rows; the top edge of the top
+// tile row folds onto row 0 (the single-rank guard add, PPNACGUARD2L).
+__device__ __forceinline__ void cell_nodes(const TileGeom& tg, int noffp, int moffp, int cell,
+                                           long long* o0, long long* o2) {
+  const int nn = cell % TN, mm = cell / TN;
+  const int y1 = moffp + mm + 1;
+  *o0 = (long long)(moffp + mm) * tg.rp + noffp + nn;
+  *o2 = (long long)(y1 == tg.ny ? 0 : y1) * tg.rp + noffp + nn;
+}
+
+// Add a run's 4 corners x 8 sums to the densities.
+template <bool NODE>
+__device__ __forceinline__ void deposit_run(const Densities& d, const TileGeom& tg, int noffp,
+                                            int moffp, int cell, const float (&acc)[4][8]) {
+  long long o0, o2;
+  cell_nodes(tg, noffp, moffp, cell, &o0, &o2);
+  add_node<NODE>(d, o0, acc[0]);
+  add_node<NODE>(d, o0 + 1, acc[1]);
+  add_node<NODE>(d, o2, acc[2]);
+  add_node<NODE>(d, o2 + 1, acc[3]);
 }
 
 // deposit_run for a lane's last run, merged across lanes: the right corners
@@ -295,30 +402,34 @@ __device__ __forceinline__ void deposit_run(float* const* pl, const TileGeom& tg
 // take is set, and this run's right corners are left to the next lane when
 // give is set.  Every lane of the warp must call it (the shuffles); a lane
 // with no run (cell < 0) only passes values on.
-__device__ __forceinline__ void deposit_last(float* const* pl, const TileGeom& tg, int noffp,
-                                             int moffp, int cell, const float (*acc)[4],
-                                             bool take, bool give) {
+template <bool NODE>
+__device__ __forceinline__ void deposit_last(const Densities& d, const TileGeom& tg, int noffp,
+                                             int moffp, int cell, float (&acc)[4][8], bool take,
+                                             bool give) {
   const unsigned full = 0xffffffffu;
-  const int c = cell < 0 ? 0 : cell;
-  const int nn = c % TN, mm = c / TN;
-  const long long o0 = (long long)(moffp + mm) * tg.rp + noffp + nn;
-  const int y1 = moffp + mm + 1;
-  const long long o2 = (long long)(y1 == tg.ny ? 0 : y1) * tg.rp + noffp + nn;
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
-    const float r1 = __shfl_up_sync(full, acc[q][1], 1);
-    const float r3 = __shfl_up_sync(full, acc[q][3], 1);
-    if (cell >= 0) {
-      atomicAdd(pl[q] + o0, take ? acc[q][0] + r1 : acc[q][0]);
-      atomicAdd(pl[q] + o2, take ? acc[q][2] + r3 : acc[q][2]);
-      if (!give) {
-        atomicAdd(pl[q] + o0 + 1, acc[q][1]);
-        atomicAdd(pl[q] + o2 + 1, acc[q][3]);
-      }
+    const float r1 = __shfl_up_sync(full, acc[1][q], 1);
+    const float r3 = __shfl_up_sync(full, acc[3][q], 1);
+    if (take) {
+      acc[0][q] += r1;
+      acc[2][q] += r3;
     }
+  }
+  if (cell < 0) return;
+  long long o0, o2;
+  cell_nodes(tg, noffp, moffp, cell, &o0, &o2);
+  add_node<NODE>(d, o0, acc[0]);
+  add_node<NODE>(d, o2, acc[2]);
+  if (!give) {
+    add_node<NODE>(d, o0 + 1, acc[1]);
+    add_node<NODE>(d, o2 + 1, acc[3]);
   }
 }
 
+// The half push and the deposit of 8 densities x 4 corners.  Bound by issue
+// (about 380 instructions per particle) and by the reductions in L2, not by
+// memory.
 // Each thread takes 4 consecutive particles (float4 loads of each component)
 // and keeps the deposits of a run of particles in one cell in registers,
 // adding them to the global planes when the cell changes (deposit_run).  With
@@ -326,26 +437,23 @@ __device__ __forceinline__ void deposit_last(float* const* pl, const TileGeom& t
 // reductions spread over neighbouring nodes.  The per-particle products are
 // those of the reference; only the order in which a node's contributions are
 // summed differs.  The planes must be zero on entry.
+template <bool NODE>
 __global__ void __launch_bounds__(256, 3) k_amjdp(PartBuf P, TileGeom tg, GatherPlanes f,
-                                               float* cux, float* cuy, float* cuz, float* dcx,
-                                               float* dcy, float* amxx, float* amyy,
-                                               float* amxy, float qbm, float dt, float dex,
-                                               float scale, DevStatus* st) {
+                                                  const __grid_constant__ Densities den, float qbm,
+                                                  float dt, float dex, float scale,
+                                                  DevStatus* st) {
   grid_dep_sync();
-  __shared__ float sf[7][TN * TN];
+  __shared__ FieldTile sf;
+  __shared__ float spsi[TN * TN];
   if (st && st->error) return;
   if (pass_skipped(st, f.pass)) return;
-  float* const pl[8] = {cux, cuy, cuz, dcx, dcy, amxx, amyy, amxy};
   const int t = blockIdx.x;
   int noffp, moffp;
   tile_origin(tg, t, &noffp, &moffp);
-  const bool ext = f.psi != nullptr;
+  const bool ext = f.ext || f.psi != nullptr;
   // the count is read with the field planes, so the two waits overlap
   const int n = P.count[t];
-  {
-    const float* const planes[7] = {f.fx, f.fy, f.bx, f.by, f.bz, f.psit, f.psi};
-    stage_planes<7>(sf, planes, ext ? 7 : 6, tg, noffp, moffp);
-  }
+  stage_fields<NODE>(sf, ext ? spsi : nullptr, f, tg, noffp, moffp);
   __syncthreads();
   const float qtmh = 0.5f * qbm * dt;
   const float dti = 1.f / dt;
@@ -379,7 +487,7 @@ __global__ void __launch_bounds__(256, 3) k_amjdp(PartBuf P, TileGeom tg, Gather
     float p6s[4] = {P6.x, P6.y, P6.z, P6.w}, p7s[4] = {P7.x, P7.y, P7.z, P7.w};
     const float qms[4] = {QM.x, QM.y, QM.z, QM.w};
     float p6o[4] = {P6.x, P6.y, P6.z, P6.w};
-    float acc[8][4];
+    float acc[4][8];
     int cell = -1;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -394,7 +502,7 @@ __global__ void __launch_bounds__(256, 3) k_amjdp(PartBuf P, TileGeom tg, Gather
         }
         if (ext) {
           // WPGPSIPOST2L_QP for this particle, the same arithmetic as k_extpsi
-          float d = gather(sf[6], nn, mm, 1.f - dxp, 1.f - dyp, dxp, dyp);
+          float d = gather(spsi, nn, mm, 1.f - dxp, 1.f - dyp, dxp, dyp);
           d = -d * dx2 * qbm;
           p7s[j] = 1.f + d;
           p6s[j] = d + (dx2 * (vxs[j] * vxs[j] + vys[j] * vys[j]) - d * d - 2.f * d) /
@@ -413,17 +521,17 @@ __global__ void __launch_bounds__(256, 3) k_amjdp(PartBuf P, TileGeom tg, Gather
         for (int r = 0; r < 4; ++r) ws[r] = o.w[r] * scale;
         const int c = mm * TN + nn;
         if (c != cell) {
-          if (cell >= 0) deposit_run(pl, tg, noffp, moffp, cell, acc);
+          if (cell >= 0) deposit_run<NODE>(den, tg, noffp, moffp, cell, acc);
           cell = c;
 #pragma unroll
-          for (int q = 0; q < 8; ++q)
+          for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int r = 0; r < 4; ++r) acc[q][r] = o.v[q] * ws[r];
+            for (int q = 0; q < 8; ++q) acc[r][q] = o.v[q] * ws[r];
         } else {
 #pragma unroll
-          for (int q = 0; q < 8; ++q)
+          for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int r = 0; r < 4; ++r) acc[q][r] = __fmaf_rn(o.v[q], ws[r], acc[q][r]);
+            for (int q = 0; q < 8; ++q) acc[r][q] = __fmaf_rn(o.v[q], ws[r], acc[r][q]);
         }
       }
     }
@@ -434,7 +542,7 @@ __global__ void __launch_bounds__(256, 3) k_amjdp(PartBuf P, TileGeom tg, Gather
     int cnext = __shfl_down_sync(full, cell, 1);
     if (lane == 0) cprev = -1;
     if (lane == 31) cnext = -1;
-    deposit_last(pl, tg, noffp, moffp, cell, acc, cprev >= 0 && cell == cprev + 1,
+    deposit_last<NODE>(den, tg, noffp, moffp, cell, acc, cprev >= 0 && cell == cprev + 1,
                  cell >= 0 && cnext == cell + 1);
     if (live) {
       P6 = make_float4(p6o[0], p6o[1], p6o[2], p6o[3]);
@@ -467,7 +575,7 @@ __global__ void __launch_bounds__(256) k_push(PartBuf A, PartBuf B, Inbox ib, Ti
   constexpr int CH = MODE != 0 ? PUSH_CHUNK : 1;
   constexpr int NC = MODE != 0 ? 256 : 1;
   constexpr int NR = MODE != 0 ? CH / 256 : 1;  // rounds of 256 slots per chunk
-  __shared__ float sf[6][TN * TN];
+  __shared__ FieldTile sf;
   __shared__ float stg[NCOMP][CH];      // the chunk's stayers, by chunk slot
   __shared__ short perm[CH];            // output order -> chunk slot
   __shared__ unsigned char wcnt[8][NC];  // per warp: its stayers of each cell so far
@@ -489,15 +597,42 @@ __global__ void __launch_bounds__(256) k_push(PartBuf A, PartBuf B, Inbox ib, Ti
       f.zero_q[(long long)(moffp + i / w) * tg.rp + noffp + i % w] = 0.f;
   }
   if (MODE != 2) {
-    const float* const planes[6] = {f.fx, f.fy, f.bx, f.by, f.bz, f.psit};
-    stage_planes<6>(sf, planes, 6, tg, noffp, moffp);
+    if (f.fb)
+      stage_fields<true>(sf, nullptr, f, tg, noffp, moffp);
+    else
+      stage_fields<false>(sf, nullptr, f, tg, noffp, moffp);
     __syncthreads();
     if (f.combine) {
-      // the slice's final force: fxy = -fxy + (bxyz(2), -bxyz(1)), simulation_class.f03:722-724
+      long long so = 0;
+      if (f.be[0] && f.store_planes) {
+        const int cur = st->cursor;
+        if (cur < 0 || cur >= f.store_planes) {  // never store outside the 3D arrays
+          if (threadIdx.x == 0) raise_error(st, -7);
+          return;
+        }
+        so = cur * f.store_stride;
+      }
+      // the slice's final force: fxy = -fxy + (bxyz(2), -bxyz(1)), simulation_class.f03:722-724;
+      // and the slice's stores (727-735): fxy dex and psit, bxy dex and bz.  The
+      // nodes are already here, so the stores cost 6 coalesced 64-byte writes per
+      // tile row where a kernel of its own read 6 planes, wrote 10 and was a launch
+      const int x1 = noffp + TILE >= tg.nx ? TN : TILE, y1 = moffp + TILE >= tg.ny ? TN : TILE;
       for (int i = threadIdx.x; i < TN * TN; i += blockDim.x) {
-        const float fx = -1.f * sf[0][i], fy = -1.f * sf[1][i];
-        sf[0][i] = fx + sf[3][i];
-        sf[1][i] = fy - sf[2][i];
+        const float4 b = sf.b[i];
+        const float2 v = sf.f[i];
+        const float fx = -1.f * v.x, fy = -1.f * v.y;
+        const float gx = fx + b.z, gy = fy - b.y;
+        sf.f[i] = make_float2(gx, gy);
+        const int nx = i % TN, ny = i / TN;
+        if (f.be[0] && nx < x1 && ny < y1) {  // every node is stored by one tile
+          const long long o = so + (long long)(moffp + ny) * tg.rp + noffp + nx;
+          f.be[0][o] = gx * dex;
+          f.be[1][o] = gy * dex;
+          f.be[2][o] = b.x;
+          f.bb[0][o] = b.y * dex;
+          f.bb[1][o] = b.z * dex;
+          f.bb[2][o] = b.w;
+        }
       }
     }
   }
@@ -565,13 +700,11 @@ __global__ void __launch_bounds__(256) k_push(PartBuf A, PartBuf B, Inbox ib, Ti
           mm = 0;
         }
         const float amx = 1.f - dxp, amy = 1.f - dyp;
-        float dx = gather(sf[0], nn, mm, amx, amy, dxp, dyp);
-        float dy = gather(sf[1], nn, mm, amx, amy, dxp, dyp);
-        float dz = gather(sf[5], nn, mm, amx, amy, dxp, dyp);
+        const Gathered g = gather6(sf, nn, mm, amx, amy, dxp, dyp);
+        float dx = g.fx, dy = g.fy, dz = g.psit;
         dz = dz * idex;
-        float ox = gather(sf[2], nn, mm, amx, amy, dxp, dyp);
-        float oy = gather(sf[3], nn, mm, amx, amy, dxp, dyp);
-        const float oz = gather(sf[4], nn, mm, amx, amy, dxp, dyp);
+        float ox = g.bx, oy = g.by;
+        const float oz = g.bz;
         ox = ox * dex;
         oy = oy * dex;
         dx = qtmh2 * dx;
@@ -811,7 +944,9 @@ __global__ void __launch_bounds__(256) k_insert(PartBuf B, Inbox ib, TileGeom tg
 // write of the live buffer, component blockIdx.y, four slots per thread (in
 // place of a fill, a strided copy per component and a scaling pass over q).
 // Both capacities are multiples of 4, so a float4 never spans two tiles.
-__global__ void __launch_bounds__(256) k_renew(PartBuf P0, PartBuf A, int ntiles, float qm) {
+__global__ void __launch_bounds__(256) k_renew(const __grid_constant__ PartBuf P0,
+                                               const __grid_constant__ PartBuf A, int ntiles,
+                                               float qm) {
   grid_dep_sync();
   const int c = blockIdx.y;
   const int na = A.cap >> 2, np = P0.cap >> 2;
@@ -867,8 +1002,20 @@ void launch_extpsi(const PartBuf& P, const TileGeom& tg, const float* psi, float
 void launch_amjdp(const PartBuf& P, const TileGeom& tg, const GatherPlanes& f, float* const* acc,
                   float qbm, float dt, float dex, float scale, const DevStatus* st,
                   cudaStream_t s) {
-  launch_pdl(k_amjdp, tg.ntiles, 256, 0, s, P, tg, f, acc[0], acc[1], acc[2], acc[3], acc[4],
-             acc[5], acc[6], acc[7], qbm, dt, dex, scale, const_cast<DevStatus*>(st));
+  Densities d{};
+  for (int i = 0; i < 8; ++i) d.pl[i] = acc[i];
+  launch_pdl(k_amjdp<false>, tg.ntiles, 256, 0, s, P, tg, f, d, qbm, dt, dex, scale,
+             const_cast<DevStatus*>(st));
+}
+
+void launch_amjdp_node(const PartBuf& P, const TileGeom& tg, const GatherPlanes& f, float* node,
+                       float* cz, float qbm, float dt, float dex, float scale,
+                       const DevStatus* st, cudaStream_t s) {
+  Densities d{};
+  d.node = node;
+  d.cz = cz;
+  launch_pdl(k_amjdp<true>, tg.ntiles, 256, 0, s, P, tg, f, d, qbm, dt, dex, scale,
+             const_cast<DevStatus*>(st));
 }
 
 void launch_push(int mode, const PartBuf& A, const PartBuf& B, const Inbox& ib,

@@ -30,8 +30,11 @@ struct TileGeom {
   int rp;
 };
 
-// field planes a particle kernel gathers from (real space)
+// field planes a particle kernel gathers from (real space): node-major
+// (fb, ff; the fused step) or, with fb null, one plane per component
 struct GatherPlanes {
+  const float4* fb;  // (psit, bx, by, bz)
+  const float4* ff;  // (fx, fy, psi, unused)
   const float* fx;   // fxy(1)
   const float* fy;   // fxy(2)
   const float* bx;   // bxyz(1)
@@ -40,9 +43,17 @@ struct GatherPlanes {
   const float* psit; // psit
   int combine;       // 1: the push uses -fxy + (by, -bx), the final slice force
   const float* psi;  // amjdp only, optional: form p6, p7 from psi first (extpsi)
+  int ext;           // amjdp only: the same with psi from ff
   int pass;          // amjdp only: predictor-corrector pass (pass_skipped), 0 = none
   float* zero_q;     // push only, optional: clear the charge-plane nodes this tile
                      // owns (k_insert then deposits the next slice's charge)
+  // push with combine only, optional: the slice's fields go to these planes --
+  // fxy dex and psit to be, bxy dex and bz to bb -- at plane `cursor` of stacks
+  // of store_planes (0: at the pointers themselves)
+  float* be[3];
+  float* bb[3];
+  long long store_stride;
+  int store_planes;
 };
 
 int part_kernels_init();
@@ -55,6 +66,11 @@ void launch_extpsi(const PartBuf& P, const TileGeom& tg, const float* psi, float
 void launch_amjdp(const PartBuf& P, const TileGeom& tg, const GatherPlanes& f, float* const* acc,
                   float qbm, float dt, float dex, float scale, const DevStatus* st,
                   cudaStream_t s);
+// the same into node-major densities node[y][x][8] (cu x/y/z, dcu x/y, amu
+// xx/yy/xy), from node-major fields; cz (optional) also takes the z current
+void launch_amjdp_node(const PartBuf& P, const TileGeom& tg, const GatherPlanes& f, float* node,
+                       float* cz, float qbm, float dt, float dex, float scale,
+                       const DevStatus* st, cudaStream_t s);
 // mode 0: push in place (partpush); 1: push A -> B with re-binning (push + pmove);
 // 2: re-bin only (pmove) A -> B
 void launch_push(int mode, const PartBuf& A, const PartBuf& B, const Inbox& ib,

@@ -53,9 +53,12 @@ __global__ void __launch_bounds__(256) k_slice_a(SliceA a, GridDims g, KCoef K, 
     reg_line_load<(P > 0 ? P : 1)>((warp == 0 ? a.qe : a.qb) + co, nullptr, a.norm, r, lane);
   const StatusSnap sn = status_snap(st);
   if (sn.error) return;
-  // a new slice: no pass of it has converged yet (the passes follow this kernel)
+  // a new slice: the cursor moves on to it (no other CTA of this kernel reads
+  // the cursor, the x pass before it reads the plane after the cursor), and no
+  // pass of it has converged yet (the passes follow this kernel)
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     DevStatus* ws = const_cast<DevStatus*>(st);
+    ws->cursor = sn.cursor + 1;
     ws->pass_done = 0;
     ws->resid_hist[0] = ws->resid_hist[1] = 1e30f;
   }
@@ -125,19 +128,13 @@ __global__ void __launch_bounds__(256) k_slice_a(SliceA a, GridDims g, KCoef K, 
   __syncthreads();
   // phase 3: inverse y; y parities: psi S, fx S, fy C, psit S, bx C, by S, bz C
   if (warp != 1) {
-    float* dst;
-    int par;
-    switch (warp) {
-      case 0: dst = a.out_bz; par = 1; break;
-      case 2: dst = a.out_psi; par = 0; break;
-      case 3: dst = a.out_fx; par = 0; break;
-      case 4: dst = a.out_fy; par = 1; break;
-      case 5: dst = a.out_psit; par = 0; break;
-      case 6: dst = a.out_bx; par = 1; break;
-      default: dst = a.out_by; par = 0; break;
-    }
+    const int par = (warp == 0 || warp == 4 || warp == 6) ? 1 : 0;
     line_transform<P>(L, nullptr, 1.f, L, S, g.indy, par, ty, T, lane);
-    line_store(dst + co, L, n, 1.f, lane);
+  }
+  __syncthreads();
+  for (int y = threadIdx.x; y <= n; y += blockDim.x) {
+    a.out_b[co + y] = make_float4(line[5][y], line[6][y], line[7][y], line[0][y]);
+    a.out_f[co + y] = make_float4(line[3][y], line[4][y], line[2][y], 0.f);
   }
 }
 
@@ -161,11 +158,13 @@ __global__ void __launch_bounds__(288) k_slice_b(SliceB b, GridDims g, KCoef K, 
   grid_dep_sync();
   if (st->error) return;
   if (pass_skipped(st, b.pass)) return;
-  if (P > 0) __syncthreads();
+  // the column's 8 components into the shared lines, then
   // phase 1: forward y of cu(3), dcu(2), amu(3): y parities S C S, S C, S S C
+  stage_lines8<P>(b.in + 2 * co, n, pitch, smem, 288);
+  __syncthreads();
   if (warp < 8) {
     const int par = (warp == 1 || warp == 4 || warp == 7) ? 1 : 0;
-    line_transform<P>(b.in[warp] + co, nullptr, b.norm, L, S, g.indy, par, ty, T, lane);
+    line_transform<P>(L, nullptr, b.norm, L, S, g.indy, par, ty, T, lane);
   } else if (b.q_in) {
     line_transform<P>(b.q_in + co, nullptr, b.norm, L, S, g.indy, 0, ty, T, lane);
   }
@@ -198,7 +197,8 @@ __global__ void __launch_bounds__(288) k_slice_b(SliceB b, GridDims g, KCoef K, 
     line[1][ky] = bx;
     line[2][ky] = by;
     line[3][ky] = bz;
-    if (b.q_in) line[8][ky] = k_smooth(K, kx, ky, line[8][ky]);
+    // the transform is linear: q + cu_z is formed here
+    if (b.q_in) line[8][ky] = k_smooth(K, kx, ky, QA(line[8][ky], cz));
     if (b.vpot_out[0]) {
       float ax, ay, az;
       k_vpot(K, kx, ky, cx, cy, cz, &ax, &ay, &az);
@@ -258,7 +258,6 @@ __global__ void __launch_bounds__(288) k_slice_b(SliceB b, GridDims g, KCoef K, 
   if (warp < 4) {
     const int par = (warp == 1 || warp == 3) ? 1 : 0;
     line_transform<P>(L, nullptr, 1.f, L, S, g.indy, par, ty, T, lane);
-    line_store(b.out[warp] + co, L, n, 1.f, lane);
   } else if (warp == 8) {
     if (b.q_in) {
       line_transform<P>(L, nullptr, 1.f, L, S, g.indy, 0, ty, T, lane);
@@ -267,11 +266,15 @@ __global__ void __launch_bounds__(288) k_slice_b(SliceB b, GridDims g, KCoef K, 
   } else if (b.nzero) {
     // zero the real-space accumulators for the next pass (their values were
     // consumed by the x pass that precedes this kernel)
-    const long long per = (g.rplane + gridDim.x - 1) / gridDim.x;
-    const long long lo = per * kx, hi = min(g.rplane, lo + per);
+    const long long n4 = g.rplane >> 2, per = (n4 + gridDim.x - 1) / gridDim.x;
+    const long long lo = per * kx, hi = min(n4, lo + per);
     for (int z = 0; z < b.nzero; ++z)
-      for (long long i = lo + (threadIdx.x - 128); i < hi; i += 128) b.zero[z][i] = 0.f;
+      for (long long i = lo + (threadIdx.x - 128); i < hi; i += 128)
+        reinterpret_cast<float4*>(b.zero[z])[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
+  __syncthreads();
+  for (int y = threadIdx.x; y <= n; y += blockDim.x)
+    b.out[co + y] = make_float4(line[0][y], line[1][y], line[2][y], line[3][y]);
 }
 
 }  // namespace

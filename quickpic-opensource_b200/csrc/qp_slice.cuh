@@ -8,7 +8,8 @@ namespace qp {
 
 // Slice start.  qe, qb: x-transformed columns ([kx][y]); cu_*: the extrapolated
 // Fourier-space current of the previous slice; epw_*: B_perp of the previous
-// slice; epwb_*: out, beam E_perp; out_*: y-inverse columns for the x pass.
+// slice; epwb_*: out, beam E_perp; out_*: y-inverse columns [kx][y][4] for the x
+// pass.
 struct SliceA {
   const float* qe;
   const float* qb;  // null without beams
@@ -20,20 +21,21 @@ struct SliceA {
   float *epw_prev_x, *epw_prev_y;
   float *epw_prev2_x, *epw_prev2_y;  // quadratic predictor only
   float *epwb_x, *epwb_y;
-  float *out_psi, *out_fx, *out_fy, *out_psit, *out_bx, *out_by, *out_bz;
+  float4* out_b;  // (psit, bx, by, bz) of every node of the column
+  float4* out_f;  // (fx, fy, psi, 0)
   float norm, dex;
 };
 
-// One predictor-corrector pass.  in[0..7]: x-transformed cu(3), dcu(2),
-// amu(3); the Fourier-space cu is written back extrapolated to cu_*; epw_* is
-// read and updated; out[0..3]: y-inverse columns of psit, bx, by, bz.
+// One predictor-corrector pass.  in: x-transformed cu(3), dcu(2), amu(3),
+// [kx][y][8]; the Fourier-space cu is written back extrapolated to cu_*; epw_* is
+// read and updated; out: y-inverse columns (psit, bx, by, bz), [kx][y][4].
 struct SliceB {
-  const float* in[8];
+  const float4* in;  // [kx][y][8]
   float *cu_x, *cu_y, *cu_z;
   float *epw_x, *epw_y;
   const float *epwb_x, *epwb_y;
-  float* out[4];
-  const float* q_in;  // optional x-transformed q + cu_z (species2d%cbq)
+  float4* out;
+  const float* q_in;  // optional x-transformed q (species2d%cbq smooths q + cu_z)
   float* q_out;
   float* vpot_out[3];  // optional: the vector potential of the pass's current (Fourier space)
   float* zero[8];     // real-space planes to clear for the next pass
