@@ -28,16 +28,20 @@
 // K-major layout.  One thread issues the 9*Cin/16 MMAs (M=128, N=Cout, K=16)
 // into a 32-column TMEM accumulator, commits them to an mbarrier, and the four
 // warps read their 32 TMEM lanes back (tcgen05.ld 32x32b) for the epilogue.
-// The halo of the CTA's next tile is loaded while the current one is computed.
+// Two halo buffers and two accumulators: the copies and MMAs of the CTA's next
+// tiles run while the current one is written out, one barrier per tile.
 //
 // Weight gradient: dW[tap][cin][cout] = sum_px X[px + shift(tap)][cin] dY[px][cout],
-// per tap a GEMM with M = cout, N = cin, K = pixels.  The reduction runs over
-// pixels, so the threads first rewrite the TMA-loaded tiles as K-major
-// operands (8 consecutive pixels of one channel in 16 bytes): dY as
-// A[cout][pixels] and, for each of the 9 taps, the shifted window of X as
-// B[cin][pixels].  M is padded to 128 (rows >= cout are zeros and are
-// discarded); the 9 taps accumulate in 9 * cin TMEM columns over every tile of
-// the CTA, and are added to the FP32 gradient once at the end.
+// a GEMM with K = pixels whose operands are the TMA tiles as they land: 8
+// channels of a pixel are 16 contiguous bytes and 8 pixels of a channel group
+// are one core matrix of an MN-major operand.  In the halo [G][3 rows][130][8]
+// the (group, row) pairs follow one another at one stride, so a single operand
+// covers M = (group, dy, channel) -- the 3 row shifts of every input channel --
+// and the 3 column shifts dx are three start addresses 16 bytes apart: 24 MMAs
+// (M=128, N=cout, K=16) per tile of 128 pixels.  A block of ones behind the
+// halo is the next (group, row): its row of the product is the bias gradient.
+// The accumulators (3 x cout TMEM columns) run over every tile of the CTA and
+// are added to the FP32 gradient once at the end.
 //
 // Every wait on an mbarrier is bounded (about 1 s of %globaltimer); on expiry
 // the kernel records an error, waits (bounded) for its own copies and MMAs in
@@ -251,21 +255,19 @@ __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtenso
   extern __shared__ __align__(128) unsigned char sm[];
   unsigned char* wsm = sm;
   unsigned char* halo[2] = {sm + WBYTES, sm + WBYTES + HB};
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + WBYTES + 2 * HB);  // [0,1] tma, [2] mma
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 3);
-  int* s_err = reinterpret_cast<int*>(tslot + 1);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + WBYTES + 2 * HB);  // [0,1] tma, [2,3] mma
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 4);
+  float* sbias = reinterpret_cast<float*>(bar + 6);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int segs = a.W / TM;
   const int ntiles = a.NB * a.H * segs;
 
   if (tid == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    mbar_init(&bar[2], 1);
-    *s_err = 0;
+    for (int i = 0; i < 4; ++i) mbar_init(&bar[i], 1);
     fence_barrier_init();
   }
-  if (warp == 0) tmem_alloc(tslot, 32);
+  if (warp == 0) tmem_alloc(tslot, 64);  // two accumulators of 32 columns
+  if (tid < COUT) sbias[tid] = a.bias ? a.bias[tid] : 0.f;
   // weights: global image of the shared layout, 16 bytes per thread and step
   {
     const uint4* src = reinterpret_cast<const uint4*>(a.w);
@@ -292,51 +294,57 @@ __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtenso
     tma_load5(halo[buf], &tin, &bar[buf], x0 - 1, y - 1, a.b0 + b);
   };
 
-  int k = 0;
-  // thread 0's record of what it has in flight, for the error path
-  int pf_buf = -1, pf_k = 0;    // a prefetch not yet waited for: buffer and tile number
-  bool mma_out = false;         // MMAs committed and not yet seen complete
+  // Tile k of this CTA: halo buffer and accumulator k & 1.  While the warps
+  // write tile k out, tile k + 1's MMAs run and tile k + 2's halo is on its way.
+  // Thread 0 keeps what it has in flight, for the error path.
+  int pf_k = -1;   // the last tile whose copy has been issued
+  int mma_k = -1;  // the last tile whose MMAs have been committed
+  auto start = [&](int k) {  // thread 0: tile k's MMAs, once its halo has landed
+    const int buf = k & 1;
+    // false: the halo never arrived, no MMA issued for this tile
+    if (!mbar_wait(&bar[buf], (uint32_t)((k >> 1) & 1))) return false;
+    tc_after();
+    const uint32_t hbase = su32(halo[buf]), wbase = su32(wsm);
+#pragma unroll 1
+    for (int s = 0; s < KSTEPS; ++s) {
+      const int tap = s / (CIN / 16), h = s - tap * (CIN / 16);
+      const int dy = tap / 3, dx = tap - dy * 3;
+      const uint32_t aa = hbase + (uint32_t)(2 * h * HALO_G + (dy * HW_ + dx) * 16);
+      const uint64_t ad = sdesc(aa, HALO_G, 128);
+      const uint64_t bd = sdesc(wbase + (uint32_t)(2 * s) * LBO_B, LBO_B, 128);
+      mma_bf16(tbase + 32u * (uint32_t)buf, ad, bd, IDESC, s > 0 ? 1u : 0u);
+    }
+    mma_commit(&bar[2 + buf]);
+    mma_k = k;
+    return true;
+  };
+  const int step = (int)gridDim.x;
+  bool bad = false;
   if (tid == 0 && (int)blockIdx.x < ntiles) {
     issue(blockIdx.x, 0);
-    pf_buf = 0;
     pf_k = 0;
-  }
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++k) {
-    const int buf = k & 1;
-    if (tid == 0) {
-      const int tn = t + gridDim.x;
-      if (mbar_wait(&bar[buf], (uint32_t)((k >> 1) & 1))) {
-        pf_buf = -1;
-        if (tn < ntiles) {  // the other buffer was freed by the previous tile's MMAs
-          issue(tn, buf ^ 1);
-          pf_buf = buf ^ 1;
-          pf_k = k + 1;
-        }
-        tc_after();
-        const uint32_t hbase = su32(halo[buf]);
-        const uint32_t wbase = su32(wsm);
-#pragma unroll 1
-        for (int s = 0; s < KSTEPS; ++s) {
-          const int tap = s / (CIN / 16), h = s - tap * (CIN / 16);
-          const int dy = tap / 3, dx = tap - dy * 3;
-          const uint32_t aa = hbase + (uint32_t)(2 * h * HALO_G + (dy * HW_ + dx) * 16);
-          const uint64_t ad = sdesc(aa, HALO_G, 128);
-          const uint64_t bd = sdesc(wbase + (uint32_t)(2 * s) * LBO_B, LBO_B, 128);
-          mma_bf16(tbase, ad, bd, IDESC, s > 0 ? 1u : 0u);
-        }
-        mma_commit(&bar[2]);
-        mma_out = true;
-      } else {
-        *s_err = 1;  // the halo never arrived: no MMA issued for this tile
-      }
+    if ((int)blockIdx.x + step < ntiles) {
+      issue(blockIdx.x + step, 1);
+      pf_k = 1;
     }
-    __syncthreads();
-    if (*s_err) break;
+    bad = !start(0);
+  }
+  // a wait that expired in any thread ends the loop for all of them
+  bool failed = __syncthreads_or(bad) != 0;
+  int k = 0;
+  for (int t = blockIdx.x; t < ntiles && !failed; t += step, ++k) {
+    const int buf = k & 1;
     // every thread waits for the accumulator (bounded)
-    if (!mbar_wait(&bar[2], (uint32_t)(k & 1))) atomicExch(s_err, 1);
-    __syncthreads();
-    if (*s_err) break;
-    if (tid == 0) mma_out = false;
+    bad = !mbar_wait(&bar[2 + buf], (uint32_t)((k >> 1) & 1));
+    if (tid == 0 && !bad) {
+      if (t + 2 * step < ntiles) {  // tile k's MMAs are done with its halo
+        issue(t + 2 * step, buf);
+        pf_k = k + 2;
+      }
+      // its accumulator was read before the last barrier
+      if (t + step < ntiles) bad = !start(k + 1);
+    }
+    __syncwarp();  // the tensor-memory loads are warp-synchronous
     tc_after();
     int b, y, x0;
     tile_coord(t, b, y, x0);
@@ -344,7 +352,7 @@ __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtenso
     float acc[32];
     {
       uint32_t r[16];
-      const uint32_t ta = tbase + ((uint32_t)(warp * 32) << 16);
+      const uint32_t ta = tbase + ((uint32_t)(warp * 32) << 16) + 32u * (uint32_t)buf;
       QP_TLD16(r, ta);
 #pragma unroll
       for (int i = 0; i < 16; ++i) acc[i] = __uint_as_float(r[i]);
@@ -361,7 +369,7 @@ __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtenso
         const size_t o = ((((size_t)g * a.NB + b) * a.H + y) * a.W + x) * 8;
         float v[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = acc[8 * g + i] + (a.bias ? a.bias[8 * g + i] : 0.f);
+        for (int i = 0; i < 8; ++i) v[i] = acc[8 * g + i] + sbias[8 * g + i];
         if (EPI == EPI_RELU) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) v[i] = fmaxf(v[i], 0.f);
@@ -382,7 +390,7 @@ __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtenso
 #pragma unroll
       for (int c = 0; c < NN_OUT; ++c)
         a.out32[(((size_t)b * NN_OUT + c) * a.H + y) * a.W + x] =
-            acc[c] + (a.bias ? a.bias[c] : 0.f);
+            acc[c] + sbias[c];
     } else {  // EPI_EPW: pixel (y, x) = mode (kx, ky); start of the slice's passes
       const int kx = y, ky = x;
       const size_t o = (size_t)kx * a.kp + ky;
@@ -396,25 +404,26 @@ __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtenso
       a.pl.prev_y[o] = e1y;
       float px = nn_base(e1x, e0x, emx), py = nn_base(e1y, e0y, emy);
       if (kx >= 1 && ky >= 1) {  // the modes kx = 0, ky = 0 take the extrapolation alone
-        px += nn_bounded(sB * (acc[0] + a.bias[0]), px - e1x, e1x);
-        py += nn_bounded(sB * (acc[1] + a.bias[1]), py - e1y, e1y);
+        px += nn_bounded(sB * (acc[0] + sbias[0]), px - e1x, e1x);
+        py += nn_bounded(sB * (acc[1] + sbias[1]), py - e1y, e1y);
       }
       a.pl.epw_x[o] = px;
       a.pl.epw_y[o] = py;
     }
     tc_before();
-    __syncthreads();
+    failed = __syncthreads_or(bad) != 0;
   }
-  if (tid == 0 && *s_err) {
+  if (tid == 0 && failed) {
     // let this CTA's own copies and MMAs in flight land before its shared and
     // tensor memory are released (each wait bounded again)
-    if (pf_buf >= 0) mbar_wait(&bar[pf_buf], (uint32_t)((pf_k >> 1) & 1));
-    if (mma_out) mbar_wait(&bar[2], (uint32_t)(k & 1));
+    for (int j = max(0, pf_k - 1); j <= pf_k; ++j) mbar_wait(&bar[j & 1], (uint32_t)((j >> 1) & 1));
+    for (int j = max(0, mma_k - 1); j <= mma_k; ++j)
+      mbar_wait(&bar[2 + (j & 1)], (uint32_t)((j >> 1) & 1));
     flag_error(a.err, 1);
   }
   // EPI_EPW: the modes outside the conv image (the network's low-mode window)
   // take the quadratic extrapolation alone, spread over every CTA
-  if (EPI == EPI_EPW && !*s_err) {
+  if (EPI == EPI_EPW && !failed) {
     const long long nm = (long long)(a.nx + 1) * (a.ny + 1);
     for (long long i = (long long)blockIdx.x * 128 + tid; i < nm; i += (long long)gridDim.x * 128) {
       const int kx = (int)(i / (a.ny + 1)), ky = (int)(i - (long long)kx * (a.ny + 1));
@@ -432,7 +441,7 @@ __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtenso
     }
   }
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tbase, 32);
+  if (warp == 0) tmem_dealloc(tbase, 64);
 }
 
 
@@ -440,46 +449,58 @@ __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtenso
 struct WgradArgs {
   float* dw;        // [9][CIN][COUT] fp32, accumulated
   float* db;        // [COUT] fp32, accumulated
-  const __nv_bfloat16* dy;  // the tile's dY (for the bias sums through shared memory)
   int couts;        // output channels that exist (the rest are padding)
   int H, W, NB;     // dY images
   int xb0;          // first image of the launch in the X map
   int* err;
 };
 
+constexpr int WG_STAGES = 3;
+constexpr int WG_ROW = HW_ * 16;  // bytes of a halo row: the M-direction core-matrix stride
+// byte offsets within a stage: halo, ones, dY (TMA destinations 128-byte aligned)
+constexpr int wg_dy_off(int cin) { return ((cin / 8) * HALO_G + WG_ROW + 127) & ~127; }
+constexpr int wg_stage(int cin, int cout) { return wg_dy_off(cin) + (cout / 8) * TM * 16; }
+// M = 128 reads 16 rows of 2080 bytes from a stage's start (plus the shift dx),
+// whatever the stage holds: rows past the ones are discarded, but the bytes
+// have to be there behind the last stage too
+constexpr int wg_tail(int cin, int cout) {
+  const int need = 16 * WG_ROW + 64, st = wg_stage(cin, cout);
+  return need > st ? ((need - st + 127) & ~127) : 0;
+}
+
+// Bound by the tiles' way from L2 (a halo is 3 times its pixels): 33 KB per
+// tile of 128 pixels, three tiles in flight per CTA, two CTAs per SM.
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(128) k_wgrad(const __grid_constant__ CUtensorMap tx,
                                                const __grid_constant__ CUtensorMap tdy,
                                                WgradArgs a) {
-  constexpr int GIN = CIN / 8, GOUT = COUT / 8;
+  constexpr int GIN = CIN / 8, GOUT = COUT / 8, NS = WG_STAGES;
   constexpr int HALO_BYTES = GIN * HALO_G;
-  constexpr int DY_BYTES = GOUT * TM * 16;
-  constexpr int DY_OFF = (HALO_BYTES + 127) & ~127;               // TMA destinations 128-aligned
-  constexpr int STG = ((DY_OFF + DY_BYTES) + 127) & ~127;        // one staging buffer
-  constexpr int AT_BYTES = (TM / 8) * 128 * 16;                 // [16 pixel groups][128 rows][8]
-  constexpr int XT_ONE = (TM / 8) * CIN * 16;                   // [16 pixel groups][CIN][8]
-  constexpr uint32_t TCOLS = CIN == 32 ? 512 : 256;
-  constexpr uint32_t IDESC = idesc_bf16(128, CIN, 0, 0);
+  constexpr int DY_OFF = wg_dy_off(CIN);
+  constexpr int STG = wg_stage(CIN, COUT);
+  constexpr uint32_t TCOLS = 3 * COUT <= 64 ? 64 : 128;
+  constexpr uint32_t IDESC = idesc_bf16(128, COUT, 1, 1);
   extern __shared__ __align__(128) unsigned char sm[];
-  unsigned char* stg[2] = {sm, sm + STG};
-  unsigned char* at = sm + 2 * STG;
-  unsigned char* xt = at + AT_BYTES;  // 9 copies, (dx, dy) major
-  uint64_t* bar = reinterpret_cast<uint64_t*>(xt + 9 * XT_ONE);  // [0,1] tma, [2] mma
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 3);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + NS * STG + wg_tail(CIN, COUT));
+  uint64_t* full = bar;        // [NS] the tile has landed
+  uint64_t* empty = bar + NS;  // [NS] the tile's MMAs are done
+  uint64_t* done = bar + 2 * NS;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
   int* s_err = reinterpret_cast<int*>(tslot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int segs = a.W / TM;
   const int ntiles = a.NB * a.H * segs;
 
   if (tid == 0) {
-    for (int i = 0; i < 3; ++i) mbar_init(&bar[i], 1);
+    for (int i = 0; i < 2 * NS + 1; ++i) mbar_init(&bar[i], 1);
     *s_err = 0;
     fence_barrier_init();
   }
   if (warp == 0) tmem_alloc(tslot, TCOLS);
-  {  // the rows of the A operand past the real output channels stay zero
-    uint4* z = reinterpret_cast<uint4*>(at);
-    for (int i = tid; i < AT_BYTES / 16; i += 128) z[i] = make_uint4(0, 0, 0, 0);
+  for (int i = tid; i < NS * (WG_ROW / 16); i += 128) {  // bf16 ones behind every halo
+    const int st = i / (WG_ROW / 16), p = i - st * (WG_ROW / 16);
+    *reinterpret_cast<uint4*>(sm + st * STG + HALO_BYTES + p * 16) =
+        make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
   }
   fence_async_smem();
   tc_before();
@@ -487,133 +508,92 @@ __global__ void __launch_bounds__(128) k_wgrad(const __grid_constant__ CUtensorM
   tc_after();
   const uint32_t tbase = *tslot;
 
-  auto tile_coord = [&](int t, int& b, int& y, int& x0) {
-    const int per = a.H * segs;
-    b = t / per;
-    const int r = t - b * per;
-    y = r / segs;
-    x0 = (r - y * segs) * TM;
-  };
-  auto issue = [&](int t, int buf) {
-    int b, y, x0;
-    tile_coord(t, b, y, x0);
-    mbar_expect_tx(&bar[buf], (uint32_t)(HALO_BYTES + DY_BYTES));
-    tma_load5(stg[buf], &tx, &bar[buf], x0 - 1, y - 1, a.xb0 + b);
-    tma_load5(stg[buf] + DY_OFF, &tdy, &bar[buf], x0, y, b);
-  };
-
-  float bsum = 0.f;  // thread c < COUT: sum of dY channel c
-  int k = 0;
-  int pf_buf = -1, pf_k = 0;
-  int mma_last = -1;
-  bool mma_seen = true;
-  if (tid == 0 && (int)blockIdx.x < ntiles) {
-    issue(blockIdx.x, 0);
-    pf_buf = 0;
-    pf_k = 0;
-  }
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++k) {
-    const int buf = k & 1;
-    if (tid == 0) {
-      // this tile's operands, and the transposed buffers free of the last tile's MMAs
-      if (!mbar_wait(&bar[buf], (uint32_t)((k >> 1) & 1))) {
-        *s_err = 1;
-      } else {
-        pf_buf = -1;
-        if (mma_last >= 0 && !mma_seen) {
-          if (mbar_wait(&bar[2], (uint32_t)(mma_last & 1))) mma_seen = true;
-          else *s_err = 1;
-        }
+  // one thread feeds the tiles and issues the MMAs; the others wait below
+  if (tid == 0) {
+    int issued = 0;  // tiles whose copies have been issued
+    auto issue = [&](int k) {
+      const int t = (int)blockIdx.x + k * (int)gridDim.x;
+      const int per = a.H * segs, b = t / per, r = t - b * per, y = r / segs;
+      const int x0 = (r - y * segs) * TM, s = k % NS;
+      mbar_expect_tx(&full[s], (uint32_t)(HALO_BYTES + GOUT * TM * 16));
+      tma_load5(sm + s * STG, &tx, &full[s], x0 - 1, y - 1, a.xb0 + b);
+      tma_load5(sm + s * STG + DY_OFF, &tdy, &full[s], x0, y, b);
+      issued = k + 1;
+    };
+    const int mine = (int)blockIdx.x < ntiles
+                         ? (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x
+                         : 0;
+    for (int k = 0; k < NS && k < mine; ++k) issue(k);
+    int err = 0, k = 0;
+    for (; k < mine; ++k) {
+      const int s = k % NS;
+      if (!mbar_wait(&full[s], (uint32_t)((k / NS) & 1))) {
+        err = 1;
+        break;
       }
-    }
-    __syncthreads();
-    if (*s_err) break;
-    if (tid == 0 && t + (int)gridDim.x < ntiles) {
-      issue(t + gridDim.x, buf ^ 1);
-      pf_buf = buf ^ 1;
-      pf_k = k + 1;
-    }
-    // K-major operands from the channel-group tiles: A[cout][8 pixels] and,
-    // for each tap, B[cin][8 pixels] of the shifted window
-    const __nv_bfloat16* hx = reinterpret_cast<const __nv_bfloat16*>(stg[buf]);
-    const __nv_bfloat16* hy = reinterpret_cast<const __nv_bfloat16*>(stg[buf] + DY_OFF);
-    for (int it = tid; it < COUT * (TM / 8); it += 128) {
-      const int m = it % COUT, kg = it / COUT;
-      uint32_t w[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int p0 = kg * 8 + 2 * j;
-        const __nv_bfloat16 v0 = hy[((m >> 3) * TM + p0) * 8 + (m & 7)];
-        const __nv_bfloat16 v1 = hy[((m >> 3) * TM + p0 + 1) * 8 + (m & 7)];
-        w[j] = (uint32_t)__bfloat16_as_ushort(v0) | ((uint32_t)__bfloat16_as_ushort(v1) << 16);
-      }
-      *reinterpret_cast<uint4*>(at + ((size_t)kg * 128 + m) * 16) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
-    for (int it = tid; it < 9 * (TM / 8) * CIN; it += 128) {
-      const int n = it % CIN, r = it / CIN, kg = r % (TM / 8), tap = r / (TM / 8);
-      const int dy = tap / 3, dx = tap - dy * 3;
-      uint32_t w[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int p0 = dy * HW_ + kg * 8 + 2 * j + dx;
-        const __nv_bfloat16 v0 = hx[((n >> 3) * 3 * HW_ + p0) * 8 + (n & 7)];
-        const __nv_bfloat16 v1 = hx[((n >> 3) * 3 * HW_ + p0 + 1) * 8 + (n & 7)];
-        w[j] = (uint32_t)__bfloat16_as_ushort(v0) | ((uint32_t)__bfloat16_as_ushort(v1) << 16);
-      }
-      *reinterpret_cast<uint4*>(xt + (size_t)tap * XT_ONE + ((size_t)kg * CIN + n) * 16) =
-          make_uint4(w[0], w[1], w[2], w[3]);
-    }
-    if (tid < COUT) {
-      for (int p = 0; p < TM; ++p) bsum += __bfloat162float(hy[((tid >> 3) * TM + p) * 8 + (tid & 7)]);
-    }
-    fence_async_smem();
-    __syncthreads();
-    if (tid == 0) {
       tc_after();
-      const uint32_t ab = su32(at), xb = su32(xt);
+      const uint32_t hb = su32(sm + s * STG), yb = hb + DY_OFF;
 #pragma unroll 1
       for (int q = 0; q < TM / 16; ++q)
-#pragma unroll 1
-        for (int tap = 0; tap < 9; ++tap) {
-          const uint64_t ad = sdesc(ab + (uint32_t)(2 * q * 128 * 16), 128 * 16, 128);
-          const uint64_t bd =
-              sdesc(xb + (uint32_t)(tap * XT_ONE + 2 * q * CIN * 16), CIN * 16, 128);
-          mma_bf16(tbase + (uint32_t)(tap * CIN), ad, bd, IDESC, (k > 0 || q > 0) ? 1u : 0u);
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx) {
+          const uint64_t ad = sdesc(hb + (uint32_t)(q * 256 + dx * 16), 128, WG_ROW);
+          const uint64_t bd = sdesc(yb + (uint32_t)(q * 256), 128, TM * 16);
+          mma_bf16(tbase + (uint32_t)(dx * COUT), ad, bd, IDESC, (k > 0 || q > 0) ? 1u : 0u);
         }
-      mma_commit(&bar[2]);
-      mma_last = k;
-      mma_seen = false;
+      mma_commit(&empty[s]);
+      // the stage of the tile before this one is free once its MMAs are done;
+      // this tile's are queued behind them
+      if (k > 0 && k - 1 + NS < mine) {
+        if (!mbar_wait(&empty[(k - 1) % NS], (uint32_t)(((k - 1) / NS) & 1))) {
+          err = 2;
+          ++k;
+          break;
+        }
+        issue(k - 1 + NS);
+      }
     }
-  }
-  if (tid == 0) {
-    if (!*s_err && mma_last >= 0 && !mma_seen) {
-      if (mbar_wait(&bar[2], (uint32_t)(mma_last & 1))) mma_seen = true;
-      else *s_err = 2;
+    if (k > 0) {  // every MMA issued so far
+      mma_commit(done);
+      if (!mbar_wait(done, 0)) err = 2;
     }
-    if (*s_err) {
-      if (pf_buf >= 0) mbar_wait(&bar[pf_buf], (uint32_t)((pf_k >> 1) & 1));
-      if (mma_last >= 0 && !mma_seen) mbar_wait(&bar[2], (uint32_t)(mma_last & 1));
+    if (err) {
+      // let the copies in flight land before the shared memory is released
+      for (int j = k; j < issued; ++j)
+        mbar_wait(&full[j % NS], (uint32_t)((j / NS) & 1));
+      *s_err = err;
       flag_error(a.err, 2);
     }
   }
   __syncthreads();
-  // every CTA of the grid has at least one tile; the condition must be the
-  // same in all 32 lanes of warp 0, whose tcgen05.ld is warp-synchronous
-  // (mma_last is known to thread 0 only)
+  // row r of the product = (group, dy, channel) of X; every CTA of the grid
+  // has at least one tile, and the condition is the same in all threads
   if (!*s_err && (int)blockIdx.x < ntiles) {
     tc_after();
-    if (warp == 0) {  // TMEM lanes 0..31 hold the rows cout = 0..31
-      for (int tap = 0; tap < 9; ++tap)
-        for (int c0 = 0; c0 < CIN; c0 += 16) {
-          uint32_t r[16];
-          QP_TLD16(r, tbase + (uint32_t)(tap * CIN + c0));
-          tmem_wait_ld();
-          if (lane < a.couts)
-            for (int i = 0; i < 16; ++i)
-              atomicAdd(&a.dw[((size_t)tap * CIN + c0 + i) * COUT + lane], __uint_as_float(r[i]));
+    const int r = warp * 32 + lane, m = r >> 3, g = m / 3, dy = m - 3 * g, ci = 8 * g + (r & 7);
+    const bool in = m < 3 * GIN, ones = m == 3 * GIN && (r & 7) == 0;
+    for (int dx = 0; dx < 3; ++dx)
+      for (int c0 = 0; c0 < COUT; c0 += 16) {
+        uint32_t v[16];
+        QP_TLD16(v, tbase + ((uint32_t)(warp * 32) << 16) + (uint32_t)(dx * COUT + c0));
+        tmem_wait_ld();
+        float* p = in ? a.dw + ((size_t)((3 * dy + dx) * CIN + ci)) * COUT + c0
+                      : (ones && dx == 0 ? a.db + c0 : nullptr);
+        if (!p) continue;
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) {
+          if (c0 + i + 4 <= a.couts) {
+            asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p + i),
+                         "f"(__uint_as_float(v[i])), "f"(__uint_as_float(v[i + 1])),
+                         "f"(__uint_as_float(v[i + 2])), "f"(__uint_as_float(v[i + 3]))
+                         : "memory");
+          } else {
+#pragma unroll
+            for (int j = i; j < i + 4; ++j)
+              if (c0 + j < a.couts) atomicAdd(p + j, __uint_as_float(v[j]));
+          }
         }
-    }
-    if (tid < a.couts) atomicAdd(&a.db[tid], bsum);
+      }
   }
   tc_before();
   __syncthreads();
@@ -830,7 +810,11 @@ __global__ void k_nn_loss(const float* y, NNData d, int b0, int B, int H, int W,
 }
 
 // a minibatch: pairs idx[0..B) of the set copied into the batch buffers
-__global__ void k_nn_gather(NNData src, const int* idx, NNData dst) {
+// (and the gradient of the step, ng floats, cleared)
+__global__ void k_nn_gather(NNData src, const int* idx, NNData dst, float* grad, int ng) {
+  for (int i = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; i < ng;
+       i += gridDim.x * gridDim.y * blockDim.x)
+    grad[i] = 0.f;
   const size_t C2 = (size_t)NN_CROP * NN_CROP;
   const int b = blockIdx.y, slot = idx[b];
   const uint4* si = reinterpret_cast<const uint4*>(src.img);
@@ -845,37 +829,81 @@ __global__ void k_nn_gather(NNData src, const int* idx, NNData dst) {
   if (blockIdx.x == 0 && threadIdx.x == 0) dst.scale[b] = src.scale[slot];
 }
 
+// The bf16 operands of every layer: forward (Cout x 9 Cin) and data gradient
+// (Cin x 9 Cout, taps flipped), canonical K-major layouts.
+struct PackArgs {
+  __nv_bfloat16* wf[NN_LAYERS];
+  __nv_bfloat16* wd[NN_LAYERS];
+};
+
+// parameter i of the network, value w, into both operands (biases are read as
+// they are)
+__device__ __forceinline__ void nn_pack_one(const PackArgs& p, int i, float w) {
+  int l = 0, cin = NN_CIN0, cout = NN_CH, at = 0;
+#pragma unroll
+  for (l = 0; l < NN_LAYERS; ++l) {
+    cin = l == 0 ? NN_CIN0 : NN_CH;
+    cout = l == NN_LAYERS - 1 ? NN_NLAST : NN_CH;
+    const int n = 9 * cin * cout + cout;
+    if (i < at + n) break;
+    at += n;
+  }
+  const int k = i - at;
+  if (l >= NN_LAYERS || k >= 9 * cin * cout) return;
+  const int t = k / (cin * cout), r = k - t * cin * cout, ci = r / cout, co = r - ci * cout;
+  const __nv_bfloat16 v = __float2bfloat16_rn(w);
+  {  // forward: n = co, k = t*cin + ci
+    const int q = t * cin + ci;
+    p.wf[l][((q >> 3) * (cout >> 3) + (co >> 3)) * 64 + (co & 7) * 8 + (q & 7)] = v;
+  }
+  {  // data gradient: n = ci, k = (8 - t)*cout + co
+    const int q = (8 - t) * cout + co;
+    p.wd[l][((q >> 3) * (cin >> 3) + (ci >> 3)) * 64 + (ci & 7) * 8 + (q & 7)] = v;
+  }
+}
+
+__global__ void k_nn_pack(const float* w, int n, const __grid_constant__ PackArgs p) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    nn_pack_one(p, i, w[i]);
+}
+
+// one Adam step and the operands of the new weights
 __global__ void k_nn_adam(float* w, const float* g, float* m, float* v, int n, float lr,
-                          float b1, float b2, float c1, float c2, float eps) {
+                          float b1, float b2, float c1, float c2, float eps,
+                          const __grid_constant__ PackArgs p) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float gi = g[i];
     const float mi = b1 * m[i] + (1.f - b1) * gi;
     const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    w[i] = wi;
+    nn_pack_one(p, i, wi);
   }
 }
 
-// the bf16 B operands of layer l from the fp32 master: forward (Cout x 9 Cin)
-// and data gradient (Cin x 9 Cout, taps flipped), canonical K-major layouts
-__global__ void k_nn_pack(const float* wl, int cin, int cout, __nv_bfloat16* wf,
-                          __nv_bfloat16* wd) {
-  const int n = 9 * cin * cout;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int t = i / (cin * cout), r = i - t * cin * cout, ci = r / cout, co = r - ci * cout;
-    const __nv_bfloat16 v = __float2bfloat16_rn(wl[i]);
-    {  // forward: n = co, k = t*cin + ci
-      const int k = t * cin + ci;
-      wf[((k >> 3) * (cout >> 3) + (co >> 3)) * 64 + (co & 7) * 8 + (k & 7)] = v;
-    }
-    {  // data gradient: n = ci, k = (8 - t)*cout + co
-      const int k = (8 - t) * cout + co;
-      wd[((k >> 3) * (cin >> 3) + (ci >> 3)) * 64 + (ci & 7) * 8 + (k & 7)] = v;
-    }
+// fp32 images [NB][16][H][W] -> bf16 [2][NB][H][W][8]; thread = pixel and
+// channel group (8 coalesced reads, one 16-byte write).  scale (optional): every
+// image counts.  Bound by memory; on the host the same conversion was 6 of a
+// gradient call's 8 ms (4 images of 128 x 128).
+__global__ void k_nn_images(const float* in, int NB, long long C2, __nv_bfloat16* img,
+                            float* scale) {
+  const long long n = 2 * (long long)NB * C2;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x) {
+    const long long g = i / ((long long)NB * C2), r = i - g * (long long)NB * C2;
+    const long long b = r / C2, px = r - b * C2;
+    const float* f = in + (b * NN_CIN0 + 8 * g) * C2 + px;
+    uint4 u;
+    u.x = pack_bf16(f[0], f[C2]);
+    u.y = pack_bf16(f[2 * C2], f[3 * C2]);
+    u.z = pack_bf16(f[4 * C2], f[5 * C2]);
+    u.w = pack_bf16(f[6 * C2], f[7 * C2]);
+    reinterpret_cast<uint4*>(img)[i] = u;
+    if (scale && i < NB) scale[i] = 1.f;
   }
 }
-
 
 // ---------------------------------------------------------------- host side
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -916,11 +944,10 @@ int tile_map(CUtensorMap* m, const void* base, int G, int NB, int H, int W) {
 }
 
 constexpr size_t conv_smem(int cin, int cout) {
-  return (size_t)cout * 9 * cin * 2 + 2 * (size_t)(((cin / 8) * HALO_G + 127) & ~127) + 64;
+  return (size_t)cout * 9 * cin * 2 + 2 * (size_t)(((cin / 8) * HALO_G + 127) & ~127) + 256;
 }
 constexpr size_t wgrad_smem(int cin, int cout) {
-  return 2 * (size_t)(((((cin / 8) * HALO_G + 127) & ~127) + (cout / 8) * TM * 16 + 127) & ~127) +
-         (size_t)(TM / 8) * 128 * 16 + 9 * (size_t)(TM / 8) * cin * 16 + 64;
+  return (size_t)WG_STAGES * wg_stage(cin, cout) + wg_tail(cin, cout) + 128;
 }
 
 int g_num_sms = 0;
@@ -954,7 +981,7 @@ cudaError_t wgrad_launch(const CUtensorMap& tx, const CUtensorMap& tdy, const Wg
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int ntiles = a.NB * a.H * (a.W / TM);
-  const int grid = std::min(ntiles, num_sms());
+  const int grid = std::min(ntiles, num_sms() * 2);
   k_wgrad<CIN, COUT><<<grid, 128, smem, s>>>(tx, tdy, a);
   return cudaGetLastError();
 }
@@ -963,6 +990,75 @@ cudaError_t wgrad_launch(const CUtensorMap& tx, const CUtensorMap& tdy, const Wg
 }  // namespace qp
 
 using namespace qp;
+
+// Work buffers of one forward/backward over NB images of H x W, kept with the
+// network between calls of one shape (a gradient call spent 1 ms on its 14
+// allocations) as long as they are no larger than KEEP bytes.
+struct Work {
+  static constexpr size_t KEEP = 512u << 20;
+  int NB = 0, H = 0, W = 0;
+  __nv_bfloat16* act[4] = {};
+  __nv_bfloat16* dx[4] = {};
+  __nv_bfloat16* dy5 = nullptr;
+  __nv_bfloat16* img = nullptr;  // the input images
+  float* out32 = nullptr;
+  float* in32 = nullptr;         // the caller's images in fp32 (calls that bring some)
+  float* target = nullptr;
+  float* scale = nullptr;
+  CUtensorMap act_halo[4], dx_halo[4], dx_tile[4], dy5_tile, dy5_halo, img_halo;
+  // buffers and tensor maps for this shape; `host_in`: with room for fp32 input
+  int ensure(int nb, int h, int w, bool host_in) {
+    const size_t px = (size_t)nb * h * w;
+    if (nb != NB || h != H || w != W) {
+      free_all();
+      for (int i = 0; i < 4; ++i) {
+        if (cudaMalloc(&act[i], px * NN_CH * 2) != cudaSuccess ||
+            cudaMalloc(&dx[i], px * NN_CH * 2) != cudaSuccess)
+          return -1;
+        if (halo_map(&act_halo[i], act[i], NN_CH / 8, nb, h, w) ||
+            halo_map(&dx_halo[i], dx[i], NN_CH / 8, nb, h, w) ||
+            tile_map(&dx_tile[i], dx[i], NN_CH / 8, nb, h, w))
+          return -2;
+      }
+      if (cudaMalloc(&dy5, px * NN_NLAST * 2) != cudaSuccess ||
+          cudaMalloc(&img, px * NN_CIN0 * 2) != cudaSuccess ||
+          cudaMalloc(&out32, px * NN_OUT * sizeof(float)) != cudaSuccess ||
+          cudaMalloc(&target, px * NN_OUT * sizeof(float)) != cudaSuccess ||
+          cudaMalloc(&scale, nb * sizeof(float)) != cudaSuccess)
+        return -1;
+      if (tile_map(&dy5_tile, dy5, NN_NLAST / 8, nb, h, w) ||
+          halo_map(&dy5_halo, dy5, NN_NLAST / 8, nb, h, w) ||
+          halo_map(&img_halo, img, NN_CIN0 / 8, nb, h, w))
+        return -2;
+      NB = nb;
+      H = h;
+      W = w;
+    }
+    if (host_in && !in32 && cudaMalloc(&in32, px * NN_CIN0 * sizeof(float)) != cudaSuccess)
+      return -1;
+    return 0;
+  }
+  // after a call: give back what is too large to keep, or incomplete
+  void settle() {
+    const size_t px = (size_t)NB * H * W;
+    if (px * (8 * NN_CH * 2 + (NN_NLAST + NN_CIN0) * 2 + 4 * NN_OUT * 2 +
+              (in32 ? 4 * NN_CIN0 : 0)) > KEEP || NB == 0)
+      free_all();
+  }
+  void free_all() {
+    for (int i = 0; i < 4; ++i) {
+      cudaFree(act[i]);
+      cudaFree(dx[i]);
+      act[i] = dx[i] = nullptr;
+    }
+    for (void* p : {(void*)dy5, (void*)img, (void*)out32, (void*)in32, (void*)target,
+                    (void*)scale})
+      cudaFree(p);
+    dy5 = img = nullptr;
+    out32 = in32 = target = scale = nullptr;
+    NB = H = W = 0;
+  }
+};
 
 // The network: fp32 master parameters (layer l: W[9][cin][cout], bias[cout]),
 // their bf16 forward and data-gradient operands, Adam moments, and the
@@ -981,6 +1077,7 @@ struct qp_nn {
   long long adam_t = 0;
   int* err = nullptr;
   float* loss = nullptr;
+  Work wk;  // of the last call's shape
 };
 
 // Training pairs recorded by a simulation: 128 x 128 crops (the low modes) of
@@ -1034,11 +1131,17 @@ int nn_trace_point(const char* what, int layer, cudaStream_t s) {
     if (e_ != cudaSuccess) return nn_fail(__LINE__, cudaGetErrorString(e_)); \
   } while (0)
 
-int nn_pack(qp_nn* nn, cudaStream_t s) {
+PackArgs nn_pack_args(const qp_nn* nn) {
+  PackArgs p{};
   for (int l = 0; l < NN_LAYERS; ++l) {
-    k_nn_pack<<<64, 256, 0, s>>>(nn->master + nn->off[l], nn_cin(l), nn_cout(l), nn->wf[l],
-                                  nn->wd[l]);
+    p.wf[l] = nn->wf[l];
+    p.wd[l] = nn->wd[l];
   }
+  return p;
+}
+
+int nn_pack(qp_nn* nn, cudaStream_t s) {
+  k_nn_pack<<<148, 256, 0, s>>>(nn->master, nn->nparams, nn_pack_args(nn));
   NK(cudaGetLastError());
   return 0;
 }
@@ -1148,46 +1251,6 @@ int nn_check_err(qp_nn* nn, cudaStream_t s) {
   return 0;
 }
 
-// Work buffers of one forward/backward over NB images of H x W.
-struct Work {
-  int NB = 0, H = 0, W = 0;
-  __nv_bfloat16* act[4] = {};
-  __nv_bfloat16* dx[4] = {};
-  __nv_bfloat16* dy5 = nullptr;
-  float* out32 = nullptr;
-  CUtensorMap act_halo[4], dx_halo[4], dx_tile[4], dy5_tile, dy5_halo;
-  int alloc(int nb, int h, int w) {
-    NB = nb;
-    H = h;
-    W = w;
-    const size_t px = (size_t)nb * h * w;
-    for (int i = 0; i < 4; ++i) {
-      if (cudaMalloc(&act[i], px * NN_CH * 2) != cudaSuccess ||
-          cudaMalloc(&dx[i], px * NN_CH * 2) != cudaSuccess)
-        return -1;
-      if (halo_map(&act_halo[i], act[i], NN_CH / 8, nb, h, w) ||
-          halo_map(&dx_halo[i], dx[i], NN_CH / 8, nb, h, w) ||
-          tile_map(&dx_tile[i], dx[i], NN_CH / 8, nb, h, w))
-        return -2;
-    }
-    if (cudaMalloc(&dy5, px * NN_NLAST * 2) != cudaSuccess ||
-        cudaMalloc(&out32, px * NN_OUT * sizeof(float)) != cudaSuccess)
-      return -1;
-    if (tile_map(&dy5_tile, dy5, NN_NLAST / 8, nb, h, w) ||
-        halo_map(&dy5_halo, dy5, NN_NLAST / 8, nb, h, w))
-      return -2;
-    return 0;
-  }
-  void free_all() {
-    for (int i = 0; i < 4; ++i) {
-      cudaFree(act[i]);
-      cudaFree(dx[i]);
-    }
-    cudaFree(dy5);
-    cudaFree(out32);
-  }
-};
-
 }  // namespace
 
 // ------------------------------------------------------------------- C ABI
@@ -1230,10 +1293,12 @@ extern "C" int qp_nn_create(int device, unsigned long long seed, qp_nn** out) {
         for (int co = 0; co < cout; ++co)
           h[nn->off[l] + (t * nn_cin(l) + ci) * cout + co] = nd(rng);
   }
-  cudaMemcpy(nn->master, h.data(), pb, cudaMemcpyHostToDevice);
-  cudaMemset(nn->m, 0, pb);
-  cudaMemset(nn->v, 0, pb);
-  cudaMemset(nn->err, 0, sizeof(int));
+  // on the network's own (non-blocking) stream: a copy on the legacy stream may
+  // return before its data has arrived, and the packing would not wait for it
+  cudaMemcpyAsync(nn->master, h.data(), pb, cudaMemcpyHostToDevice, nn->stream);
+  cudaMemsetAsync(nn->m, 0, pb, nn->stream);
+  cudaMemsetAsync(nn->v, 0, pb, nn->stream);
+  cudaMemsetAsync(nn->err, 0, sizeof(int), nn->stream);
   if (nn_pack(nn, nn->stream) || cudaStreamSynchronize(nn->stream) != cudaSuccess) {
     qp_nn_destroy(nn);
     return nn_fail(__LINE__, "network set-up failed");
@@ -1246,6 +1311,7 @@ extern "C" int qp_nn_destroy(qp_nn* nn) {
   if (!nn) return 0;
   cudaSetDevice(nn->device);
   if (nn->stream) cudaStreamSynchronize(nn->stream);
+  nn->wk.free_all();
   for (void* p : {(void*)nn->master, (void*)nn->grad, (void*)nn->m, (void*)nn->v,
                   (void*)nn->err, (void*)nn->loss})
     if (p) cudaFree(p);
@@ -1268,28 +1334,24 @@ extern "C" int qp_nn_get_params(qp_nn* nn, float* out) {
 
 extern "C" int qp_nn_set_params(qp_nn* nn, const float* in) {
   if (!nn || !in) return nn_fail(__LINE__, "null argument");
-  NK(cudaMemcpy(nn->master, in, sizeof(float) * nn->nparams, cudaMemcpyHostToDevice));
+  NK(cudaMemcpyAsync(nn->master, in, sizeof(float) * nn->nparams, cudaMemcpyHostToDevice,
+                     nn->stream));
   if (nn_pack(nn, nn->stream)) return -1;
   NK(cudaStreamSynchronize(nn->stream));
   return 0;
 }
 
 namespace {
-// host images [NB][16][H][W] fp32 -> device [2][NB][H][W][8] bf16 (through a
-// host-side conversion; a test and set-up path, not the step's)
-int upload_images(const float* in, int NB, int H, int W, __nv_bfloat16** dev) {
-  const size_t px = (size_t)NB * H * W;
-  std::vector<__nv_bfloat16> h(px * NN_CIN0);
-  for (int b = 0; b < NB; ++b)
-    for (int c = 0; c < NN_CIN0; ++c)
-      for (int y = 0; y < H; ++y)
-        for (int x = 0; x < W; ++x) {
-          const size_t src = (((size_t)b * NN_CIN0 + c) * H + y) * W + x;
-          const size_t dst = ((((size_t)(c >> 3) * NB + b) * H + y) * W + x) * 8 + (c & 7);
-          h[dst] = __float2bfloat16_rn(in[src]);
-        }
-  if (cudaMalloc(dev, h.size() * 2) != cudaSuccess) return -1;
-  return cudaMemcpy(*dev, h.data(), h.size() * 2, cudaMemcpyHostToDevice) == cudaSuccess ? 0 : -1;
+// the caller's fp32 images into the work buffers' bf16 form
+int upload_images(qp_nn* nn, const float* in, cudaStream_t s) {
+  const Work& w = nn->wk;
+  const long long C2 = (long long)w.H * w.W, n = 2 * C2 * w.NB;
+  NK(cudaMemcpyAsync(w.in32, in, sizeof(float) * NN_CIN0 * (size_t)(C2 * w.NB),
+                     cudaMemcpyHostToDevice, s));
+  k_nn_images<<<(int)std::min((n + 255) / 256, 148LL * 16), 256, 0, s>>>(w.in32, w.NB, C2, w.img,
+                                                                        w.scale);
+  NK(cudaGetLastError());
+  return 0;
 }
 
 int check_shape(int NB, int H, int W) {
@@ -1303,19 +1365,18 @@ extern "C" int qp_nn_forward(qp_nn* nn, const float* in, int NB, int H, int W, f
   if (!nn || !in || !out) return nn_fail(__LINE__, "null argument");
   if (check_shape(NB, H, W)) return -1;
   cudaSetDevice(nn->device);
-  __nv_bfloat16* img = nullptr;
-  Work wk;
-  int rc = upload_images(in, NB, H, W, &img) || wk.alloc(NB, H, W) ? -1 : 0;
-  CUtensorMap m_in;
-  if (!rc && halo_map(&m_in, img, NN_CIN0 / 8, NB, H, W)) rc = -1;
-  if (!rc) rc = nn_forward(nn, m_in, 0, wk.act, wk.act_halo, NB, H, W, wk.out32, nullptr, nullptr,
-                           0, 0, 0, nn->stream);
-  if (!rc) rc = nn_check_err(nn, nn->stream);
-  if (!rc && cudaMemcpy(out, wk.out32, sizeof(float) * NN_OUT * (size_t)NB * H * W,
-                        cudaMemcpyDeviceToHost) != cudaSuccess)
+  cudaStream_t s = nn->stream;
+  Work& wk = nn->wk;
+  int rc = wk.ensure(NB, H, W, true) ? nn_fail(__LINE__, "out of device memory (network)")
+                                     : upload_images(nn, in, s);
+  if (!rc) rc = nn_forward(nn, wk.img_halo, 0, wk.act, wk.act_halo, NB, H, W, wk.out32, nullptr,
+                           nullptr, 0, 0, 0, s);
+  if (!rc && cudaMemcpyAsync(out, wk.out32, sizeof(float) * NN_OUT * (size_t)NB * H * W,
+                             cudaMemcpyDeviceToHost, s) != cudaSuccess)
     rc = nn_fail(__LINE__, "download failed");
-  cudaFree(img);
-  wk.free_all();
+  if (!rc) rc = nn_check_err(nn, s);
+  cudaStreamSynchronize(s);
+  wk.settle();
   return rc;
 }
 
@@ -1328,43 +1389,34 @@ extern "C" int qp_nn_loss_grad(qp_nn* nn, const float* in, const float* target, 
   if (check_shape(NB, H, W)) return -1;
   cudaSetDevice(nn->device);
   cudaStream_t s = nn->stream;
-  __nv_bfloat16* img = nullptr;
-  Work wk;
-  NNData d{};
-  int rc = upload_images(in, NB, H, W, &img) || wk.alloc(NB, H, W) ? -1 : 0;
+  Work& wk = nn->wk;
   const size_t px = (size_t)NB * H * W;
-  std::vector<float> ones(NB, 1.f);
-  if (!rc && (cudaMalloc(&d.target, sizeof(float) * 2 * px) != cudaSuccess ||
-              cudaMalloc(&d.scale, sizeof(float) * NB) != cudaSuccess))
-    rc = -1;
+  int rc = wk.ensure(NB, H, W, true) ? nn_fail(__LINE__, "out of device memory (network)")
+                                     : upload_images(nn, in, s);
+  if (!rc && cudaMemcpyAsync(wk.target, target, sizeof(float) * 2 * px, cudaMemcpyHostToDevice,
+                             s) != cudaSuccess)
+    rc = nn_fail(__LINE__, "upload failed");
+  if (!rc) rc = nn_forward(nn, wk.img_halo, 0, wk.act, wk.act_halo, NB, H, W, wk.out32, nullptr,
+                           nullptr, 0, 0, 0, s);
+  float l = 0.f;
   if (!rc) {
-    d.cap = NB;
-    cudaMemcpy(d.target, target, sizeof(float) * 2 * px, cudaMemcpyHostToDevice);
-    cudaMemcpy(d.scale, ones.data(), sizeof(float) * NB, cudaMemcpyHostToDevice);
-  }
-  CUtensorMap m_in;
-  if (!rc && halo_map(&m_in, img, NN_CIN0 / 8, NB, H, W)) rc = -1;
-  if (!rc) rc = nn_forward(nn, m_in, 0, wk.act, wk.act_halo, NB, H, W, wk.out32, nullptr, nullptr,
-                           0, 0, 0, s);
-  if (!rc) {
+    NNData d{NB, wk.img, wk.target, wk.scale};
     cudaMemsetAsync(nn->loss, 0, sizeof(float), s);
     cudaMemsetAsync(nn->grad, 0, sizeof(float) * nn->nparams, s);
     k_nn_loss<<<256, 256, 0, s>>>(wk.out32, d, 0, NB, H, W, 1.f / (2.f * (float)px), wk.dy5,
                                   nn->loss);
-    rc = nn_backward(nn, m_in, 0, wk.act, wk.act_halo, wk.dy5, wk.dy5_tile, wk.dy5_halo, wk.dx,
-                     wk.dx_tile, wk.dx_halo, NB, H, W, s);
+    rc = nn_backward(nn, wk.img_halo, 0, wk.act, wk.act_halo, wk.dy5, wk.dy5_tile, wk.dy5_halo,
+                     wk.dx, wk.dx_tile, wk.dx_halo, NB, H, W, s);
   }
-  if (!rc) rc = nn_check_err(nn, s);
-  float l = 0.f;
-  if (!rc && (cudaMemcpy(&l, nn->loss, sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess ||
-              cudaMemcpy(grad, nn->grad, sizeof(float) * nn->nparams, cudaMemcpyDeviceToHost) !=
-                  cudaSuccess))
+  if (!rc && (cudaMemcpyAsync(&l, nn->loss, sizeof(float), cudaMemcpyDeviceToHost, s) !=
+                  cudaSuccess ||
+              cudaMemcpyAsync(grad, nn->grad, sizeof(float) * nn->nparams, cudaMemcpyDeviceToHost,
+                              s) != cudaSuccess))
     rc = nn_fail(__LINE__, "download failed");
+  if (!rc) rc = nn_check_err(nn, s);
+  cudaStreamSynchronize(s);
   if (loss) *loss = l;
-  cudaFree(img);
-  cudaFree(d.target);
-  cudaFree(d.scale);
-  wk.free_all();
+  wk.settle();
   return rc;
 }
 
@@ -1429,25 +1481,18 @@ extern "C" int qp_nn_train(qp_nn* nn, qp_nn_data* t, const qp_nn_train_desc* d,
   cudaSetDevice(nn->device);
   cudaStream_t s = nn->stream;
   const int B = d->batch, H = NN_CROP, W = NN_CROP;
-  const size_t C2 = (size_t)H * W;
-  Work wk;
-  NNData bt{};
-  bt.cap = B;
+  Work& wk = nn->wk;
   int* idx = nullptr;
   std::vector<int> hidx((size_t)d->steps * B);
   std::mt19937_64 rng(d->seed);
   std::uniform_int_distribution<int> pick(0, t->count - 1);
   for (auto& v : hidx) v = pick(rng);
-  CUtensorMap m_in;
   int rc = 0;
-  if (wk.alloc(B, H, W) || cudaMalloc(&bt.img, (size_t)B * C2 * NN_CIN0 * 2) != cudaSuccess ||
-      cudaMalloc(&bt.target, (size_t)B * C2 * 2 * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&bt.scale, (size_t)B * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&idx, sizeof(int) * hidx.size()) != cudaSuccess ||
-      halo_map(&m_in, bt.img, NN_CIN0 / 8, B, H, W))
+  if (wk.ensure(B, H, W, false) || cudaMalloc(&idx, sizeof(int) * hidx.size()) != cudaSuccess)
     rc = nn_fail(__LINE__, "out of device memory (training buffers)");
-  if (!rc && cudaMemcpy(idx, hidx.data(), sizeof(int) * hidx.size(), cudaMemcpyHostToDevice) !=
-                 cudaSuccess)
+  const NNData bt{B, wk.img, wk.target, wk.scale};  // the minibatch
+  if (!rc && cudaMemcpyAsync(idx, hidx.data(), sizeof(int) * hidx.size(),
+                             cudaMemcpyHostToDevice, s) != cudaSuccess)
     rc = nn_fail(__LINE__, "upload failed");
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
@@ -1461,23 +1506,23 @@ extern "C" int qp_nn_train(qp_nn* nn, qp_nn_data* t, const qp_nn_train_desc* d,
               cudaMemsetAsync(hist, 0, sizeof(float) * d->steps, s) != cudaSuccess))
     rc = nn_fail(__LINE__, "out of device memory (training buffers)");
   for (int it = 0; it < d->steps && !rc; ++it) {
-    k_nn_gather<<<dim3(32, B), 256, 0, s>>>(t->d, idx + (size_t)it * B, bt);
+    k_nn_gather<<<dim3(32, B), 256, 0, s>>>(t->d, idx + (size_t)it * B, bt, nn->grad,
+                                            nn->nparams);
     // the learning rate steps down to 0.3 and 0.1 of its start at 1/2 and 3/4 of the run
     const float lr = d->lr * (it < d->steps / 2 ? 1.f : (it < 3 * d->steps / 4 ? 0.3f : 0.1f));
-    rc = nn_forward(nn, m_in, 0, wk.act, wk.act_halo, B, H, W, wk.out32, nullptr, nullptr, 0, 0,
-                    0, s);
+    rc = nn_forward(nn, wk.img_halo, 0, wk.act, wk.act_halo, B, H, W, wk.out32, nullptr, nullptr,
+                    0, 0, 0, s);
     if (rc) break;
-    cudaMemsetAsync(nn->grad, 0, sizeof(float) * nn->nparams, s);
     k_nn_loss<<<256, 256, 0, s>>>(wk.out32, bt, 0, B, H, W, inv_n, wk.dy5, hist + it);
-    rc = nn_backward(nn, m_in, 0, wk.act, wk.act_halo, wk.dy5, wk.dy5_tile, wk.dy5_halo, wk.dx,
-                     wk.dx_tile, wk.dx_halo, B, H, W, s);
+    rc = nn_backward(nn, wk.img_halo, 0, wk.act, wk.act_halo, wk.dy5, wk.dy5_tile, wk.dy5_halo,
+                     wk.dx, wk.dx_tile, wk.dx_halo, B, H, W, s);
     if (rc) break;
     ++nn->adam_t;
     const float c1 = 1.f - std::pow(b1, (float)nn->adam_t);
     const float c2 = 1.f - std::pow(b2, (float)nn->adam_t);
-    k_nn_adam<<<64, 256, 0, s>>>(nn->master, nn->grad, nn->m, nn->v, nn->nparams, lr, b1, b2, c1,
-                                 c2, 1e-8f);
-    rc = nn_pack(nn, s);
+    k_nn_adam<<<148, 256, 0, s>>>(nn->master, nn->grad, nn->m, nn->v, nn->nparams, lr, b1, b2, c1,
+                                  c2, 1e-8f, nn_pack_args(nn));
+    if (cudaGetLastError() != cudaSuccess) rc = nn_fail(__LINE__, "optimizer launch failed");
   }
   std::vector<float> losses(d->steps, 0.f);
   if (!rc && cudaMemcpyAsync(losses.data(), hist, sizeof(float) * d->steps,
@@ -1493,10 +1538,7 @@ extern "C" int qp_nn_train(qp_nn* nn, qp_nn_data* t, const qp_nn_train_desc* d,
   cudaStreamSynchronize(s);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  wk.free_all();
-  cudaFree(bt.img);
-  cudaFree(bt.target);
-  cudaFree(bt.scale);
+  wk.settle();
   cudaFree(idx);
   cudaFree(hist);
   if (!rc && st) {
