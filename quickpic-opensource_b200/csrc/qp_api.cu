@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstring>
 #include <cstdlib>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -142,6 +143,150 @@ static int ensure_staging(qp_ctx* ctx, size_t bytes) {
   return 0;
 }
 
+// ---- fields and particles to and from the caller's arrays.  A kernel converts
+// the layout and writes (reads) pinned host memory, in parts of BOUNCE floats
+// through two halves: one half crosses PCIe while the host copies the other to
+// or from the caller's pageable array.
+//
+// Pinning costs milliseconds whatever the size, so the halves are kept: a call
+// takes a pair from a pool of the process (its own for the time of the call, so
+// threads and contexts do not share one) and returns it; at most POOL_KEEP
+// pairs stay, and the last context to go frees them.
+static const size_t BOUNCE = 1u << 16;
+static const size_t POOL_KEEP = 4;
+struct Bounce {
+  int device = -1;
+  float* h[2] = {nullptr, nullptr};
+  cudaEvent_t ev[2] = {nullptr, nullptr};
+};
+static std::mutex g_pool_mutex;
+static std::vector<Bounce> g_pool;
+static int g_pool_users = 0;  // live contexts
+
+static void bounce_free(Bounce& b) {
+  for (cudaEvent_t e : b.ev)
+    if (e) cudaEventDestroy(e);
+  if (b.h[0]) cudaFreeHost(b.h[0]);
+  b = Bounce{};
+}
+
+static int bounce_take(qp_ctx* ctx, Bounce* b) {
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    for (size_t i = 0; i < g_pool.size(); ++i)
+      if (g_pool[i].device == ctx->device) {
+        *b = g_pool[i];
+        g_pool.erase(g_pool.begin() + i);
+        return 0;
+      }
+  }
+  b->device = ctx->device;
+  CK(cudaMallocHost(&b->h[0], sizeof(float) * 2 * BOUNCE));
+  b->h[1] = b->h[0] + BOUNCE;
+  for (cudaEvent_t& e : b->ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  return 0;
+}
+
+static void bounce_give(Bounce& b) {
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  if (g_pool_users > 0 && g_pool.size() < POOL_KEEP && b.ev[1])
+    g_pool.push_back(b);
+  else
+    bounce_free(b);
+}
+
+// a context comes (its device has a pair ready from then on) or goes
+static int pool_enter(qp_ctx* ctx) {
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    ++g_pool_users;
+  }
+  Bounce b;
+  const int rc = bounce_take(ctx, &b);
+  bounce_give(b);
+  return rc;
+}
+static void pool_leave() {
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  if (--g_pool_users > 0) return;
+  for (Bounce& b : g_pool) bounce_free(b);
+  g_pool.clear();
+}
+
+// the whole host array, complete on return
+static int to_host(qp_ctx* ctx, const PackJob& job, float* out) {
+  const size_t n = (size_t)job.dim * job.n0 * job.n1, parts = (n + BOUNCE - 1) / BOUNCE;
+  if (n == 0) return 0;
+  Bounce b;
+  int rc = bounce_take(ctx, &b);
+  auto len = [&](size_t i) { return std::min(BOUNCE, n - i * BOUNCE); };
+  auto part = [&](size_t i) -> int {
+    if (i < parts) {
+      launch_pack(job, (long long)(i * BOUNCE), (long long)len(i), b.h[i & 1], ctx->stream);
+      CK(cudaGetLastError());
+      CK(cudaEventRecord(b.ev[i & 1], ctx->stream));
+    }
+    if (i > 0) {
+      CK(cudaEventSynchronize(b.ev[(i - 1) & 1]));
+      std::memcpy(out + (i - 1) * BOUNCE, b.h[(i - 1) & 1], sizeof(float) * len(i - 1));
+    }
+    return 0;
+  };
+  for (size_t i = 0; i <= parts && !rc; ++i) rc = part(i);
+  if (rc) cudaStreamSynchronize(ctx->stream);  // nothing in flight still uses the halves
+  bounce_give(b);
+  return rc;
+}
+
+// the whole host array; complete on return
+static int to_device(qp_ctx* ctx, const PackJob& job, const float* in) {
+  const size_t n = (size_t)job.dim * job.n0 * job.valid1, parts = (n + BOUNCE - 1) / BOUNCE;
+  if (n == 0) return 0;
+  Bounce b;
+  int rc = bounce_take(ctx, &b);
+  auto part = [&](size_t i) -> int {
+    const size_t m = std::min(BOUNCE, n - i * BOUNCE);
+    if (i >= 2) CK(cudaEventSynchronize(b.ev[i & 1]));  // the half has been read
+    std::memcpy(b.h[i & 1], in + i * BOUNCE, sizeof(float) * m);
+    launch_unpack(job, (long long)(i * BOUNCE), (long long)m, b.h[i & 1], ctx->stream);
+    CK(cudaGetLastError());
+    CK(cudaEventRecord(b.ev[i & 1], ctx->stream));
+    return 0;
+  };
+  for (size_t i = 0; i < parts && !rc; ++i) rc = part(i);
+  if (cudaStreamSynchronize(ctx->stream) != cudaSuccess && !rc)
+    rc = fail(ctx, __LINE__, "upload failed");
+  bounce_give(b);
+  return rc;
+}
+
+// rows y = 0 .. rows - 1 of real-space planes as (dim, nx + 2, rows)
+static PackJob rows_job(const GridDims& g, const float* const* p, int dim, long long rows,
+                        float scale = 1.f) {
+  PackJob j{};
+  for (int c = 0; c < dim; ++c) j.plane[c] = const_cast<float*>(p[c]);
+  j.dim = dim;
+  j.n0 = g.nx + 2;
+  j.n1 = j.valid1 = (int)rows;
+  j.stride = 1;
+  j.pitch = g.rp;
+  j.scale = scale;
+  return j;
+}
+
+// columns of k-space planes as (dim, ny + 1, nx + 1)
+static PackJob cols_job(const GridDims& g, const float* const* p, int dim) {
+  PackJob j{};
+  for (int c = 0; c < dim; ++c) j.plane[c] = const_cast<float*>(p[c]);
+  j.dim = dim;
+  j.n0 = g.ny + 1;
+  j.n1 = j.valid1 = g.nx + 1;
+  j.stride = 1;
+  j.pitch = g.kp;
+  j.scale = 1.f;
+  return j;
+}
+
 // Zero freshly allocated device memory before anything else can touch it.
 // The contexts' streams are non-blocking, so a memset left pending on the
 // legacy default stream could land after later work on a context stream.
@@ -212,6 +357,10 @@ extern "C" int qp_ctx_create(const qp_grid_desc* grid, int device, qp_ctx** out)
   ctx->tg.rp = ctx->g.rp;
   CK(cudaMalloc(&ctx->st, sizeof(DevStatus)));
   if (zero_now(ctx->st, sizeof(DevStatus))) return fail(ctx, __LINE__, "status set-up failed");
+  if (pool_enter(ctx)) {
+    pool_leave();
+    return -1;
+  }
   CK(cudaDeviceSynchronize());
   *out = ctx;
   return 0;
@@ -230,6 +379,7 @@ extern "C" int qp_ctx_destroy(qp_ctx* ctx) {
   if (ctx->t0) cudaEventDestroy(ctx->t0);
   if (ctx->t1) cudaEventDestroy(ctx->t1);
   cudaStreamDestroy(ctx->stream);
+  pool_leave();
   delete ctx;
   return 0;
 }
@@ -301,71 +451,33 @@ extern "C" int qp_field2d_dim(const qp_field2d* f) { return f->dim; }
 
 extern "C" int qp_field2d_upload_rs(qp_field2d* f, const float* rf) {
   qp_ctx* ctx = f->ctx;
-  const GridDims& g = ctx->g;
-  const int nxv = g.nx + 2;
-  std::vector<float> h((size_t)f->dim * g.rplane, 0.f);
-  for (int c = 0; c < f->dim; ++c)
-    for (int y = 0; y <= g.ny; ++y)
-      for (int x = 0; x < nxv; ++x)
-        h[(size_t)c * g.rplane + (size_t)y * g.rp + x] =
-            rf[(size_t)c + (size_t)f->dim * ((size_t)x + (size_t)nxv * y)];
-  for (int c = 0; c < f->dim; ++c)
-    CK(cudaMemcpyAsync(f->rs[c], &h[(size_t)c * g.rplane], sizeof(float) * g.rplane,
-                       cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
+  if (to_device(ctx, rows_job(ctx->g, f->rs, f->dim, ctx->g.ny + 1), rf)) return -1;
   f->state = 0;
   return 0;
 }
 
-extern "C" int qp_field2d_download_rs(qp_field2d* f, float* rf) {
-  qp_ctx* ctx = f->ctx;
+// rf(dim, nx+2, 2 ny + 1): rows past the guard row are zero
+static int download_rs(qp_ctx* ctx, const float* const* p, int dim, float* rf,
+                       float scale = 1.f) {
   const GridDims& g = ctx->g;
-  const int nxv = g.nx + 2, nypmx = 2 * g.ny + 1;
-  std::vector<float> h((size_t)f->dim * g.rplane);
-  for (int c = 0; c < f->dim; ++c)
-    CK(cudaMemcpyAsync(&h[(size_t)c * g.rplane], f->rs[c], sizeof(float) * g.rplane,
-                       cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
-  std::memset(rf, 0, sizeof(float) * (size_t)f->dim * nxv * nypmx);
-  for (int c = 0; c < f->dim; ++c)
-    for (int y = 0; y <= g.ny; ++y)
-      for (int x = 0; x < nxv; ++x)
-        rf[(size_t)c + (size_t)f->dim * ((size_t)x + (size_t)nxv * y)] =
-            h[(size_t)c * g.rplane + (size_t)y * g.rp + x];
-  return 0;
+  const size_t row = (size_t)dim * (g.nx + 2);
+  std::memset(rf + row * (g.ny + 1), 0, sizeof(float) * row * g.ny);
+  return to_host(ctx, rows_job(g, p, dim, g.ny + 1, scale), rf);
+}
+
+extern "C" int qp_field2d_download_rs(qp_field2d* f, float* rf) {
+  return download_rs(f->ctx, f->rs, f->dim, rf);
 }
 
 extern "C" int qp_field2d_upload_ks(qp_field2d* f, const float* kf) {
   qp_ctx* ctx = f->ctx;
-  const GridDims& g = ctx->g;
-  std::vector<float> h((size_t)f->dim * g.kplane, 0.f);
-  for (int c = 0; c < f->dim; ++c)
-    for (int kx = 0; kx <= g.nx; ++kx)
-      for (int ky = 0; ky <= g.ny; ++ky)
-        h[(size_t)c * g.kplane + (size_t)kx * g.kp + ky] =
-            kf[(size_t)c + (size_t)f->dim * ((size_t)ky + (size_t)(g.ny + 1) * kx)];
-  for (int c = 0; c < f->dim; ++c)
-    CK(cudaMemcpyAsync(f->ks[c], &h[(size_t)c * g.kplane], sizeof(float) * g.kplane,
-                       cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
+  if (to_device(ctx, cols_job(ctx->g, f->ks, f->dim), kf)) return -1;
   f->state = 1;
   return 0;
 }
 
 extern "C" int qp_field2d_download_ks(qp_field2d* f, float* kf) {
-  qp_ctx* ctx = f->ctx;
-  const GridDims& g = ctx->g;
-  std::vector<float> h((size_t)f->dim * g.kplane);
-  for (int c = 0; c < f->dim; ++c)
-    CK(cudaMemcpyAsync(&h[(size_t)c * g.kplane], f->ks[c], sizeof(float) * g.kplane,
-                       cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
-  for (int c = 0; c < f->dim; ++c)
-    for (int kx = 0; kx <= g.nx; ++kx)
-      for (int ky = 0; ky <= g.ny; ++ky)
-        kf[(size_t)c + (size_t)f->dim * ((size_t)ky + (size_t)(g.ny + 1) * kx)] =
-            h[(size_t)c * g.kplane + (size_t)kx * g.kp + ky];
-  return 0;
+  return to_host(f->ctx, cols_job(f->ctx->g, f->ks, f->dim), kf);
 }
 
 // sine (0) / cosine (1) parity of component c along x (axis 0) or y (axis 1)
@@ -813,9 +925,15 @@ static int species_load(qp_species* sp, float s) {
   for (int k = 0; k < NCOMP; ++k) {
     std::fill(h.begin(), h.end(), 0.f);
     for (long long n = 0; n < np; ++n) h[slot[n]] = c[k][n];
-    CK(cudaMemcpy(sp->P0.c[k], h.data(), sizeof(float) * h.size(), cudaMemcpyHostToDevice));
+    // on the context's (non-blocking) stream, and complete before h is filled
+    // again: a copy on the legacy stream may return before its data has arrived
+    CK(cudaMemcpyAsync(sp->P0.c[k], h.data(), sizeof(float) * h.size(), cudaMemcpyHostToDevice,
+                       ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
   }
-  CK(cudaMemcpy(sp->P0.count, cnt.data(), sizeof(int) * tg.ntiles, cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(sp->P0.count, cnt.data(), sizeof(int) * tg.ntiles, cudaMemcpyHostToDevice,
+                     ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
   return species_renew_device(sp, s);
 }
 
@@ -1049,24 +1167,31 @@ extern "C" long long qp_species_np(qp_species* sp) {
   return n;
 }
 
+// the particles as ppart(8, nppmx, ntiles), zero past each tile's count
+static PackJob particles_job(const qp_species* sp, int nppmx) {
+  PackJob j{};
+  for (int c = 0; c < NCOMP; ++c) j.plane[c] = sp->A.c[c];
+  j.dim = NCOMP;
+  j.n0 = nppmx;
+  j.n1 = j.valid1 = sp->ctx->tg.ntiles;
+  j.stride = 1;
+  j.pitch = sp->A.cap;
+  j.count = sp->A.count;
+  j.scale = 1.f;
+  return j;
+}
+
 extern "C" int qp_species_download(qp_species* sp, float* ppart, int* kpic, int nppmx_ld) {
   qp_ctx* ctx = sp->ctx;
-  const int nt = ctx->tg.ntiles, cap = sp->A.cap;
+  const int nt = ctx->tg.ntiles;
   std::vector<int> cnt(nt);
   CK(cudaMemcpyAsync(cnt.data(), sp->A.count, sizeof(int) * nt, cudaMemcpyDeviceToHost,
                      ctx->stream));
-  std::vector<float> h((size_t)nt * cap);
   CK(cudaStreamSynchronize(ctx->stream));
   int mx = 0;
   for (int v : cnt) mx = std::max(mx, v);
   if (nppmx_ld < mx) return fail(ctx, __LINE__, "download: nppmx_ld too small");
-  std::memset(ppart, 0, sizeof(float) * 8 * (size_t)nppmx_ld * nt);
-  for (int c = 0; c < NCOMP; ++c) {
-    CK(cudaMemcpy(h.data(), sp->A.c[c], sizeof(float) * h.size(), cudaMemcpyDeviceToHost));
-    for (int t = 0; t < nt; ++t)
-      for (int n = 0; n < cnt[t]; ++n)
-        ppart[(size_t)c + 8 * ((size_t)n + (size_t)nppmx_ld * t)] = h[(size_t)t * cap + n];
-  }
+  if (to_host(ctx, particles_job(sp, nppmx_ld), ppart)) return -1;
   std::memcpy(kpic, cnt.data(), sizeof(int) * nt);
   return 0;
 }
@@ -1082,16 +1207,12 @@ extern "C" int qp_species_upload(qp_species* sp, const float* ppart, const int* 
     part_free(&sp->A);
     if (part_alloc(&sp->A, nt, mx)) return fail(ctx, __LINE__, "out of device memory");
   }
-  const int cap = sp->A.cap;
-  std::vector<float> h((size_t)nt * cap);
-  for (int c = 0; c < NCOMP; ++c) {
-    std::fill(h.begin(), h.end(), 0.f);
-    for (int t = 0; t < nt; ++t)
-      for (int n = 0; n < kpic[t]; ++n)
-        h[(size_t)t * cap + n] = ppart[(size_t)c + 8 * ((size_t)n + (size_t)nppmx_ld * t)];
-    CK(cudaMemcpy(sp->A.c[c], h.data(), sizeof(float) * h.size(), cudaMemcpyHostToDevice));
-  }
-  CK(cudaMemcpy(sp->A.count, kpic, sizeof(int) * nt, cudaMemcpyHostToDevice));
+  LinList zero(ctx->st, ctx->stream);
+  for (int c = 0; c < NCOMP; ++c) zero.add(LIN_FILL, (long long)nt * sp->A.cap, sp->A.c[c]);
+  zero.flush();
+  CK(cudaMemcpyAsync(sp->A.count, kpic, sizeof(int) * nt, cudaMemcpyHostToDevice, ctx->stream));
+  if (to_device(ctx, particles_job(sp, nppmx_ld), ppart)) return -1;
+  CK(cudaStreamSynchronize(ctx->stream));
   return 0;
 }
 
@@ -1108,14 +1229,8 @@ extern "C" int qp_species_download_q3(qp_species* sp, int pos, float* rf) {
   qp_ctx* ctx = sp->ctx;
   const GridDims& g = ctx->g;
   if (pos < 1 || pos > ctx->nz + 1) return fail(ctx, __LINE__, "q3: slice out of range");
-  std::vector<float> h(g.rplane);
-  CK(cudaMemcpyAsync(h.data(), sp->q3 + (size_t)(pos - 1) * g.rplane, sizeof(float) * g.rplane,
-                     cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
-  const int nxv = g.nx + 2;
-  for (int y = 0; y <= g.ny; ++y)
-    for (int x = 0; x < nxv; ++x) rf[(size_t)x + (size_t)nxv * y] = h[(size_t)y * g.rp + x];
-  return 0;
+  const float* p = sp->q3 + (size_t)(pos - 1) * g.rplane;
+  return to_host(ctx, rows_job(g, &p, 1, g.ny + 1), rf);
 }
 
 // ------------------------------------------------------------------ beam
@@ -1259,6 +1374,8 @@ extern "C" int qp_beam_create(qp_ctx* ctx, const qp_beam_desc* d, qp_beam** out)
                     cudaMemcpyHostToDevice));
     }
   }
+  // the copies above have arrived before work on the context's stream reads them
+  CK(cudaStreamSynchronize(cudaStreamLegacy));
   *out = b;
   return 0;
 }
@@ -1318,27 +1435,21 @@ extern "C" int qp_beam_upload(qp_beam* b, const float* part, long long np) {
 
 extern "C" int qp_beam_download(qp_beam* b, float* part) {
   qp_ctx* ctx = b->ctx;
-  std::vector<float> h(b->b.np);
-  for (int k = 0; k < BCOMP; ++k) {
-    CK(cudaMemcpy(h.data(), b->b.c[k], sizeof(float) * h.size(), cudaMemcpyDeviceToHost));
-    for (long long n = 0; n < b->b.np; ++n) part[(size_t)k + 7 * (size_t)n] = h[n];
-  }
-  return 0;
+  PackJob j{};
+  for (int c = 0; c < BCOMP; ++c) j.plane[c] = b->b.c[c];
+  j.dim = BCOMP;
+  j.n0 = (int)b->b.np;
+  j.n1 = j.valid1 = 1;
+  j.stride = 1;
+  j.scale = 1.f;
+  return to_host(ctx, j, part);
 }
 
 extern "C" int qp_beam_download_q3d(qp_beam* b, float* rf) {
   qp_ctx* ctx = b->ctx;
   const GridDims& g = ctx->g;
-  const size_t np3 = (size_t)(ctx->nz + 1) * g.rplane;
-  std::vector<float> h(np3);
-  CK(cudaMemcpy(h.data(), b->q3d, sizeof(float) * np3, cudaMemcpyDeviceToHost));
-  const int nxv = g.nx + 2;
-  for (int l = 0; l <= ctx->nz; ++l)
-    for (int y = 0; y <= g.ny; ++y)
-      for (int x = 0; x < nxv; ++x)
-        rf[(size_t)x + (size_t)nxv * ((size_t)y + (size_t)(g.ny + 1) * l)] =
-            h[(size_t)l * g.rplane + (size_t)y * g.rp + x];
-  return 0;
+  const float* p = b->q3d;
+  return to_host(ctx, rows_job(g, &p, 1, (long long)(ctx->nz + 1) * (g.ny + 1)), rf);
 }
 
 // ---------------------------------------------------------------- beam restart

@@ -180,22 +180,11 @@ __global__ void k_beam_aos_to_soa(const float* aos, BeamBuf b) {
   }
 }
 
-// on-axis line of a stack of 3D planes: out[l] = p[l][y][x]
-__global__ void k_lineout(const float* p, long long plane, long long off, int n, float* out) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l < n) out[l] = p[(long long)l * plane + off];
-}
-
 }  // namespace
 
 void launch_beam_aos_to_soa(const float* aos, const BeamBuf& b, cudaStream_t s) {
   if (b.np == 0) return;
   k_beam_aos_to_soa<<<148 * 8, 256, 0, s>>>(aos, b);
-}
-
-void launch_lineout(const float* p, long long plane, long long off, int n, float* out,
-                    cudaStream_t s) {
-  k_lineout<<<(n + 255) / 256, 256, 0, s>>>(p, plane, off, n, out);
 }
 
 void launch_beam_push(const BeamBuf& b, const GridDims& g, int nz, const Fields3& f, float qtmh,

@@ -13,8 +13,6 @@ struct BeamBuf {
 };
 
 void launch_beam_aos_to_soa(const float* aos, const BeamBuf& b, cudaStream_t s);
-void launch_lineout(const float* p, long long plane, long long off, int n, float* out,
-                    cudaStream_t s);
 void launch_beam_deposit(const BeamBuf& b, const GridDims& g, int nz, float* q3, DevStatus* st,
                          cudaStream_t s);
 

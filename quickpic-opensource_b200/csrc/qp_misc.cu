@@ -167,6 +167,39 @@ __global__ void k_guard_add(Planes3 pl, GridDims g, const DevStatus* st) {
   }
 }
 
+// One host element per thread and step.  The host side is contiguous and, for
+// the transfers of the C ABI, pinned host memory: the kernel itself moves the
+// data over PCIe, in place of a copy of each plane and a strided loop on the
+// host (2 ms per 512 x 512 vector; bound now by the host's page faults on the
+// caller's fresh array, 1 us per 4 KB).
+__global__ void __launch_bounds__(256) k_pack(const __grid_constant__ PackJob j, long long i0,
+                                              long long n, float* out) {
+  grid_dep_sync();
+  const long long row = (long long)j.dim * j.n0;
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
+       k += (long long)gridDim.x * blockDim.x) {
+    const long long i = i0 + k, b = i / row, r = i - b * row, a = r / j.dim;
+    const int c = (int)(r - a * j.dim);
+    float v = 0.f;
+    if (b < j.valid1 && (!j.count || a < j.count[b]))
+      v = j.plane[c][b * j.pitch + a * j.stride] * j.scale;
+    out[k] = v;
+  }
+}
+
+__global__ void __launch_bounds__(256) k_unpack(const __grid_constant__ PackJob j, long long i0,
+                                                long long n, const float* in) {
+  grid_dep_sync();
+  const long long row = (long long)j.dim * j.n0;
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
+       k += (long long)gridDim.x * blockDim.x) {
+    const long long i = i0 + k, b = i / row, r = i - b * row, a = r / j.dim;
+    const int c = (int)(r - a * j.dim);
+    if (b < j.valid1 && (!j.count || a < j.count[b]))
+      j.plane[c][b * j.pitch + a * j.stride] = in[k];
+  }
+}
+
 __global__ void k_cursor(DevStatus* st, int v) {
   grid_dep_sync();
   if (st->error) return;
@@ -242,6 +275,19 @@ void launch_guard_add(float* const* p, int count, const GridDims& g, const DevSt
                       cudaStream_t s) {
   launch_pdl(k_guard_add, dim3((g.nx + 1 + 255) / 256, count), 256, 0, s, planes3(p, count), g,
              st);
+}
+
+static int pack_blocks(long long n) {
+  return (int)std::max(1LL, std::min((n + 255) / 256, 148LL * 8));
+}
+
+void launch_pack(const PackJob& job, long long i0, long long n, float* out, cudaStream_t s) {
+  launch_pdl(k_pack, pack_blocks(n), 256, 0, s, job, i0, n, out);
+}
+
+void launch_unpack(const PackJob& job, long long i0, long long n, const float* in,
+                   cudaStream_t s) {
+  launch_pdl(k_unpack, pack_blocks(n), 256, 0, s, job, i0, n, in);
 }
 
 void launch_cursor(DevStatus* st, int v, cudaStream_t s) {

@@ -83,5 +83,24 @@ void launch_guard_copy(float* const* p, int count, const GridDims& g, const DevS
                        cudaStream_t s);
 void launch_guard_add(float* const* p, int count, const GridDims& g, const DevStatus* st,
                       cudaStream_t s);
+// Between device planes and the caller's interleaved arrays: element
+// c + dim (a + n0 b) of the host array is scale * src[c][b pitch + a stride]
+// for b < n1 (and a < count[b] when count is given), 0 otherwise.
+struct PackJob {
+  float* plane[8];
+  int dim, n0, n1;      // host extents: components, fast index, slow index
+  int valid1;           // slow indices that have data
+  int stride;           // floats between consecutive fast indices of a plane
+  long long pitch;      // floats between consecutive slow indices of a plane
+  const int* count;
+  float scale;
+};
+// elements [i0, i0 + n) of the host array; `out` and `in` are pinned host (or
+// device) memory and start at element i0.  No status check: a caller may look at
+// the fields after an error.
+void launch_pack(const PackJob& job, long long i0, long long n, float* out, cudaStream_t s);
+// the reverse, data within valid1 and count only
+void launch_unpack(const PackJob& job, long long i0, long long n, const float* in,
+                   cudaStream_t s);
 void launch_cursor(DevStatus* st, int v, cudaStream_t s);
 }  // namespace qp

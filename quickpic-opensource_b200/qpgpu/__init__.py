@@ -190,7 +190,7 @@ class Field2d:
         self._c(self.ctx._L.qp_field2d_upload_rs(self.h, _ptr(a)))
 
     def get_rs(self):
-        out = np.zeros(self.ctx.rs_shape(self.dim), dtype=np.float32, order="F")
+        out = np.empty(self.ctx.rs_shape(self.dim), dtype=np.float32, order="F")
         self._c(self.ctx._L.qp_field2d_download_rs(self.h, _ptr(out)))
         return out
 
@@ -199,7 +199,7 @@ class Field2d:
         self._c(self.ctx._L.qp_field2d_upload_ks(self.h, _ptr(a)))
 
     def get_ks(self):
-        out = np.zeros(self.ctx.ks_shape(self.dim), dtype=np.float32, order="F")
+        out = np.empty(self.ctx.ks_shape(self.dim), dtype=np.float32, order="F")
         self._c(self.ctx._L.qp_field2d_download_ks(self.h, _ptr(out)))
         return out
 
@@ -358,7 +358,7 @@ class Species2d:
     def get_particles(self, nppmx=None):
         """(ppart(8, nppmx, ntiles), kpic(ntiles)) in the reference layout."""
         nppmx = nppmx or self.nppmx
-        pp = np.zeros((8, nppmx, self.ntiles), dtype=np.float32, order="F")
+        pp = np.empty((8, nppmx, self.ntiles), dtype=np.float32, order="F")
         kp = np.zeros(self.ntiles, dtype=np.int32)
         self._c(self.ctx._L.qp_species_download(self.h, _ptr(pp), _ptr(kp), nppmx))
         return pp, kp
@@ -369,17 +369,17 @@ class Species2d:
         self._c(self.ctx._L.qp_species_upload(self.h, _ptr(pp), _ptr(kp), pp.shape[1]))
 
     def get_qn(self):
-        out = np.zeros(self.ctx.rs_shape(1), dtype=np.float32, order="F")
+        out = np.empty(self.ctx.rs_shape(1), dtype=np.float32, order="F")
         self._c(self.ctx._L.qp_species_download_qn(self.h, _ptr(out)))
         return out
 
     def get_q(self):
-        out = np.zeros(self.ctx.rs_shape(1), dtype=np.float32, order="F")
+        out = np.empty(self.ctx.rs_shape(1), dtype=np.float32, order="F")
         self._c(self.ctx._L.qp_species_download_q(self.h, _ptr(out)))
         return out
 
     def get_q3(self, pos):
-        out = np.zeros((self.ctx.nx + 2, self.ctx.ny + 1), dtype=np.float32, order="F")
+        out = np.empty((self.ctx.nx + 2, self.ctx.ny + 1), dtype=np.float32, order="F")
         self._c(self.ctx._L.qp_species_download_q3(self.h, pos, _ptr(out)))
         return out
 
@@ -458,7 +458,7 @@ class Beam3d:
         self.ctx._check(self.ctx._L.qp_beam_push(self.h, sim.h, C.c_float(dt)))
 
     def get_particles(self):
-        out = np.zeros((7, self.np()), dtype=np.float32, order="F")
+        out = np.empty((7, self.np()), dtype=np.float32, order="F")
         self.ctx._check(self.ctx._L.qp_beam_download(self.h, _ptr(out)))
         return out
 
@@ -478,7 +478,7 @@ class Beam3d:
 
     def get_q3d(self):
         c = self.ctx
-        out = np.zeros((c.nx + 2, c.ny + 1, c.nz + 1), dtype=np.float32, order="F")
+        out = np.empty((c.nx + 2, c.ny + 1, c.nz + 1), dtype=np.float32, order="F")
         c._check(c._L.qp_beam_download_q3d(self.h, _ptr(out)))
         return out
 
@@ -551,7 +551,7 @@ class Simulation:
         "q3", "qb" (nx+2, ny+1)."""
         c = self.ctx
         shape = (c.nx + 2, c.ny + 1) if name in ("q3", "qb") else (3, c.nx + 2, c.ny + 1)
-        out = np.zeros(shape, dtype=np.float32, order="F")
+        out = np.empty(shape, dtype=np.float32, order="F")
         c._check(c._L.qp_sim_download_plane(self.h, name.encode(), int(plane), _ptr(out)))
         return out
 
@@ -562,7 +562,7 @@ class Simulation:
         dim = dims[name]
         ks = ("epw", "cu_k", "epwb", "epw_prev", "epw_prev2")
         shape = c.ks_shape(dim) if name in ks else c.rs_shape(dim)
-        out = np.zeros(shape, dtype=np.float32, order="F")
+        out = np.empty(shape, dtype=np.float32, order="F")
         c._check(c._L.qp_sim_download_field(self.h, name.encode(), _ptr(out)))
         return out
 
@@ -572,7 +572,7 @@ class Simulation:
             shape = (c.nx + 2, c.ny + 1, c.nz + 1)
         else:
             shape = (3, c.nx + 2, c.ny + 1, c.nz + 1)
-        out = np.zeros(shape, dtype=np.float32, order="F")
+        out = np.empty(shape, dtype=np.float32, order="F")
         c._check(c._L.qp_sim_download_3d(self.h, name.encode(), _ptr(out)))
         return out
 
