@@ -279,6 +279,10 @@ __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtenso
   __syncthreads();
   tc_after();
   const uint32_t tbase = *tslot;
+  // everything above (barriers, tensor memory, weights) may run before the
+  // kernel ahead is done: the weights are never written by that kernel (Adam
+  // and the packing are followed by a gather, an image conversion or the host)
+  grid_dep_sync();
 
   auto tile_coord = [&](int t, int& b, int& y, int& x0) {
     const int per = a.H * segs;
@@ -507,6 +511,7 @@ __global__ void __launch_bounds__(128) k_wgrad(const __grid_constant__ CUtensorM
   __syncthreads();
   tc_after();
   const uint32_t tbase = *tslot;
+  grid_dep_sync();
 
   // one thread feeds the tiles and issues the MMAs; the others wait below
   if (tid == 0) {
@@ -602,6 +607,7 @@ __global__ void __launch_bounds__(128) k_wgrad(const __grid_constant__ CUtensorM
 
 // ------------------------------------------------------- features and records
 __global__ void k_nn_norms(NNSlicePlanes p, int nx, int ny, int kp, float* part) {
+  grid_dep_sync();
   __shared__ float red[3][8];
   float sb = 0.f, sj = 0.f, sz = 0.f;
   const long long n = (long long)(nx + 1) * (ny + 1);
@@ -682,6 +688,7 @@ __device__ __forceinline__ void nn_feature(const NNSlicePlanes& p, size_t o, int
 // window kx < hc, ky < wc; scale_out = the epw scale
 __global__ void k_nn_features(NNSlicePlanes p, int nx, int ny, int kp, int hc, int wc,
                               const float* part, __nv_bfloat16* img, float* scale_out) {
+  grid_dep_sync();
   __shared__ float sc[3];
   nn_scales(part, nx, ny, sc);
   if (blockIdx.x == 0 && threadIdx.x == 0) scale_out[0] = sc[0];
@@ -710,6 +717,7 @@ struct NNData {
 // for every mode (epw_prev2 <- epw_prev, epw_prev <- epw)
 __global__ void k_nn_record_start(NNSlicePlanes p, int nx, int ny, int kp, const float* part,
                                   NNData d, int slot) {
+  grid_dep_sync();
   __shared__ float sc[3];
   nn_scales(part, nx, ny, sc);
   if (blockIdx.x == 0 && threadIdx.x == 0) d.scale[slot] = sc[0];
@@ -741,6 +749,7 @@ __global__ void k_nn_record_start(NNSlicePlanes p, int nx, int ny, int kp, const
 
 // recording, slice end: target slot += converged epw / scale
 __global__ void k_nn_record_end(NNSlicePlanes p, int kp, NNData d, int slot) {
+  grid_dep_sync();
   const float sB = d.scale[slot];
   const size_t C2 = (size_t)NN_CROP * NN_CROP;
   float* t = d.target + (size_t)slot * 2 * C2;
@@ -758,6 +767,7 @@ __global__ void k_nn_record_end(NNSlicePlanes p, int kp, NNData d, int slot) {
 // correction the network can learn from; its scale is set to 0, which takes
 // it out of the loss
 __global__ void k_nn_record_validate(NNData d, int slot) {
+  grid_dep_sync();
   __shared__ float red[32];
   const size_t C2 = (size_t)NN_CROP * NN_CROP;
   const float* t = d.target + (size_t)slot * 2 * C2;
@@ -778,6 +788,7 @@ __global__ void k_nn_record_validate(NNData d, int slot) {
 // weight); dY = 2 (y - t) / n as the last layer's output gradient
 __global__ void k_nn_loss(const float* y, NNData d, int b0, int B, int H, int W, float inv_n,
                           __nv_bfloat16* dy, float* loss) {
+  grid_dep_sync();
   __shared__ float red[8];
   const long long n = (long long)B * H * W;
   const size_t C2 = (size_t)H * W;
@@ -812,6 +823,7 @@ __global__ void k_nn_loss(const float* y, NNData d, int b0, int B, int H, int W,
 // a minibatch: pairs idx[0..B) of the set copied into the batch buffers
 // (and the gradient of the step, ng floats, cleared)
 __global__ void k_nn_gather(NNData src, const int* idx, NNData dst, float* grad, int ng) {
+  grid_dep_sync();
   for (int i = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; i < ng;
        i += gridDim.x * gridDim.y * blockDim.x)
     grad[i] = 0.f;
@@ -863,6 +875,7 @@ __device__ __forceinline__ void nn_pack_one(const PackArgs& p, int i, float w) {
 }
 
 __global__ void k_nn_pack(const float* w, int n, const __grid_constant__ PackArgs p) {
+  grid_dep_sync();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     nn_pack_one(p, i, w[i]);
 }
@@ -871,6 +884,7 @@ __global__ void k_nn_pack(const float* w, int n, const __grid_constant__ PackArg
 __global__ void k_nn_adam(float* w, const float* g, float* m, float* v, int n, float lr,
                           float b1, float b2, float c1, float c2, float eps,
                           const __grid_constant__ PackArgs p) {
+  grid_dep_sync();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float gi = g[i];
     const float mi = b1 * m[i] + (1.f - b1) * gi;
@@ -889,6 +903,7 @@ __global__ void k_nn_adam(float* w, const float* g, float* m, float* v, int n, f
 // gradient call's 8 ms (4 images of 128 x 128).
 __global__ void k_nn_images(const float* in, int NB, long long C2, __nv_bfloat16* img,
                             float* scale) {
+  grid_dep_sync();
   const long long n = 2 * (long long)NB * C2;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
@@ -969,8 +984,7 @@ cudaError_t conv_launch(const CUtensorMap& tin, const ConvArgs& a, cudaStream_t 
   if (e != cudaSuccess) return e;
   const int ntiles = a.NB * a.H * (a.W / TM);
   const int grid = std::min(ntiles, num_sms() * 4);
-  k_conv3x3<CIN, COUT, EPI><<<grid, 128, smem, s>>>(tin, a);
-  return cudaGetLastError();
+  return launch_pdl(k_conv3x3<CIN, COUT, EPI>, grid, 128, smem, s, tin, a);
 }
 
 template <int CIN, int COUT>
@@ -982,8 +996,7 @@ cudaError_t wgrad_launch(const CUtensorMap& tx, const CUtensorMap& tdy, const Wg
   if (e != cudaSuccess) return e;
   const int ntiles = a.NB * a.H * (a.W / TM);
   const int grid = std::min(ntiles, num_sms() * 2);
-  k_wgrad<CIN, COUT><<<grid, 128, smem, s>>>(tx, tdy, a);
-  return cudaGetLastError();
+  return launch_pdl(k_wgrad<CIN, COUT>, grid, 128, smem, s, tx, tdy, a);
 }
 
 }  // namespace
@@ -1141,7 +1154,7 @@ PackArgs nn_pack_args(const qp_nn* nn) {
 }
 
 int nn_pack(qp_nn* nn, cudaStream_t s) {
-  k_nn_pack<<<148, 256, 0, s>>>(nn->master, nn->nparams, nn_pack_args(nn));
+  launch_pdl(k_nn_pack, 148, 256, 0, s, nn->master, nn->nparams, nn_pack_args(nn));
   NK(cudaGetLastError());
   return 0;
 }
@@ -1348,7 +1361,7 @@ int upload_images(qp_nn* nn, const float* in, cudaStream_t s) {
   const long long C2 = (long long)w.H * w.W, n = 2 * C2 * w.NB;
   NK(cudaMemcpyAsync(w.in32, in, sizeof(float) * NN_CIN0 * (size_t)(C2 * w.NB),
                      cudaMemcpyHostToDevice, s));
-  k_nn_images<<<(int)std::min((n + 255) / 256, 148LL * 16), 256, 0, s>>>(w.in32, w.NB, C2, w.img,
+  launch_pdl(k_nn_images, (int)std::min((n + 255) / 256, 148LL * 16), 256, 0, s, w.in32, w.NB, C2, w.img,
                                                                         w.scale);
   NK(cudaGetLastError());
   return 0;
@@ -1403,7 +1416,7 @@ extern "C" int qp_nn_loss_grad(qp_nn* nn, const float* in, const float* target, 
     NNData d{NB, wk.img, wk.target, wk.scale};
     cudaMemsetAsync(nn->loss, 0, sizeof(float), s);
     cudaMemsetAsync(nn->grad, 0, sizeof(float) * nn->nparams, s);
-    k_nn_loss<<<256, 256, 0, s>>>(wk.out32, d, 0, NB, H, W, 1.f / (2.f * (float)px), wk.dy5,
+    launch_pdl(k_nn_loss, 256, 256, 0, s, wk.out32, d, 0, NB, H, W, 1.f / (2.f * (float)px), wk.dy5,
                                   nn->loss);
     rc = nn_backward(nn, wk.img_halo, 0, wk.act, wk.act_halo, wk.dy5, wk.dy5_tile, wk.dy5_halo,
                      wk.dx, wk.dx_tile, wk.dx_halo, NB, H, W, s);
@@ -1506,21 +1519,21 @@ extern "C" int qp_nn_train(qp_nn* nn, qp_nn_data* t, const qp_nn_train_desc* d,
               cudaMemsetAsync(hist, 0, sizeof(float) * d->steps, s) != cudaSuccess))
     rc = nn_fail(__LINE__, "out of device memory (training buffers)");
   for (int it = 0; it < d->steps && !rc; ++it) {
-    k_nn_gather<<<dim3(32, B), 256, 0, s>>>(t->d, idx + (size_t)it * B, bt, nn->grad,
+    launch_pdl(k_nn_gather, dim3(32, B), 256, 0, s, t->d, idx + (size_t)it * B, bt, nn->grad,
                                             nn->nparams);
     // the learning rate steps down to 0.3 and 0.1 of its start at 1/2 and 3/4 of the run
     const float lr = d->lr * (it < d->steps / 2 ? 1.f : (it < 3 * d->steps / 4 ? 0.3f : 0.1f));
     rc = nn_forward(nn, wk.img_halo, 0, wk.act, wk.act_halo, B, H, W, wk.out32, nullptr, nullptr,
                     0, 0, 0, s);
     if (rc) break;
-    k_nn_loss<<<256, 256, 0, s>>>(wk.out32, bt, 0, B, H, W, inv_n, wk.dy5, hist + it);
+    launch_pdl(k_nn_loss, 256, 256, 0, s, wk.out32, bt, 0, B, H, W, inv_n, wk.dy5, hist + it);
     rc = nn_backward(nn, wk.img_halo, 0, wk.act, wk.act_halo, wk.dy5, wk.dy5_tile, wk.dy5_halo,
                      wk.dx, wk.dx_tile, wk.dx_halo, B, H, W, s);
     if (rc) break;
     ++nn->adam_t;
     const float c1 = 1.f - std::pow(b1, (float)nn->adam_t);
     const float c2 = 1.f - std::pow(b2, (float)nn->adam_t);
-    k_nn_adam<<<148, 256, 0, s>>>(nn->master, nn->grad, nn->m, nn->v, nn->nparams, lr, b1, b2, c1,
+    launch_pdl(k_nn_adam, 148, 256, 0, s, nn->master, nn->grad, nn->m, nn->v, nn->nparams, lr, b1, b2, c1,
                                   c2, 1e-8f, nn_pack_args(nn));
     if (cudaGetLastError() != cudaSuccess) rc = nn_fail(__LINE__, "optimizer launch failed");
   }
@@ -1601,8 +1614,8 @@ void nn_runtime_destroy(NNRuntime* r) {
 int nn_predict(NNRuntime* r, const void* net, const NNSlicePlanes& p, const GridDims& g,
                DevStatus* st, cudaStream_t s) {
   qp_nn* nn = const_cast<qp_nn*>(static_cast<const qp_nn*>(net));
-  k_nn_norms<<<NN_NORM_BLOCKS, 256, 0, s>>>(p, g.nx, g.ny, g.kp, r->part);
-  k_nn_features<<<NN_NORM_BLOCKS, 256, 0, s>>>(p, g.nx, g.ny, g.kp, r->hc, r->wc, r->part,
+  launch_pdl(k_nn_norms, NN_NORM_BLOCKS, 256, 0, s, p, g.nx, g.ny, g.kp, r->part);
+  launch_pdl(k_nn_features, NN_NORM_BLOCKS, 256, 0, s, p, g.nx, g.ny, g.kp, r->hc, r->wc, r->part,
                                                 r->img, r->scale);
   // layers 1-4 ping-pong between the two activation buffers; every layer's
   // input is the previous output, so the four maps cycle through them
@@ -1621,8 +1634,8 @@ int nn_record_start(NNRuntime* r, void* data, const NNSlicePlanes& p, const Grid
   (void)st;
   if (t->count >= t->d.cap) return 0;
   const int slot = t->count;
-  k_nn_norms<<<NN_NORM_BLOCKS, 256, 0, s>>>(p, g.nx, g.ny, g.kp, r->part);
-  k_nn_record_start<<<NN_NORM_BLOCKS * 4, 256, 0, s>>>(p, g.nx, g.ny, g.kp, r->part, t->d, slot);
+  launch_pdl(k_nn_norms, NN_NORM_BLOCKS, 256, 0, s, p, g.nx, g.ny, g.kp, r->part);
+  launch_pdl(k_nn_record_start, NN_NORM_BLOCKS * 4, 256, 0, s, p, g.nx, g.ny, g.kp, r->part, t->d, slot);
   return 2;
 }
 
@@ -1633,8 +1646,8 @@ int nn_record_end(NNRuntime* r, void* data, const NNSlicePlanes& p, const GridDi
   (void)st;
   if (t->count >= t->d.cap) return 0;
   const int slot = t->count;
-  k_nn_record_end<<<64, 256, 0, s>>>(p, g.kp, t->d, slot);
-  k_nn_record_validate<<<1, 1024, 0, s>>>(t->d, slot);
+  launch_pdl(k_nn_record_end, 64, 256, 0, s, p, g.kp, t->d, slot);
+  launch_pdl(k_nn_record_validate, 1, 1024, 0, s, t->d, slot);
   t->count++;
   return 2;
 }
