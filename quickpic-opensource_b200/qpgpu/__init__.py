@@ -77,6 +77,15 @@ def _ptr(a):
     return a.ctypes.data_as(C.c_void_p)
 
 
+# component lists are 1 to 3 values: a ctypes array costs a tenth of a numpy one
+def _ints(v):
+    return (C.c_int * len(v))(*map(int, v))
+
+
+def _floats(v):
+    return (C.c_float * len(v))(*map(float, v))
+
+
 class _GridDesc(C.Structure):
     _fields_ = [("indx", C.c_int), ("indy", C.c_int), ("indz", C.c_int),
                 ("box", (C.c_double * 2) * 3)]
@@ -245,26 +254,22 @@ class Field2d:
         if dim is None:
             self._c(self.ctx._L.qp_field2d_add(self.h, a1.h, a2.h))
         else:
-            d, d1, d2 = (np.asarray(v, dtype=np.int32) for v in (dim, dim1, dim2))
-            self._c(self.ctx._L.qp_field2d_add_comp(self.h, a1.h, a2.h, _ptr(d), _ptr(d1),
-                                                    _ptr(d2), len(d)))
+            self._c(self.ctx._L.qp_field2d_add_comp(self.h, a1.h, a2.h, _ints(dim), _ints(dim1),
+                                                    _ints(dim2), len(dim)))
 
     def sub(self, a1, a2, dim=None, dim1=None, dim2=None):
         if dim is None:
             self._c(self.ctx._L.qp_field2d_sub(self.h, a1.h, a2.h))
         else:
-            d, d1, d2 = (np.asarray(v, dtype=np.int32) for v in (dim, dim1, dim2))
-            self._c(self.ctx._L.qp_field2d_sub_comp(self.h, a1.h, a2.h, _ptr(d), _ptr(d1),
-                                                    _ptr(d2), len(d)))
+            self._c(self.ctx._L.qp_field2d_sub_comp(self.h, a1.h, a2.h, _ints(dim), _ints(dim1),
+                                                    _ints(dim2), len(dim)))
 
     def mult(self, a1, value, dim=None, dim1=None):
         if dim is None:
             self._c(self.ctx._L.qp_field2d_mult(self.h, a1.h, C.c_float(value)))
         else:
-            d, d1 = (np.asarray(v, dtype=np.int32) for v in (dim, dim1))
-            v = np.asarray(value, dtype=np.float32)
-            self._c(self.ctx._L.qp_field2d_mult_comp(self.h, a1.h, _ptr(d), _ptr(d1), _ptr(v),
-                                                     len(d)))
+            self._c(self.ctx._L.qp_field2d_mult_comp(self.h, a1.h, _ints(dim), _ints(dim1),
+                                                     _floats(value), len(dim)))
 
     def cg(self):
         self._c(self.ctx._L.qp_field2d_cg(self.h))
