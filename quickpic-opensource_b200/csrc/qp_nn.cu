@@ -1010,6 +1010,7 @@ using namespace qp;
 struct Work {
   static constexpr size_t KEEP = 512u << 20;
   int NB = 0, H = 0, W = 0;
+  unsigned char* slab = nullptr;  // holds every buffer but in32
   __nv_bfloat16* act[4] = {};
   __nv_bfloat16* dx[4] = {};
   __nv_bfloat16* dy5 = nullptr;
@@ -1024,21 +1025,38 @@ struct Work {
     const size_t px = (size_t)nb * h * w;
     if (nb != NB || h != H || w != W) {
       free_all();
+      // one allocation, cut into 256-byte aligned buffers
+      size_t total = 0;
+      auto room = [&](size_t bytes) {
+        const size_t at = total;
+        total += (bytes + 255) & ~size_t(255);
+        return at;
+      };
+      size_t oa[4], od[4];
       for (int i = 0; i < 4; ++i) {
-        if (cudaMalloc(&act[i], px * NN_CH * 2) != cudaSuccess ||
-            cudaMalloc(&dx[i], px * NN_CH * 2) != cudaSuccess)
-          return -1;
+        oa[i] = room(px * NN_CH * 2);
+        od[i] = room(px * NN_CH * 2);
+      }
+      const size_t oy = room(px * NN_NLAST * 2), oi = room(px * NN_CIN0 * 2),
+                   oo = room(px * NN_OUT * sizeof(float)), ot = room(px * NN_OUT * sizeof(float)),
+                   os = room(nb * sizeof(float));
+      if (cudaMalloc(&slab, total) != cudaSuccess) {
+        slab = nullptr;
+        return -1;
+      }
+      for (int i = 0; i < 4; ++i) {
+        act[i] = reinterpret_cast<__nv_bfloat16*>(slab + oa[i]);
+        dx[i] = reinterpret_cast<__nv_bfloat16*>(slab + od[i]);
         if (halo_map(&act_halo[i], act[i], NN_CH / 8, nb, h, w) ||
             halo_map(&dx_halo[i], dx[i], NN_CH / 8, nb, h, w) ||
             tile_map(&dx_tile[i], dx[i], NN_CH / 8, nb, h, w))
           return -2;
       }
-      if (cudaMalloc(&dy5, px * NN_NLAST * 2) != cudaSuccess ||
-          cudaMalloc(&img, px * NN_CIN0 * 2) != cudaSuccess ||
-          cudaMalloc(&out32, px * NN_OUT * sizeof(float)) != cudaSuccess ||
-          cudaMalloc(&target, px * NN_OUT * sizeof(float)) != cudaSuccess ||
-          cudaMalloc(&scale, nb * sizeof(float)) != cudaSuccess)
-        return -1;
+      dy5 = reinterpret_cast<__nv_bfloat16*>(slab + oy);
+      img = reinterpret_cast<__nv_bfloat16*>(slab + oi);
+      out32 = reinterpret_cast<float*>(slab + oo);
+      target = reinterpret_cast<float*>(slab + ot);
+      scale = reinterpret_cast<float*>(slab + os);
       if (tile_map(&dy5_tile, dy5, NN_NLAST / 8, nb, h, w) ||
           halo_map(&dy5_halo, dy5, NN_NLAST / 8, nb, h, w) ||
           halo_map(&img_halo, img, NN_CIN0 / 8, nb, h, w))
@@ -1059,14 +1077,10 @@ struct Work {
       free_all();
   }
   void free_all() {
-    for (int i = 0; i < 4; ++i) {
-      cudaFree(act[i]);
-      cudaFree(dx[i]);
-      act[i] = dx[i] = nullptr;
-    }
-    for (void* p : {(void*)dy5, (void*)img, (void*)out32, (void*)in32, (void*)target,
-                    (void*)scale})
-      cudaFree(p);
+    if (slab) cudaFree(slab);
+    if (in32) cudaFree(in32);
+    slab = nullptr;
+    for (int i = 0; i < 4; ++i) act[i] = dx[i] = nullptr;
     dy5 = img = nullptr;
     out32 = in32 = target = scale = nullptr;
     NB = H = W = 0;
