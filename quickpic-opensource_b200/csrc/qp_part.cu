@@ -343,6 +343,29 @@ __device__ __forceinline__ void amjdp_one(const FieldTile& sf, int nn, int mm, f
   o->v[7] = v3;
 }
 
+// K consecutive floats (a multiple of K from a tile's 16-byte aligned start)
+template <int K>
+__device__ __forceinline__ void load_k(const float* p, float (&v)[K]) {
+  if constexpr (K == 4) {
+    const float4 f = *reinterpret_cast<const float4*>(p);
+    v[0] = f.x;
+    v[1] = f.y;
+    v[2] = f.z;
+    v[3] = f.w;
+  } else {
+    const float2 f = *reinterpret_cast<const float2*>(p);
+    v[0] = f.x;
+    v[1] = f.y;
+  }
+}
+template <int K>
+__device__ __forceinline__ void store_k(float* p, const float (&v)[K]) {
+  if constexpr (K == 4)
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  else
+    *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
+}
+
 // Where amjdp adds its 8 densities: node-major [y][x][8] (node, the fused
 // step) or one plane each.  cz (node form only, optional): the z current also
 // goes to this plane.
@@ -437,7 +460,10 @@ __device__ __forceinline__ void deposit_last(const Densities& d, const TileGeom&
 // reductions spread over neighbouring nodes.  The per-particle products are
 // those of the reference; only the order in which a node's contributions are
 // summed differs.  The planes must be zero on entry.
-template <bool NODE>
+// K = 4 particles per thread and CTA = tile is the form for grids that fill the
+// GPU.  Grids of few tiles leave most of it idle and wait for one CTA's serial
+// work: there two CTAs share a tile with 2 particles per thread.
+template <bool NODE, int K>
 __global__ void __launch_bounds__(256, 3) k_amjdp(PartBuf P, TileGeom tg, GatherPlanes f,
                                                   const __grid_constant__ Densities den, float qbm,
                                                   float dt, float dex, float scale,
@@ -468,29 +494,27 @@ __global__ void __launch_bounds__(256, 3) k_amjdp(PartBuf P, TileGeom tg, Gather
   // the whole warp loops while one of its lanes has particles (the shuffles
   // of the last runs); a lane past the count reads the tile's first slots and
   // neither deposits nor writes them
-  for (int k0 = 4 * threadIdx.x; k0 - 4 * lane < n; k0 += 4 * blockDim.x) {
+  const int first = K == 4 ? 4 * threadIdx.x : K * (threadIdx.x + 256 * blockIdx.y);
+  for (int k0 = first; k0 - K * lane < n; k0 += 4 * blockDim.x) {
     const bool live = k0 < n;
     const long long kb = base + (live ? k0 : 0);
-    const float4 X = *reinterpret_cast<const float4*>(P.c[0] + kb);
-    const float4 Y = *reinterpret_cast<const float4*>(P.c[1] + kb);
-    const float4 VX = *reinterpret_cast<const float4*>(P.c[2] + kb);
-    const float4 VY = *reinterpret_cast<const float4*>(P.c[3] + kb);
+    float xs[K], ys[K], vxs[K], vys[K], p6s[K], p7s[K], qms[K];
+    load_k<K>(P.c[0] + kb, xs);
+    load_k<K>(P.c[1] + kb, ys);
+    load_k<K>(P.c[2] + kb, vxs);
+    load_k<K>(P.c[3] + kb, vys);
     // with ext, p6 and p7 are formed here from psi (k_extpsi) instead of read
-    float4 P6 = make_float4(0.f, 0.f, 0.f, 0.f), P7 = P6;
+#pragma unroll
+    for (int j = 0; j < K; ++j) p6s[j] = p7s[j] = 0.f;
     if (!ext) {
-      P6 = *reinterpret_cast<const float4*>(P.c[5] + kb);
-      P7 = *reinterpret_cast<const float4*>(P.c[6] + kb);
+      load_k<K>(P.c[5] + kb, p6s);
+      load_k<K>(P.c[6] + kb, p7s);
     }
-    const float4 QM = *reinterpret_cast<const float4*>(P.c[7] + kb);
-    const float xs[4] = {X.x, X.y, X.z, X.w}, ys[4] = {Y.x, Y.y, Y.z, Y.w};
-    const float vxs[4] = {VX.x, VX.y, VX.z, VX.w}, vys[4] = {VY.x, VY.y, VY.z, VY.w};
-    float p6s[4] = {P6.x, P6.y, P6.z, P6.w}, p7s[4] = {P7.x, P7.y, P7.z, P7.w};
-    const float qms[4] = {QM.x, QM.y, QM.z, QM.w};
-    float p6o[4] = {P6.x, P6.y, P6.z, P6.w};
+    load_k<K>(P.c[7] + kb, qms);
     float acc[4][8];
     int cell = -1;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < K; ++j) {
       if (k0 + j < n) {
         int nn = (int)xs[j], mm = (int)ys[j];
         const float dxp = xs[j] - (float)nn, dyp = ys[j] - (float)mm;
@@ -512,7 +536,7 @@ __global__ void __launch_bounds__(256, 3) k_amjdp(PartBuf P, TileGeom tg, Gather
         AmjOut o;
         amjdp_one(sf, nn, mm, dxp, dyp, vxs[j], vys[j], p6s[j], p7s[j], qms[j], qbm, qtmh, dti,
                   dex, idex, &o);
-        p6o[j] = o.p6;
+        p6s[j] = o.p6;
         // the moments only feed the deposit: the scale goes on the corner
         // weights and the run sums use fused multiply-adds (FP32 roundoff of
         // the sums, like the order of the reductions)
@@ -545,11 +569,8 @@ __global__ void __launch_bounds__(256, 3) k_amjdp(PartBuf P, TileGeom tg, Gather
     deposit_last<NODE>(den, tg, noffp, moffp, cell, acc, cprev >= 0 && cell == cprev + 1,
                  cell >= 0 && cnext == cell + 1);
     if (live) {
-      P6 = make_float4(p6o[0], p6o[1], p6o[2], p6o[3]);
-      *reinterpret_cast<float4*>(P.c[5] + base + k0) = P6;
-      if (ext)
-        *reinterpret_cast<float4*>(P.c[6] + base + k0) =
-            make_float4(p7s[0], p7s[1], p7s[2], p7s[3]);
+      store_k<K>(P.c[5] + base + k0, p6s);
+      if (ext) store_k<K>(P.c[6] + base + k0, p7s);
     }
   }
 }
@@ -865,7 +886,9 @@ __global__ void __launch_bounds__(256) k_push(PartBuf A, PartBuf B, Inbox ib, Ti
 // Insert the movers of tile t after its stayers, sorted by their key so that
 // the particle order does not depend on the order in which the atomics of the
 // push handed out inbox slots.
-__global__ void __launch_bounds__(256) k_insert(PartBuf B, Inbox ib, TileGeom tg, int p2max,
+// At most 32 registers: 8 CTAs per SM hold the 1024 tiles of a 512 x 512 grid in
+// one wave (6 left a second one of 136 CTAs).
+__global__ void __launch_bounds__(256, 8) k_insert(PartBuf B, Inbox ib, TileGeom tg, int p2max,
                                                 DevStatus* st, float* dq) {
   grid_dep_sync();
   extern __shared__ unsigned long long skey[];
@@ -888,47 +911,69 @@ __global__ void __launch_bounds__(256) k_insert(PartBuf B, Inbox ib, TileGeom tg
     atomicMax(&st->need_cap, stay + nin);
     return;
   }
-  int p2 = 1;
-  while (p2 < nin) p2 <<= 1;
-  const long long ib0 = (long long)t * ib.cap;
-  for (int i = threadIdx.x; i < p2; i += blockDim.x) {
-    skey[i] = (i < nin) ? ib.key[ib0 + i] : ~0ull;
-    sidx[i] = i;
-  }
-  __syncthreads();
-  for (int k = 2; k <= p2; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = threadIdx.x; i < p2; i += blockDim.x) {
-        const int ixj = i ^ j;
-        if (ixj > i) {
-          const bool up = (i & k) == 0;
-          const unsigned long long a = skey[i], b = skey[ixj];
-          if ((a > b) == up) {
-            skey[i] = b;
-            skey[ixj] = a;
-            const int ti = sidx[i];
-            sidx[i] = sidx[ixj];
-            sidx[ixj] = ti;
+  const long long ib0 = (long long)t * ib.cap, ob = (long long)t * B.cap + stay;
+  if (nin <= (int)blockDim.x) {
+    // one mover per thread: its place is the number of smaller keys (the keys
+    // differ), found without the sort's barriers (a 512 x 512 step moves 20 to
+    // 60 particles into a tile: 21 barriers of a bitonic sort).  The mover's
+    // components are on their way meanwhile.
+    const int i = threadIdx.x;
+    unsigned long long key = 0;
+    float v[NCOMP];
+    if (i < nin) {
+      key = ib.key[ib0 + i];
+#pragma unroll
+      for (int c = 0; c < NCOMP; ++c) v[c] = ib.c[c][ib0 + i];
+      skey[i] = key;
+    }
+    __syncthreads();
+    if (i < nin) {
+      int rank = 0;
+      for (int k = 0; k < nin; ++k) rank += skey[k] < key || (skey[k] == key && k < i) ? 1 : 0;
+#pragma unroll
+      for (int c = 0; c < NCOMP; ++c) B.c[c][ob + rank] = v[c];
+    }
+  } else {
+    int p2 = 1;
+    while (p2 < nin) p2 <<= 1;
+    for (int i = threadIdx.x; i < p2; i += blockDim.x) {
+      skey[i] = (i < nin) ? ib.key[ib0 + i] : ~0ull;
+      sidx[i] = i;
+    }
+    __syncthreads();
+    for (int k = 2; k <= p2; k <<= 1) {
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        for (int i = threadIdx.x; i < p2; i += blockDim.x) {
+          const int ixj = i ^ j;
+          if (ixj > i) {
+            const bool up = (i & k) == 0;
+            const unsigned long long a = skey[i], b = skey[ixj];
+            if ((a > b) == up) {
+              skey[i] = b;
+              skey[ixj] = a;
+              const int ti = sidx[i];
+              sidx[i] = sidx[ixj];
+              sidx[ixj] = ti;
+            }
           }
         }
+        __syncthreads();
       }
-      __syncthreads();
     }
-  }
-  const long long ob = (long long)t * B.cap + stay;
-  for (int i = threadIdx.x; i < nin; i += blockDim.x) {
-    const int si = sidx[i];
-    if (si < 0 || si >= nin) {  // the sort must map the first nin keys onto filled slots
-      raise_error(st, -8);
-      continue;
+    for (int i = threadIdx.x; i < nin; i += blockDim.x) {
+      const int si = sidx[i];
+      if (si < 0 || si >= nin) {  // the sort must map the first nin keys onto filled slots
+        raise_error(st, -8);
+        continue;
+      }
+      const long long src = ib0 + si;
+      // all loads before the stores, so the mover waits for L2 once
+      float v[NCOMP];
+#pragma unroll
+      for (int c = 0; c < NCOMP; ++c) v[c] = ib.c[c][src];
+#pragma unroll
+      for (int c = 0; c < NCOMP; ++c) B.c[c][ob + i] = v[c];
     }
-    const long long src = ib0 + si;
-    // all loads before the stores, so the mover waits for L2 once
-    float v[NCOMP];
-#pragma unroll
-    for (int c = 0; c < NCOMP; ++c) v[c] = ib.c[c][src];
-#pragma unroll
-    for (int c = 0; c < NCOMP; ++c) B.c[c][ob + i] = v[c];
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -1004,7 +1049,7 @@ void launch_amjdp(const PartBuf& P, const TileGeom& tg, const GatherPlanes& f, f
                   cudaStream_t s) {
   Densities d{};
   for (int i = 0; i < 8; ++i) d.pl[i] = acc[i];
-  launch_pdl(k_amjdp<false>, tg.ntiles, 256, 0, s, P, tg, f, d, qbm, dt, dex, scale,
+  launch_pdl(k_amjdp<false, 4>, tg.ntiles, 256, 0, s, P, tg, f, d, qbm, dt, dex, scale,
              const_cast<DevStatus*>(st));
 }
 
@@ -1014,8 +1059,13 @@ void launch_amjdp_node(const PartBuf& P, const TileGeom& tg, const GatherPlanes&
   Densities d{};
   d.node = node;
   d.cz = cz;
-  launch_pdl(k_amjdp<true>, tg.ntiles, 256, 0, s, P, tg, f, d, qbm, dt, dex, scale,
-             const_cast<DevStatus*>(st));
+  // two CTAs per tile while they all fit at once: 3 per SM of 148
+  if (tg.ntiles <= 222)
+    launch_pdl(k_amjdp<true, 2>, dim3(tg.ntiles, 2), 256, 0, s, P, tg, f, d, qbm, dt, dex, scale,
+               const_cast<DevStatus*>(st));
+  else
+    launch_pdl(k_amjdp<true, 4>, tg.ntiles, 256, 0, s, P, tg, f, d, qbm, dt, dex, scale,
+               const_cast<DevStatus*>(st));
 }
 
 void launch_push(int mode, const PartBuf& A, const PartBuf& B, const Inbox& ib,
