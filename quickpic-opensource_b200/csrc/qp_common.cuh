@@ -59,11 +59,9 @@ struct LineTables {
 };
 
 // Layout of LineTables::lane for P = n / 64 (offsets in floats).
-__host__ __device__ constexpr int lt_sn0(int P) { return 0; }
-__host__ __device__ constexpr int lt_sn1(int P) { return 32 * P; }
-__host__ __device__ constexpr int lt_cs0(int P) { return 64 * P; }
-__host__ __device__ constexpr int lt_cs1(int P) { return 96 * P; }
-__host__ __device__ constexpr int lt_tw4(int P) { return 128 * P; }   // float2 [P][32]
+__host__ __device__ constexpr int lt_sn(int P) { return 0; }          // float2 [P][32]: 2 sin
+__host__ __device__ constexpr int lt_cs(int P) { return 64 * P; }     // float2 [P][32]
+__host__ __device__ constexpr int lt_tw4(int P) { return 128 * P; }   // float2 [P][32]: half
 __host__ __device__ constexpr int lt_uw(int P) { return 192 * P; }    // float2 [P][32]
 __host__ __device__ constexpr int lt_tw5(int P) { return 256 * P; }   // float2 [4][32]
 __host__ __device__ constexpr int lt_tw3(int P) { return 256 * P + 256; }  // float2 [16]

@@ -46,14 +46,16 @@ int line_tables_build(LineTablesHost* t, int logn) {
     for (int a = 0; a < P; ++a)
       for (int l = 0; l < 32; ++l) {
         const int m = l + 32 * a, j0 = 2 * m, j1 = 2 * m + 1;
-        lt[lt_sn0(P) + 32 * a + l] = sn[std::min(j0, n - j0)];
-        lt[lt_sn1(P) + 32 * a + l] = sn[std::min(j1, n - j1)];
-        lt[lt_cs0(P) + 32 * a + l] = cs[j0];
-        lt[lt_cs1(P) + 32 * a + l] = cs[j1];
+        // twice the sines and half the twiddles after the first DFT: the factor
+        // 0.5 of the pre-twiddle costs nothing there (powers of two are exact)
+        f2(lt_sn(P), 32 * a + l,
+           make_float2(2.f * sn[std::min(j0, n - j0)], 2.f * sn[std::min(j1, n - j1)]));
+        f2(lt_cs(P), 32 * a + l, make_float2(cs[j0], cs[j1]));
       }
     for (int k2 = 0; k2 < P; ++k2)
       for (int l = 0; l < 32; ++l) {
-        f2(lt_tw4(P), 32 * k2 + l, tw[l * k2]);
+        const float2 t4 = tw[l * k2];
+        f2(lt_tw4(P), 32 * k2 + l, make_float2(0.5f * t4.x, 0.5f * t4.y));
         f2(lt_uw(P), 32 * k2 + l, uw[k2 + P * (line_xs(P) ? l : brev5(l))]);
       }
     for (int si = 0; si < 4; ++si) {
@@ -312,7 +314,7 @@ __global__ void __launch_bounds__(256) k_xinv4(const __grid_constant__ X4Job job
 // stores of 16 bytes per thread at 512 points, where the planar form loads 8
 // bytes and stores 4 at a time.  Planar components follow, 8 rows per CTA.
 template <int P>
-__global__ void __launch_bounds__(256) k_xfwd8(const __grid_constant__ X8Job job, GridDims g,
+__global__ void __launch_bounds__(256, P == 8 ? 4 : P == 16 ? 3 : 0) k_xfwd8(const __grid_constant__ X8Job job, GridDims g,
                                                LineTables tx, const DevStatus* st) {
   extern __shared__ __align__(16) float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

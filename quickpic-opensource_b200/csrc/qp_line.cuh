@@ -292,6 +292,27 @@ __device__ __forceinline__ void dft8(float2 (&x)[8]) {
   x[7] = make_float2(h1.x - k1.y, h1.y + k1.x);  // h1 + i k1
 }
 
+// Real-FFT unscramble of mode k from Z[k] = a and Z[n/2 - k] = b, with uw =
+// exp(-2 pi i k / n): 2 Y[k] = (a + conj b) - i uw (a - conj b), and
+//   sine:   out[2k] = -2 Im Y[k], out[2k+1] = Re Y[0] + 2 sum_{m=1..k} Re Y[m]
+//   cosine: out[2k] =  2 Re Y[k], out[2k+1] = 2 sigma - 2 sum_{m=1..k} Im Y[m]
+// ev = out[2k], term = k's term of the sum; k = 0 (`zero`): Y[0] = Re a + Im a,
+// and yh = Y[n/2] = Re a - Im a.
+__device__ __forceinline__ void unscramble(float2 a, float2 b, float2 uw, bool zero, int parity,
+                                           float* ev, float* term, float* yh) {
+  const float2 D = make_float2(a.x - b.x, a.y + b.y);
+  const float2 u = cmul(uw, D);
+  float re = (a.x + b.x) + u.y, im = (a.y - b.y) - u.x;  // 2 Y[k]
+  if (parity == 0) {
+    *ev = zero ? 0.f : -im;
+    *term = zero ? a.x + a.y : re;
+  } else {
+    *ev = zero ? 2.f * (a.x + a.y) : re;
+    *term = zero ? 0.f : -im;
+  }
+  if (zero) *yh = a.x - a.y;
+}
+
 // Steps 5-8 of the register transform for P = 8 (256-point complex FFT,
 // 8 values per lane), through shared memory instead of 5 shuffle stages.
 // In: w[k2] = f_k2(lane), the input of the 32-point DFT over the lanes.
@@ -365,27 +386,9 @@ __device__ __forceinline__ void reg_line_tail_xs(float2 (&w)[P], float* out, int
   float run = 0.f;
 #pragma unroll
   for (int k2 = 0; k2 < P; ++k2) {
-    const int k = k2 + P * lane;
-    const float2 a = A[k2];
-    const float2 b = make_float2(B[k2].x, -B[k2].y);
-    float2 Y;
-    if (k == 0) {
-      Y = make_float2(a.x + a.y, 0.f);
-      yh = a.x - a.y;
-    } else {
-      const float2 E = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y + b.y));
-      const float2 D = make_float2(a.x - b.x, a.y - b.y);
-      const float2 u = cmul(uwl[32 * k2 + lane], D);
-      Y = make_float2(E.x + 0.5f * u.y, E.y - 0.5f * u.x);
-    }
     float term;
-    if (parity == 0) {
-      ev[k2] = (k == 0) ? 0.f : -2.f * Y.y;
-      term = (k == 0) ? Y.x : 2.f * Y.x;
-    } else {
-      ev[k2] = 2.f * Y.x;
-      term = (k == 0) ? 0.f : -2.f * Y.y;
-    }
+    unscramble(A[k2], B[k2], uwl[32 * k2 + lane], k2 == 0 && lane == 0, parity, &ev[k2], &term,
+               &yh);
     run += term;
     od[k2] = run;
   }
@@ -414,6 +417,8 @@ template <int P>
 __device__ __forceinline__ void reg_line_core(const LineRegs<P>& r, float* out, int parity,
                                               const float* T, int lane) {
   // T: the lane table of this line length staged in shared memory (lt_* layout)
+  const float2* sn = reinterpret_cast<const float2*>(T + lt_sn(P));
+  const float2* cs = reinterpret_cast<const float2*>(T + lt_cs(P));
   const float2* tw3 = reinterpret_cast<const float2*>(T + lt_tw3(P));
   const float2* tw4 = reinterpret_cast<const float2*>(T + lt_tw4(P));
   const float2* tw5 = reinterpret_cast<const float2*>(T + lt_tw5(P));
@@ -429,56 +434,65 @@ __device__ __forceinline__ void reg_line_core(const LineRegs<P>& r, float* out, 
     float acc = 0.f;
 #pragma unroll
     for (int a = 0; a < P; ++a) {
-      const int j = 2 * (lane + 32 * a);
-      if (j) acc += xp[a].x * T[lt_cs0(P) + 32 * a + lane];
-      acc += xp[a].y * T[lt_cs1(P) + 32 * a + lane];
+      const float2 c = cs[32 * a + lane];
+      if (a || lane) acc += xp[a].x * c.x;
+      acc += xp[a].y * c.y;
     }
     acc = warp_sum(acc);
     sigma = __shfl_sync(FULL, 0.5f * (xp[0].x - xn), 0) + acc;
   }
-  // 2. pre-twiddle: z[a] = y[2m] + i y[2m+1]
+  // 2. pre-twiddle: z[a] = 2 (y[2m] + i y[2m+1]) (the sines carry the factor 2;
+  //    step 4 takes it out)
   float2 z[P];
 #pragma unroll
   for (int a = 0; a < P; ++a) {
-    const int m = lane + 32 * a;
     float r0 = __shfl_sync(FULL, xp[P - 1 - a].x, (32 - lane) & 31);  // x[n - 2m]
     if (lane == 0) r0 = (a == 0) ? xn : xp[(P - a) % P].x;
     const float r1 = __shfl_xor_sync(FULL, xp[P - 1 - a].y, 31);  // x[n - 2m - 1]
-    const float s0 = T[lt_sn0(P) + 32 * a + lane], s1 = T[lt_sn1(P) + 32 * a + lane];
+    const float2 s = sn[32 * a + lane];
     const float x0 = xp[a].x, x1 = xp[a].y;
+    const float p0 = x0 + r0, m0 = x0 - r0, p1 = x1 + r1, m1 = x1 - r1;
     float y0, y1;
     if (parity == 0) {
-      y0 = (m == 0) ? 0.f : s0 * (x0 + r0) + 0.5f * (x0 - r0);
-      y1 = s1 * (x1 + r1) + 0.5f * (x1 - r1);
+      y0 = (a == 0 && lane == 0) ? 0.f : fmaf(s.x, p0, m0);
+      y1 = fmaf(s.y, p1, m1);
     } else {
-      y0 = 0.5f * (x0 + r0) - s0 * (x0 - r0);
-      y1 = 0.5f * (x1 + r1) - s1 * (x1 - r1);
+      y0 = fmaf(-s.x, m0, p0);
+      y1 = fmaf(-s.y, m1, p1);
     }
     z[a] = make_float2(y0, y1);
   }
-  // 3. P-point DFT over a in registers (radix-2 DIF, output in bit-reversed order);
+  // 3. P-point DFT over a in registers: for P = 8 the radix 2 x 4 form, whose
+  //    twiddles are constants; else radix-2 DIF, output in bit-reversed order,
   //    exp(-2 pi i k / 32) = tw[k P]
+  float2 w[P];
+  if constexpr (P == 8) {
+    dft8(z);
 #pragma unroll
-  for (int s = P / 2; s >= 1; s >>= 1) {
+    for (int k2 = 0; k2 < P; ++k2) w[k2] = z[k2];
+  } else {
 #pragma unroll
-    for (int i = 0; i < P; ++i) {
-      if (!(i & s)) {
-        const float2 A = z[i], B = z[i + s];
-        z[i] = make_float2(A.x + B.x, A.y + B.y);
-        float2 D = make_float2(A.x - B.x, A.y - B.y);
-        const int k = (i & (s - 1)) * (16 / s);
-        if (k == 8)
-          D = make_float2(D.y, -D.x);  // exp(-2 pi i 8 / 32) = -i
-        else if (k)
-          D = cmul(D, tw3[k]);
-        z[i + s] = D;
+    for (int s = P / 2; s >= 1; s >>= 1) {
+#pragma unroll
+      for (int i = 0; i < P; ++i) {
+        if (!(i & s)) {
+          const float2 A = z[i], B = z[i + s];
+          z[i] = make_float2(A.x + B.x, A.y + B.y);
+          float2 D = make_float2(A.x - B.x, A.y - B.y);
+          const int k = (i & (s - 1)) * (16 / s);
+          if (k == 8)
+            D = make_float2(D.y, -D.x);  // exp(-2 pi i 8 / 32) = -i
+          else if (k)
+            D = cmul(D, tw3[k]);
+          z[i + s] = D;
+        }
       }
     }
-  }
-  float2 w[P];
 #pragma unroll
-  for (int k2 = 0; k2 < P; ++k2) w[k2] = z[brev_p<P>(k2)];
-  // 4. twiddle exp(-2 pi i lane k2 / (n/2))
+    for (int k2 = 0; k2 < P; ++k2) w[k2] = z[brev_p<P>(k2)];
+  }
+  // 4. twiddle 0.5 exp(-2 pi i lane k2 / (n/2))
+  w[0] = make_float2(0.5f * w[0].x, 0.5f * w[0].y);
 #pragma unroll
   for (int k2 = 1; k2 < P; ++k2) w[k2] = cmul(w[k2], tw4[32 * k2 + lane]);
   if constexpr (line_xs(P)) {
@@ -513,29 +527,10 @@ __device__ __forceinline__ void reg_line_core(const LineRegs<P>& r, float* out, 
   #pragma unroll
     for (int k2 = 0; k2 < P; ++k2) {
       float2 B = (k2 == 0) ? shfl2(w[0], src0) : shfl_xor2(w[(P - k2) % P], 31);
-      B.y = -B.y;
-      const int k = k2 + P * k1;
-      const float2 A = w[k2];
-      float2 Y;
-      if (k == 0) {
-        Y = make_float2(A.x + A.y, 0.f);
-        yh = A.x - A.y;
-      } else {
-        const float2 E = make_float2(0.5f * (A.x + B.x), 0.5f * (A.y + B.y));
-        const float2 D = make_float2(A.x - B.x, A.y - B.y);
-        const float2 q = cmul(uwl[32 * k2 + lane], D);
-        Y = make_float2(E.x + 0.5f * q.y, E.y - 0.5f * q.x);
-      }
-      // sine:   out[2k] = -2 Im Y[k], out[2k+1] = Re Y[0] + 2 sum_{m=1..k} Re Y[m]
-      // cosine: out[2k] =  2 Re Y[k], out[2k+1] = 2 sigma - 2 sum_{m=1..k} Im Y[m]
+      // (k1 is 0 on lane 0 only)
       float term;
-      if (parity == 0) {
-        ev[k2] = (k == 0) ? 0.f : -2.f * Y.y;
-        term = (k == 0) ? Y.x : 2.f * Y.x;
-      } else {
-        ev[k2] = 2.f * Y.x;
-        term = (k == 0) ? 0.f : -2.f * Y.y;
-      }
+      unscramble(w[k2], B, uwl[32 * k2 + lane], k2 == 0 && lane == 0, parity, &ev[k2], &term,
+                 &yh);
       run += term;
       od[k2] = run;
     }

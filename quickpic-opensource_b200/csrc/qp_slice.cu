@@ -32,7 +32,7 @@ namespace {
 __host__ __device__ int col_pitch(int n) { return n + 4; }
 
 template <int P>
-__global__ void __launch_bounds__(256) k_slice_a(SliceA a, GridDims g, KCoef K, LineTables ty,
+__global__ void __launch_bounds__(256, P == 8 ? 4 : P == 16 ? 3 : 0) k_slice_a(SliceA a, GridDims g, KCoef K, LineTables ty,
                                                  const DevStatus* st) {
   extern __shared__ __align__(16) float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -140,8 +140,11 @@ __global__ void __launch_bounds__(256) k_slice_a(SliceA a, GridDims g, KCoef K, 
 
 // 9 warps: warps 0-7 carry the 8 transformed components, warp 8 the optional
 // cbq line (q + cu_z).
+// 1024-point lines: 72 registers, so 3 CTAs per SM (uncapped they take 86, and 2
+// CTAs make the launch 100 us instead of 88).  No cap elsewhere (0): a cap makes
+// the compiler spend registers up to it, which slowed the short lines.
 template <int P>
-__global__ void __launch_bounds__(288) k_slice_b(SliceB b, GridDims g, KCoef K, LineTables ty,
+__global__ void __launch_bounds__(288, P == 16 ? 3 : 0) k_slice_b(SliceB b, GridDims g, KCoef K, LineTables ty,
                                                  DevStatus* st) {
   extern __shared__ __align__(16) float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
