@@ -642,12 +642,18 @@ __global__ void k_nn_norms(NNSlicePlanes p, int nx, int ny, int kp, float* part)
 
 // scales of the slice from the norm partials: epw, current (x, y), current z
 __device__ void nn_scales(const float* part, int nx, int ny, float* sc) {
-  if (threadIdx.x < 3) {
+  // one warp per scale, 5 loads per lane in flight together (a thread that sums
+  // all 148 costs 2 us more per slice)
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (w < 3) {
     float v = 0.f;
-    for (int i = 0; i < NN_NORM_BLOCKS; ++i) v += part[3 * i + threadIdx.x];
-    const float cnt = (float)(nx + 1) * (float)(ny + 1) * (threadIdx.x < 2 ? 2.f : 1.f);
-    const float r = sqrtf(v / cnt);
-    sc[threadIdx.x] = r > 1e-30f ? r : 0.f;
+    for (int i = lane; i < NN_NORM_BLOCKS; i += 32) v += part[3 * i + w];
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) {
+      const float cnt = (float)(nx + 1) * (float)(ny + 1) * (w < 2 ? 2.f : 1.f);
+      const float r = sqrtf(v / cnt);
+      sc[w] = r > 1e-30f ? r : 0.f;
+    }
   }
   __syncthreads();
 }
@@ -1010,7 +1016,7 @@ using namespace qp;
 struct Work {
   static constexpr size_t KEEP = 512u << 20;
   int NB = 0, H = 0, W = 0;
-  unsigned char* slab = nullptr;  // holds every buffer but in32
+  unsigned char* slab = nullptr;  // holds every buffer
   __nv_bfloat16* act[4] = {};
   __nv_bfloat16* dx[4] = {};
   __nv_bfloat16* dy5 = nullptr;
@@ -1023,7 +1029,7 @@ struct Work {
   // buffers and tensor maps for this shape; `host_in`: with room for fp32 input
   int ensure(int nb, int h, int w, bool host_in) {
     const size_t px = (size_t)nb * h * w;
-    if (nb != NB || h != H || w != W) {
+    if (nb != NB || h != H || w != W || (host_in && !in32)) {
       free_all();
       // one allocation, cut into 256-byte aligned buffers
       size_t total = 0;
@@ -1039,7 +1045,8 @@ struct Work {
       }
       const size_t oy = room(px * NN_NLAST * 2), oi = room(px * NN_CIN0 * 2),
                    oo = room(px * NN_OUT * sizeof(float)), ot = room(px * NN_OUT * sizeof(float)),
-                   os = room(nb * sizeof(float));
+                   os = room(nb * sizeof(float)),
+                   o32 = host_in ? room(px * NN_CIN0 * sizeof(float)) : 0;
       if (cudaMalloc(&slab, total) != cudaSuccess) {
         slab = nullptr;
         return -1;
@@ -1057,6 +1064,7 @@ struct Work {
       out32 = reinterpret_cast<float*>(slab + oo);
       target = reinterpret_cast<float*>(slab + ot);
       scale = reinterpret_cast<float*>(slab + os);
+      in32 = host_in ? reinterpret_cast<float*>(slab + o32) : nullptr;
       if (tile_map(&dy5_tile, dy5, NN_NLAST / 8, nb, h, w) ||
           halo_map(&dy5_halo, dy5, NN_NLAST / 8, nb, h, w) ||
           halo_map(&img_halo, img, NN_CIN0 / 8, nb, h, w))
@@ -1065,8 +1073,6 @@ struct Work {
       H = h;
       W = w;
     }
-    if (host_in && !in32 && cudaMalloc(&in32, px * NN_CIN0 * sizeof(float)) != cudaSuccess)
-      return -1;
     return 0;
   }
   // after a call: give back what is too large to keep, or incomplete
@@ -1078,7 +1084,6 @@ struct Work {
   }
   void free_all() {
     if (slab) cudaFree(slab);
-    if (in32) cudaFree(in32);
     slab = nullptr;
     for (int i = 0; i < 4; ++i) act[i] = dx[i] = nullptr;
     dy5 = img = nullptr;
