@@ -81,7 +81,6 @@ struct __align__(16) DevStatus {
   int cursor;         // slice cursor of the fused 3D step (moved on by k_slice_a)
   int pass_done;      // convergence-controlled B loop: the pass of this slice
                       // whose residual met the tolerance (0 = none yet)
-  int unused0;
   int beam_drops;     // beam particles dropped at the conducting boundary
   float resid_num;    // residual of the current pass: sum |epw - epw_old|^2
   float resid_den;    //                               sum |epw|^2
@@ -111,7 +110,7 @@ __device__ __forceinline__ bool pass_skipped(const DevStatus* st, int pass) {
 }
 
 // The words of the device status a slice kernel checks before its work, read
-// with two 16-byte loads (error .. need_inbox, cursor .. beam_drops) that a
+// with two 16-byte loads (error .. need_inbox, cursor ..) that a
 // kernel issues together with its first data loads.
 struct StatusSnap {
   int error, cursor, pass_done;
@@ -120,10 +119,6 @@ __device__ __forceinline__ StatusSnap status_snap(const DevStatus* st) {
   const int4* p = reinterpret_cast<const int4*>(st);
   const int4 a = p[0], b = p[1];
   return StatusSnap{a.x, b.x, b.y};
-}
-// pass_skipped on a snapshot
-__device__ __forceinline__ bool snap_skipped(const StatusSnap& s, int pass) {
-  return pass > 1 && s.pass_done > 0 && s.pass_done < pass;
 }
 
 enum { QP_OK = 0, QP_OVERFLOW = 1 };

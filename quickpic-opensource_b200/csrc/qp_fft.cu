@@ -160,7 +160,6 @@ __global__ void __launch_bounds__(256) k_xfwd(XJob job, GridDims g, LineTables t
   if (P > 0) stage_lane_table(T, tx);  // constant tables: staged before the wait
   grid_dep_sync();
   if (st && st->error) return;
-  if (pass_skipped(st, job.pass)) return;
   const XComp c = job.c[blockIdx.y];
   if (c.cursor_stride && !cursor_ok(c, st)) return;
   xfwd_rows<P>(c, blockIdx.x * 8, g, tx, smem, T, st);
@@ -222,16 +221,10 @@ __global__ void __launch_bounds__(256) k_xinv(XJob job, GridDims g, LineTables t
   if (P > 0) stage_lane_table(T, tx);
   grid_dep_sync();
   if (st && st->error) return;
-  if (pass_skipped(st, job.pass)) return;
   const XComp c = job.c[blockIdx.y];
   if (c.cursor_stride && !cursor_ok(c, st)) return;
   const int y0 = blockIdx.x * 8;
   xinv_rows<P>(c, y0, g, tx, smem, T, st);
-  for (int z = blockIdx.y; z < job.nzero; z += job.ncomp) {
-    float* p = job.zero[z] + (long long)y0 * g.rp;
-    const int rows = min(8, g.ny + 1 - y0);
-    for (int i = threadIdx.x; i < rows * g.rp; i += 256) p[i] = 0.f;
-  }
 }
 
 // Inverse x pass of node-major fields.  A CTA takes two rows of one group of
@@ -240,6 +233,8 @@ __global__ void __launch_bounds__(256) k_xinv(XJob job, GridDims g, LineTables t
 // result is one float4 of the [y][x][4] array -- 5 loads and 5 stores of 16
 // bytes per thread at 512 points, where the planar form makes 17 of 4 bytes
 // each.  The remaining CTAs transform planar components, 8 rows each.
+// Bound by latency and the transforms' shared-memory and shuffle traffic: 14.2
+// -> 14.0 us at 512 x 512 (five components).
 template <int P>
 __global__ void __launch_bounds__(256) k_xinv4(const __grid_constant__ X4Job job, GridDims g,
                                                LineTables tx, const DevStatus* st) {
@@ -250,7 +245,7 @@ __global__ void __launch_bounds__(256) k_xinv4(const __grid_constant__ X4Job job
   if (P > 0) stage_lane_table(T, tx);  // constant tables: staged before the wait
   grid_dep_sync();
   if (st && st->error) return;
-  if (pass_skipped(st, job.x.pass)) return;
+  if (pass_skipped(st, job.pass)) return;
   float* L = smem + warp * pitch;
   float* S = smem + (8 + warp) * pitch;
   const int pairs = g.ny >> 1;
@@ -301,9 +296,9 @@ __global__ void __launch_bounds__(256) k_xinv4(const __grid_constant__ X4Job job
   // the zero planes, a share per CTA (planes are multiples of 16 bytes)
   const long long n4 = g.rplane >> 2, share = (n4 + gridDim.x - 1) / gridDim.x;
   const long long lo = share * blockIdx.x, hi = min(n4, lo + share);
-  for (int z = 0; z < job.x.nzero; ++z)
+  for (int z = 0; z < job.nzero; ++z)
     for (long long i = lo + threadIdx.x; i < hi; i += 256)
-      reinterpret_cast<float4*>(job.x.zero[z])[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      reinterpret_cast<float4*>(job.zero[z])[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // Forward x pass of node-major densities.  A CTA takes one row, its 8 warps
@@ -313,6 +308,10 @@ __global__ void __launch_bounds__(256) k_xinv4(const __grid_constant__ X4Job job
 // a node of the transposed result is one full 32-byte sector -- 5 loads and 5
 // stores of 16 bytes per thread at 512 points, where the planar form loads 8
 // bytes and stores 4 at a time.  Planar components follow, 8 rows per CTA.
+// Bound by the transforms' shared-memory and shuffle traffic: 14.7 us at 512 x
+// 512 (9.4 MB in and out); the planar form took 13.3, the staging through
+// shared memory being the price of the densities' vector reductions (amjdp
+// 2.3 us less per pass).
 template <int P>
 __global__ void __launch_bounds__(256, P == 8 ? 4 : P == 16 ? 3 : 0) k_xfwd8(const __grid_constant__ X8Job job, GridDims g,
                                                LineTables tx, const DevStatus* st) {
@@ -323,7 +322,7 @@ __global__ void __launch_bounds__(256, P == 8 ? 4 : P == 16 ? 3 : 0) k_xfwd8(con
   if (P > 0) stage_lane_table(T, tx);  // constant tables: staged before the wait
   grid_dep_sync();
   if (st && st->error) return;
-  if (pass_skipped(st, job.x.pass)) return;
+  if (pass_skipped(st, job.pass)) return;
   if ((int)blockIdx.x >= g.ny) {
     const int b = (int)blockIdx.x - g.ny, per = (g.ny + 8) >> 3;
     const XComp c = job.x.c[b / per];

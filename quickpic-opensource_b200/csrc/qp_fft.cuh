@@ -34,11 +34,6 @@ struct XComp {
 struct XJob {
   XComp c[QP_MAX_JOB];
   int ncomp;
-  // xinv only: real-space planes whose rows this launch clears (plane i is
-  // cleared by the CTAs of component i % ncomp)
-  float* zero[16];
-  int nzero;
-  int pass;  // predictor-corrector pass of the launch (pass_skipped), 0 = none
 };
 
 struct YComp {
@@ -61,13 +56,16 @@ void launch_xinv(const XJob& job, const GridDims& g, const LineTables& tx, const
 // Inverse x pass of the fused step's node-major fields: group g is
 // src [kx][y][4] -> dst [y][x][4] with the x parities par[g]; planar components
 // (c[0..ncomp), as launch_xinv) ride along, and the launch clears the zero
-// planes of the job.
+// planes.
 struct X4Job {
   const float4* src[2];
   float4* dst[2];
   int par[2][4];
   int ngroup;
   XJob x;
+  float* zero[16];  // planes that this launch clears
+  int nzero;
+  int pass;  // predictor-corrector pass of the launch (pass_skipped), 0 = none
 };
 void launch_xinv4(const X4Job& job, const GridDims& g, const LineTables& tx, const DevStatus* st,
                   cudaStream_t s);
@@ -79,6 +77,7 @@ struct X8Job {
   float4* dst;
   int par[8];
   XJob x;
+  int pass;  // as X4Job
 };
 void launch_xfwd8(const X8Job& job, const GridDims& g, const LineTables& tx, const DevStatus* st,
                   cudaStream_t s);

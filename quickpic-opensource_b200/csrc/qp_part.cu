@@ -90,7 +90,6 @@ __device__ __forceinline__ void stage_fields(FieldTile& s, float* spsi, const Ga
         vb[k] = make_float4(f.psit[o], f.bx[o], f.by[o], f.bz[o]);
         vf[k].x = f.fx[o];
         vf[k].y = f.fy[o];
-        if (f.psi) vf[k].z = f.psi[o];
       }
     }
   }
@@ -451,8 +450,11 @@ __device__ __forceinline__ void deposit_last(const Densities& d, const TileGeom&
 }
 
 // The half push and the deposit of 8 densities x 4 corners.  Bound by issue
-// (about 380 instructions per particle) and by the reductions in L2, not by
-// memory.
+// (about 380 instructions per particle, 57 % of issue slots at 3 CTAs per SM)
+// and by the reductions in L2, not by memory.  Node-major fields and densities:
+// 27.0 -> 24.7 us at 512 x 512 with 2 x 2 particles per cell (28 MB: 1.1 TB/s),
+// 79.5 -> 73.7 us at 1024 x 1024; without handing right corners to the next
+// lane 27.4 us.
 // Each thread takes 4 consecutive particles (float4 loads of each component)
 // and keeps the deposits of a run of particles in one cell in registers,
 // adding them to the global planes when the cell changes (deposit_run).  With
@@ -462,7 +464,8 @@ __device__ __forceinline__ void deposit_last(const Densities& d, const TileGeom&
 // summed differs.  The planes must be zero on entry.
 // K = 4 particles per thread and CTA = tile is the form for grids that fill the
 // GPU.  Grids of few tiles leave most of it idle and wait for one CTA's serial
-// work: there two CTAs share a tile with 2 particles per thread.
+// work: there two CTAs share a tile with 2 particles per thread (64 x 64 grid:
+// 10.8 -> 9.0 us, 128 x 128: 11.9 -> 10.2).
 template <bool NODE, int K>
 __global__ void __launch_bounds__(256, 3) k_amjdp(PartBuf P, TileGeom tg, GatherPlanes f,
                                                   const __grid_constant__ Densities den, float qbm,
@@ -476,7 +479,7 @@ __global__ void __launch_bounds__(256, 3) k_amjdp(PartBuf P, TileGeom tg, Gather
   const int t = blockIdx.x;
   int noffp, moffp;
   tile_origin(tg, t, &noffp, &moffp);
-  const bool ext = f.ext || f.psi != nullptr;
+  const bool ext = NODE && f.ext;
   // the count is read with the field planes, so the two waits overlap
   const int n = P.count[t];
   stage_fields<NODE>(sf, ext ? spsi : nullptr, f, tg, noffp, moffp);
@@ -586,6 +589,11 @@ __global__ void __launch_bounds__(256, 3) k_amjdp(PartBuf P, TileGeom tg, Gather
 // counts, and the chunk needs four CTA barriers.  Movers go to the
 // destination tile's inbox with a (cell, source tile, source slot) key, which
 // the insert kernel sorts, so they too arrive in cell order.
+// Bound by issue (550 instructions per particle, 68 % of issue slots; its
+// divisions and roots are the reference's IEEE operations): 32 us at 512 x 512
+// (1.9 TB/s with the slice's stores, which were a launch of 10.7 us and cost
+// 1.3 us here).  A chunk of 1152 slots, which would hold a tile of 1024 and its
+// movers, is slower (35 us): five rounds per warp, the last half empty.
 constexpr int PUSH_CHUNK = 1024;
 
 template <int MODE>
@@ -1059,7 +1067,9 @@ void launch_amjdp_node(const PartBuf& P, const TileGeom& tg, const GatherPlanes&
   Densities d{};
   d.node = node;
   d.cz = cz;
-  // two CTAs per tile while they all fit at once: 3 per SM of 148
+  // two CTAs per tile while they all fit at once, 3 per SM of 148 = 444; past
+  // that a second wave costs more than it saves (256 x 256, 512 CTAs at the 4
+  // per SM that 64 registers allow: 14.8 us against 14.4)
   if (tg.ntiles <= 222)
     launch_pdl(k_amjdp<true, 2>, dim3(tg.ntiles, 2), 256, 0, s, P, tg, f, d, qbm, dt, dex, scale,
                const_cast<DevStatus*>(st));

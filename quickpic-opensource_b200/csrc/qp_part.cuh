@@ -42,8 +42,7 @@ struct GatherPlanes {
   const float* bz;   // bxyz(3)
   const float* psit; // psit
   int combine;       // 1: the push uses -fxy + (by, -bx), the final slice force
-  const float* psi;  // amjdp only, optional: form p6, p7 from psi first (extpsi)
-  int ext;           // amjdp only: the same with psi from ff
+  int ext;           // amjdp only: form p6, p7 from psi first (extpsi); node-major fields
   int pass;          // amjdp only: predictor-corrector pass (pass_skipped), 0 = none
   float* zero_q;     // push only, optional: clear the charge-plane nodes this tile
                      // owns (k_insert then deposits the next slice's charge)
