@@ -445,7 +445,10 @@ int qp_sim_profile(qp_sim* sim, int nslices, char* names, int names_len, double*
  * dx the row and column offsets + 1) then bias[cout]; cin = 16 for layer 1
  * (9 input features, the rest zero), 32 otherwise; cout = 32, and 16 for
  * layer 5 (2 outputs used).  An untrained network (seeded He initialisation,
- * last layer zero) is the quadratic extrapolation. */
+ * last layer zero) is the quadratic extrapolation.
+ * Calls on one network may come from several host threads: they take turns.
+ * (A simulation that starts its passes from a network reads its weights
+ * outside of those turns: change them between steps only.) */
 typedef struct qp_nn qp_nn;
 typedef struct qp_nn_data qp_nn_data;
 int qp_nn_create(int device, unsigned long long seed, qp_nn** out);

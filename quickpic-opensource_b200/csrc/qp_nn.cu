@@ -1014,7 +1014,8 @@ using namespace qp;
 
 // Work buffers of one forward/backward over NB images of H x W, kept with the
 // network between calls of one shape (a gradient call spent 1 ms on its 14
-// allocations) as long as they are no larger than KEEP bytes.
+// allocations) as long as they are no larger than KEEP bytes.  One call uses
+// them at a time, from ensure() to settle() (qp_nn::mu).
 struct Work {
   static constexpr size_t KEEP = 512u << 20;
   int NB = 0, H = 0, W = 0;
@@ -1112,6 +1113,9 @@ struct qp_nn {
   int* err = nullptr;
   float* loss = nullptr;
   Work wk;  // of the last call's shape
+  // held by a call that runs on the network's buffers until its results are on
+  // the host: calls from several threads take turns
+  std::mutex mu;
 };
 
 // Training pairs recorded by a simulation: 128 x 128 crops (the low modes) of
@@ -1362,12 +1366,14 @@ extern "C" int qp_nn_num_params(const qp_nn* nn) { return nn ? nn->nparams : -1;
 
 extern "C" int qp_nn_get_params(qp_nn* nn, float* out) {
   if (!nn || !out) return nn_fail(__LINE__, "null argument");
+  std::lock_guard<std::mutex> turn(nn->mu);
   NK(cudaMemcpy(out, nn->master, sizeof(float) * nn->nparams, cudaMemcpyDeviceToHost));
   return 0;
 }
 
 extern "C" int qp_nn_set_params(qp_nn* nn, const float* in) {
   if (!nn || !in) return nn_fail(__LINE__, "null argument");
+  std::lock_guard<std::mutex> turn(nn->mu);
   NK(cudaMemcpyAsync(nn->master, in, sizeof(float) * nn->nparams, cudaMemcpyHostToDevice,
                      nn->stream));
   if (nn_pack(nn, nn->stream)) return -1;
@@ -1398,6 +1404,7 @@ int check_shape(int NB, int H, int W) {
 extern "C" int qp_nn_forward(qp_nn* nn, const float* in, int NB, int H, int W, float* out) {
   if (!nn || !in || !out) return nn_fail(__LINE__, "null argument");
   if (check_shape(NB, H, W)) return -1;
+  std::lock_guard<std::mutex> turn(nn->mu);
   cudaSetDevice(nn->device);
   cudaStream_t s = nn->stream;
   Work& wk = nn->wk;
@@ -1421,6 +1428,7 @@ extern "C" int qp_nn_loss_grad(qp_nn* nn, const float* in, const float* target, 
                                int W, double* loss, float* grad) {
   if (!nn || !in || !target || !grad) return nn_fail(__LINE__, "null argument");
   if (check_shape(NB, H, W)) return -1;
+  std::lock_guard<std::mutex> turn(nn->mu);
   cudaSetDevice(nn->device);
   cudaStream_t s = nn->stream;
   Work& wk = nn->wk;
@@ -1512,6 +1520,7 @@ extern "C" int qp_nn_train(qp_nn* nn, qp_nn_data* t, const qp_nn_train_desc* d,
   if (!nn || !t || !d) return nn_fail(__LINE__, "null argument");
   if (t->count < d->batch || d->batch < 1 || d->steps < 1 || !(d->lr > 0.f))
     return nn_fail(__LINE__, "training: bad settings, or fewer pairs than one minibatch");
+  std::lock_guard<std::mutex> turn(nn->mu);
   cudaSetDevice(nn->device);
   cudaStream_t s = nn->stream;
   const int B = d->batch, H = NN_CROP, W = NN_CROP;
