@@ -82,8 +82,12 @@ def _ints(v):
     return (C.c_int * len(v))(*map(int, v))
 
 
-def _floats(v):
-    return (C.c_float * len(v))(*map(float, v))
+def _floats(v, n):
+    """The values of n components; one number stands for all of them."""
+    try:
+        return (C.c_float * len(v))(*map(float, v))
+    except TypeError:  # a number, also a numpy one
+        return (C.c_float * n)(*[float(v)] * n)
 
 
 class _GridDesc(C.Structure):
@@ -269,7 +273,7 @@ class Field2d:
             self._c(self.ctx._L.qp_field2d_mult(self.h, a1.h, C.c_float(value)))
         else:
             self._c(self.ctx._L.qp_field2d_mult_comp(self.h, a1.h, _ints(dim), _ints(dim1),
-                                                     _floats(value), len(dim)))
+                                                     _floats(value, len(dim)), len(dim)))
 
     def cg(self):
         self._c(self.ctx._L.qp_field2d_cg(self.h))

@@ -79,3 +79,30 @@ def test_descriptor_layouts_match_the_header(qp, tmp_path):
         assert got[(pyname, "size")] == C.sizeof(st), pyname
         for fname, _ in st._fields_:
             assert got[(pyname, fname)] == getattr(st, fname).offset, (pyname, fname)
+
+
+def test_component_values_may_be_one_number(qp):
+    """Field2d.mult with component lists takes a sequence of values or one
+    number; what reaches the C call is one value per component."""
+    import types
+
+    import numpy as np
+
+    seen = []
+
+    def comp(h, a1, dim, dim1, value, n):
+        seen.append((list(dim), list(dim1), list(value), n))
+        return 0
+
+    f = qp.Field2d.__new__(qp.Field2d)
+    f.h = 1
+    f.ctx = types.SimpleNamespace(_L=types.SimpleNamespace(qp_field2d_mult_comp=comp),
+                                  _check=lambda rc: rc)
+    for value, want in [(2.0, [2.0]), (3, [3.0]), (np.float32(0.5), [0.5]), (np.array(4.0), [4.0]),
+                        ([1.5], [1.5]), (np.array([2.5]), [2.5])]:
+        f.mult(f, value, dim=[1], dim1=[2])
+        assert seen[-1] == ([1], [2], want, 1)
+    f.mult(f, 2.0, dim=[1, 3], dim1=(2, 1))
+    assert seen[-1] == ([1, 3], [2, 1], [2.0, 2.0], 2)
+    f.mult(f, [2.0, 3.0], dim=np.array([1, 2]), dim1=[2, 1])
+    assert seen[-1] == ([1, 2], [2, 1], [2.0, 3.0], 2)
