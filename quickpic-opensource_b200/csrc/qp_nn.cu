@@ -235,6 +235,7 @@ struct ConvArgs {
   int H, W, NB;               // output images (NB images of H x W)
   int b0;                     // first image of the launch in the input map
   int* err;                   // device error flag (nonzero on a wait that expired)
+  const DevStatus* st;        // the step's status, or null outside of a step
 };
 
 __device__ __forceinline__ void flag_error(int* err, int code) {
@@ -324,7 +325,10 @@ __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtenso
   };
   const int step = (int)gridDim.x;
   bool bad = false;
-  if (tid == 0 && (int)blockIdx.x < ntiles) {
+  // a step whose status holds an error leaves every plane as it is (one
+  // decision for the CTA, whose barriers and tensor-memory loads follow)
+  const bool skip = a.st && __syncthreads_or(a.st->error) != 0;
+  if (tid == 0 && !skip && (int)blockIdx.x < ntiles) {
     issue(blockIdx.x, 0);
     pf_k = 0;
     if ((int)blockIdx.x + step < ntiles) {
@@ -336,7 +340,7 @@ __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtenso
   // a wait that expired in any thread ends the loop for all of them
   bool failed = __syncthreads_or(bad) != 0;
   int k = 0;
-  for (int t = blockIdx.x; t < ntiles && !failed; t += step, ++k) {
+  for (int t = blockIdx.x; t < ntiles && !failed && !skip; t += step, ++k) {
     const int buf = k & 1;
     // every thread waits for the accumulator (bounded)
     bad = !mbar_wait(&bar[2 + buf], (uint32_t)((k >> 1) & 1));
@@ -427,7 +431,7 @@ __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtenso
   }
   // EPI_EPW: the modes outside the conv image (the network's low-mode window)
   // take the quadratic extrapolation alone, spread over every CTA
-  if (EPI == EPI_EPW && !failed) {
+  if (EPI == EPI_EPW && !failed && !skip) {
     const long long nm = (long long)(a.nx + 1) * (a.ny + 1);
     for (long long i = (long long)blockIdx.x * 128 + tid; i < nm; i += (long long)gridDim.x * 128) {
       const int kx = (int)(i / (a.ny + 1)), ky = (int)(i - (long long)kx * (a.ny + 1));
@@ -608,8 +612,10 @@ __global__ void __launch_bounds__(128) k_wgrad(const __grid_constant__ CUtensorM
 }
 
 // ------------------------------------------------------- features and records
-__global__ void k_nn_norms(NNSlicePlanes p, int nx, int ny, int kp, float* part) {
+__global__ void k_nn_norms(NNSlicePlanes p, int nx, int ny, int kp, float* part,
+                           const DevStatus* st) {
   grid_dep_sync();
+  if (st->error) return;
   __shared__ float red[3][8];
   float sb = 0.f, sj = 0.f, sz = 0.f;
   const long long n = (long long)(nx + 1) * (ny + 1);
@@ -695,8 +701,10 @@ __device__ __forceinline__ void nn_feature(const NNSlicePlanes& p, size_t o, int
 // inference: the input image [2][1][hc][wc][8] of the slice's low-mode
 // window kx < hc, ky < wc; scale_out = the epw scale
 __global__ void k_nn_features(NNSlicePlanes p, int nx, int ny, int kp, int hc, int wc,
-                              const float* part, __nv_bfloat16* img, float* scale_out) {
+                              const float* part, __nv_bfloat16* img, float* scale_out,
+                              const DevStatus* st) {
   grid_dep_sync();
+  if (st->error) return;
   __shared__ float sc[3];
   nn_scales(part, nx, ny, sc);
   if (blockIdx.x == 0 && threadIdx.x == 0) scale_out[0] = sc[0];
@@ -724,8 +732,9 @@ struct NNData {
 // slot = -(quadratic start) / scale, the scale; then the history moves one slice on
 // for every mode (epw_prev2 <- epw_prev, epw_prev <- epw)
 __global__ void k_nn_record_start(NNSlicePlanes p, int nx, int ny, int kp, const float* part,
-                                  NNData d, int slot) {
+                                  NNData d, int slot, const DevStatus* st) {
   grid_dep_sync();
+  if (st->error) return;
   __shared__ float sc[3];
   nn_scales(part, nx, ny, sc);
   if (blockIdx.x == 0 && threadIdx.x == 0) d.scale[slot] = sc[0];
@@ -756,8 +765,9 @@ __global__ void k_nn_record_start(NNSlicePlanes p, int nx, int ny, int kp, const
 }
 
 // recording, slice end: target slot += converged epw / scale
-__global__ void k_nn_record_end(NNSlicePlanes p, int kp, NNData d, int slot) {
+__global__ void k_nn_record_end(NNSlicePlanes p, int kp, NNData d, int slot, const DevStatus* st) {
   grid_dep_sync();
+  if (st->error) return;
   const float sB = d.scale[slot];
   const size_t C2 = (size_t)NN_CROP * NN_CROP;
   float* t = d.target + (size_t)slot * 2 * C2;
@@ -774,8 +784,9 @@ __global__ void k_nn_record_end(NNSlicePlanes p, int kp, NNData d, int slot) {
 // changes shape abruptly, mostly at the head of the beam) is not a
 // correction the network can learn from; its scale is set to 0, which takes
 // it out of the loss
-__global__ void k_nn_record_validate(NNData d, int slot) {
+__global__ void k_nn_record_validate(NNData d, int slot, const DevStatus* st) {
   grid_dep_sync();
+  if (st->error) return;
   __shared__ float red[32];
   const size_t C2 = (size_t)NN_CROP * NN_CROP;
   const float* t = d.target + (size_t)slot * 2 * C2;
@@ -1195,8 +1206,9 @@ const float* nn_bias(const qp_nn* nn, int l) {
 int nn_forward(qp_nn* nn, const CUtensorMap& in_map, int b0, __nv_bfloat16* const* act,
                const CUtensorMap* act_map, int NB, int H, int W, float* out32,
                const NNSlicePlanes* pl, const float* scale, int kp, int nx, int ny,
-               cudaStream_t s) {
+               const DevStatus* st, cudaStream_t s) {
   ConvArgs a{};
+  a.st = st;
   a.H = H;
   a.W = W;
   a.NB = NB;
@@ -1411,7 +1423,7 @@ extern "C" int qp_nn_forward(qp_nn* nn, const float* in, int NB, int H, int W, f
   int rc = wk.ensure(NB, H, W, true) ? nn_fail(__LINE__, "out of device memory (network)")
                                      : upload_images(nn, in, s);
   if (!rc) rc = nn_forward(nn, wk.img_halo, 0, wk.act, wk.act_halo, NB, H, W, wk.out32, nullptr,
-                           nullptr, 0, 0, 0, s);
+                           nullptr, 0, 0, 0, nullptr, s);
   if (!rc && cudaMemcpyAsync(out, wk.out32, sizeof(float) * NN_OUT * (size_t)NB * H * W,
                              cudaMemcpyDeviceToHost, s) != cudaSuccess)
     rc = nn_fail(__LINE__, "download failed");
@@ -1439,7 +1451,7 @@ extern "C" int qp_nn_loss_grad(qp_nn* nn, const float* in, const float* target, 
                              s) != cudaSuccess)
     rc = nn_fail(__LINE__, "upload failed");
   if (!rc) rc = nn_forward(nn, wk.img_halo, 0, wk.act, wk.act_halo, NB, H, W, wk.out32, nullptr,
-                           nullptr, 0, 0, 0, s);
+                           nullptr, 0, 0, 0, nullptr, s);
   float l = 0.f;
   if (!rc) {
     NNData d{NB, wk.img, wk.target, wk.scale};
@@ -1554,7 +1566,7 @@ extern "C" int qp_nn_train(qp_nn* nn, qp_nn_data* t, const qp_nn_train_desc* d,
     // the learning rate steps down to 0.3 and 0.1 of its start at 1/2 and 3/4 of the run
     const float lr = d->lr * (it < d->steps / 2 ? 1.f : (it < 3 * d->steps / 4 ? 0.3f : 0.1f));
     rc = nn_forward(nn, wk.img_halo, 0, wk.act, wk.act_halo, B, H, W, wk.out32, nullptr, nullptr,
-                    0, 0, 0, s);
+                    0, 0, 0, nullptr, s);
     if (rc) break;
     launch_pdl(k_nn_loss, 256, 256, 0, s, wk.out32, bt, 0, B, H, W, inv_n, wk.dy5, hist + it);
     rc = nn_backward(nn, wk.img_halo, 0, wk.act, wk.act_halo, wk.dy5, wk.dy5_tile, wk.dy5_halo,
@@ -1642,44 +1654,49 @@ void nn_runtime_destroy(NNRuntime* r) {
 }
 
 int nn_predict(NNRuntime* r, const void* net, const NNSlicePlanes& p, const GridDims& g,
-               DevStatus* st, cudaStream_t s) {
+               const DevStatus* st, cudaStream_t s) {
   qp_nn* nn = const_cast<qp_nn*>(static_cast<const qp_nn*>(net));
-  launch_pdl(k_nn_norms, NN_NORM_BLOCKS, 256, 0, s, p, g.nx, g.ny, g.kp, r->part);
+  launch_pdl(k_nn_norms, NN_NORM_BLOCKS, 256, 0, s, p, g.nx, g.ny, g.kp, r->part, st);
   launch_pdl(k_nn_features, NN_NORM_BLOCKS, 256, 0, s, p, g.nx, g.ny, g.kp, r->hc, r->wc, r->part,
-                                                r->img, r->scale);
+             r->img, r->scale, st);
   // layers 1-4 ping-pong between the two activation buffers; every layer's
   // input is the previous output, so the four maps cycle through them
   __nv_bfloat16* act[4] = {r->act[0], r->act[1], r->act[0], r->act[1]};
   const CUtensorMap amap[4] = {r->m_act[0], r->m_act[1], r->m_act[0], r->m_act[1]};
   if (nn_forward(nn, r->m_img, 0, act, amap, 1, r->hc, r->wc, nullptr, &p, r->scale, g.kp, g.nx,
-                 g.ny, s))
+                 g.ny, st, s))
     return -1;
-  (void)st;
   return 7;
 }
 
 int nn_record_start(NNRuntime* r, void* data, const NNSlicePlanes& p, const GridDims& g,
-                    DevStatus* st, cudaStream_t s) {
+                    const DevStatus* st, cudaStream_t s) {
   qp_nn_data* t = static_cast<qp_nn_data*>(data);
-  (void)st;
   if (t->count >= t->d.cap) return 0;
   const int slot = t->count;
-  launch_pdl(k_nn_norms, NN_NORM_BLOCKS, 256, 0, s, p, g.nx, g.ny, g.kp, r->part);
-  launch_pdl(k_nn_record_start, NN_NORM_BLOCKS * 4, 256, 0, s, p, g.nx, g.ny, g.kp, r->part, t->d, slot);
+  launch_pdl(k_nn_norms, NN_NORM_BLOCKS, 256, 0, s, p, g.nx, g.ny, g.kp, r->part, st);
+  launch_pdl(k_nn_record_start, NN_NORM_BLOCKS * 4, 256, 0, s, p, g.nx, g.ny, g.kp, r->part, t->d, slot,
+             st);
   return 2;
 }
 
 int nn_record_end(NNRuntime* r, void* data, const NNSlicePlanes& p, const GridDims& g,
-                  DevStatus* st, cudaStream_t s) {
+                  const DevStatus* st, cudaStream_t s) {
   qp_nn_data* t = static_cast<qp_nn_data*>(data);
   (void)r;
-  (void)st;
   if (t->count >= t->d.cap) return 0;
   const int slot = t->count;
-  launch_pdl(k_nn_record_end, 64, 256, 0, s, p, g.kp, t->d, slot);
-  launch_pdl(k_nn_record_validate, 1, 1024, 0, s, t->d, slot);
+  launch_pdl(k_nn_record_end, 64, 256, 0, s, p, g.kp, t->d, slot, st);
+  launch_pdl(k_nn_record_validate, 1, 1024, 0, s, t->d, slot, st);
   t->count++;
   return 2;
+}
+
+int nn_record_count(const void* data) { return static_cast<const qp_nn_data*>(data)->count; }
+
+void nn_record_rewind(void* data, int count) {
+  qp_nn_data* t = static_cast<qp_nn_data*>(data);
+  t->count = std::min(t->count, count);
 }
 
 }  // namespace qp

@@ -61,16 +61,21 @@ struct NNRuntime;  // per-simulation buffers and tensor maps (qp_nn.cu)
 // Per-simulation inference set-up on an nx x ny grid (ny a multiple of 128).
 int nn_runtime_create(const GridDims& g, NNRuntime** out);
 void nn_runtime_destroy(NNRuntime* r);
+// Like the step's other kernels, those below do nothing once st->error is set.
 // The start of slice j from the network (norms, features, 5 conv layers).
-// Returns the number of launches; st->error set on a device-side failure.
+// Returns the number of launches.
 int nn_predict(NNRuntime* r, const void* net, const NNSlicePlanes& p, const GridDims& g,
-               DevStatus* st, cudaStream_t s);
+               const DevStatus* st, cudaStream_t s);
 // Recording of training pairs: at the start of slice j (features of the crop,
 // minus the quadratic extrapolation into the target slot; the history moves on),
 // and at its end (plus the converged epw).  Both skip once the set is full.
+// The count of pairs goes on as the slices are enqueued; nn_record_rewind takes
+// it back to `count` when the last of them did not run.
 int nn_record_start(NNRuntime* r, void* data, const NNSlicePlanes& p, const GridDims& g,
-                    DevStatus* st, cudaStream_t s);
+                    const DevStatus* st, cudaStream_t s);
 int nn_record_end(NNRuntime* r, void* data, const NNSlicePlanes& p, const GridDims& g,
-                  DevStatus* st, cudaStream_t s);
+                  const DevStatus* st, cudaStream_t s);
+int nn_record_count(const void* data);
+void nn_record_rewind(void* data, int count);
 
 }  // namespace qp
