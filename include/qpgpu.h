@@ -454,6 +454,10 @@ typedef struct qp_nn_data qp_nn_data;
 int qp_nn_create(int device, unsigned long long seed, qp_nn** out);
 int qp_nn_destroy(qp_nn* nn);
 int qp_nn_num_params(const qp_nn* nn);
+/* Sets the network's error flag (0 clears it), as its kernels do when one of
+ * their bounded waits expires.  While it is set, calls that run the network
+ * fail, and so does a 3D step that starts its passes from it. */
+int qp_nn_flag_error(qp_nn* nn, int code);
 int qp_nn_get_params(qp_nn* nn, float* out);
 int qp_nn_set_params(qp_nn* nn, const float* in);
 /* Forward of nb images in[nb][16][h][w] (w a multiple of 128) to

@@ -235,7 +235,7 @@ struct ConvArgs {
   int H, W, NB;               // output images (NB images of H x W)
   int b0;                     // first image of the launch in the input map
   int* err;                   // device error flag (nonzero on a wait that expired)
-  const DevStatus* st;        // the step's status, or null outside of a step
+  DevStatus* st;              // the step's status, or null outside of a step
 };
 
 __device__ __forceinline__ void flag_error(int* err, int code) {
@@ -325,9 +325,10 @@ __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtenso
   };
   const int step = (int)gridDim.x;
   bool bad = false;
-  // a step whose status holds an error leaves every plane as it is (one
-  // decision for the CTA, whose barriers and tensor-memory loads follow)
-  const bool skip = a.st && __syncthreads_or(a.st->error) != 0;
+  // a step whose status holds an error leaves every plane as it is, and so does
+  // a network that has failed before (one decision for the CTA, whose barriers
+  // and tensor-memory loads follow)
+  const bool skip = a.st && __syncthreads_or(a.st->error | *a.err) != 0;
   if (tid == 0 && !skip && (int)blockIdx.x < ntiles) {
     issue(blockIdx.x, 0);
     pf_k = 0;
@@ -429,6 +430,8 @@ __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtenso
       mbar_wait(&bar[2 + (j & 1)], (uint32_t)((j >> 1) & 1));
     flag_error(a.err, 1);
   }
+  // a step ends with an error once its network has failed
+  if (tid == 0 && a.st && *(volatile int*)a.err) atomicCAS(&a.st->error, 0, NN_STATUS_FAILED);
   // EPI_EPW: the modes outside the conv image (the network's low-mode window)
   // take the quadratic extrapolation alone, spread over every CTA
   if (EPI == EPI_EPW && !failed && !skip) {
@@ -1206,7 +1209,7 @@ const float* nn_bias(const qp_nn* nn, int l) {
 int nn_forward(qp_nn* nn, const CUtensorMap& in_map, int b0, __nv_bfloat16* const* act,
                const CUtensorMap* act_map, int NB, int H, int W, float* out32,
                const NNSlicePlanes* pl, const float* scale, int kp, int nx, int ny,
-               const DevStatus* st, cudaStream_t s) {
+               DevStatus* st, cudaStream_t s) {
   ConvArgs a{};
   a.st = st;
   a.H = H;
@@ -1371,6 +1374,14 @@ extern "C" int qp_nn_destroy(qp_nn* nn) {
   }
   if (nn->stream) cudaStreamDestroy(nn->stream);
   delete nn;
+  return 0;
+}
+
+extern "C" int qp_nn_flag_error(qp_nn* nn, int code) {
+  if (!nn) return nn_fail(__LINE__, "null argument");
+  std::lock_guard<std::mutex> turn(nn->mu);
+  NK(cudaMemcpyAsync(nn->err, &code, sizeof(int), cudaMemcpyHostToDevice, nn->stream));
+  NK(cudaStreamSynchronize(nn->stream));
   return 0;
 }
 
@@ -1654,7 +1665,7 @@ void nn_runtime_destroy(NNRuntime* r) {
 }
 
 int nn_predict(NNRuntime* r, const void* net, const NNSlicePlanes& p, const GridDims& g,
-               const DevStatus* st, cudaStream_t s) {
+               DevStatus* st, cudaStream_t s) {
   qp_nn* nn = const_cast<qp_nn*>(static_cast<const qp_nn*>(net));
   launch_pdl(k_nn_norms, NN_NORM_BLOCKS, 256, 0, s, p, g.nx, g.ny, g.kp, r->part, st);
   launch_pdl(k_nn_features, NN_NORM_BLOCKS, 256, 0, s, p, g.nx, g.ny, g.kp, r->hc, r->wc, r->part,

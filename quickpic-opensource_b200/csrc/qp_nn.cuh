@@ -63,9 +63,12 @@ int nn_runtime_create(const GridDims& g, NNRuntime** out);
 void nn_runtime_destroy(NNRuntime* r);
 // Like the step's other kernels, those below do nothing once st->error is set.
 // The start of slice j from the network (norms, features, 5 conv layers).
-// Returns the number of launches.
+// Returns the number of launches, or -1 (qp_set_error) when one failed; st->error
+// becomes NN_STATUS_FAILED when a bounded wait expires in a layer, or has expired
+// in an earlier call of the network.
+constexpr int NN_STATUS_FAILED = -9;
 int nn_predict(NNRuntime* r, const void* net, const NNSlicePlanes& p, const GridDims& g,
-               const DevStatus* st, cudaStream_t s);
+               DevStatus* st, cudaStream_t s);
 // Recording of training pairs: at the start of slice j (features of the crop,
 // minus the quadratic extrapolation into the target slot; the history moves on),
 // and at its end (plus the converged epw).  Both skip once the set is full.

@@ -9,7 +9,7 @@ sums: 1e-6 per slice, carried through 32 slices; the bar is that of the
 whole-step tests."""
 import numpy as np
 import pytest
-from conftest import rel_l2
+from conftest import BOX, rel_l2
 
 FINE = [[-3.0, 3.0], [-3.0, 3.0], [0.0, 10.0]]  # tiles of 0.75 c/wp: a mild density peak fills one
 
@@ -84,3 +84,30 @@ def test_step_that_overflows_is_the_step_with_room(qp, kw):
             # the passes' iterates over their scale
             assert np.isclose(sa, sb, rtol=1e-3)
             assert rel_l2(xa, xb) < 1e-2 and np.abs(ta - tb).max() < 1e-2 + 1e-2 * np.abs(tb).max()
+
+
+@pytest.mark.parametrize("graphs", [False, True])
+def test_a_failed_network_ends_the_step(qp, graphs):
+    """The error flag that a network's kernel raises when a wait expires (set
+    here from the host) reaches the caller of the step, and a cleared one does
+    not."""
+    c = qp.Context(7, 7, 3, BOX)
+    sp = qp.Species2d(c, ppc=(2, 2))
+    bm = qp.Beam3d(c, (16, 16, 16), peak_density=1.0, center=(0.0, 0.0, 2.5),
+                   sigma=(0.5, 0.5, 0.5))
+    sim = qp.Simulation(c, [sp], [bm], iter=2, predict=3, use_graphs=graphs)
+    net = qp.Predictor(seed=1)
+    sim.set_predictor(net)
+    sim.step3d()
+    want = sim.get_3d("bexyz")
+    assert qp.lib().qp_nn_flag_error(net.h, 1) == 0
+    with pytest.raises(qp.QPError, match="learned start: a bounded wait"):
+        sim.step3d()
+    with pytest.raises(qp.QPError, match="bounded wait expired"):
+        net.forward(np.zeros((1, 16, 1, 128), dtype=np.float32))
+    assert qp.lib().qp_nn_flag_error(net.h, 0) == 0
+    sp.renew(0.0)  # the failed step has moved the particles
+    sim.step3d()
+    assert rel_l2(sim.get_3d("bexyz"), want) < 1e-5
+    for h in (sim, net, bm, sp, c):
+        h.close()
