@@ -50,6 +50,7 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -1114,6 +1115,7 @@ struct Work {
 // device error flag of the tensor-core kernels.
 struct qp_nn {
   int device = 0;
+  unsigned long long id = 0;  // of this network alone in the process (nn_id)
   cudaStream_t stream = nullptr;
   float* master = nullptr;
   float* grad = nullptr;
@@ -1311,8 +1313,10 @@ extern "C" int qp_nn_create(int device, unsigned long long seed, qp_nn** out) {
   if (!out) return nn_fail(__LINE__, "null argument");
   if (cudaSetDevice(device) != cudaSuccess) return nn_fail(__LINE__, "cudaSetDevice failed");
   if (!encode_fn()) return nn_fail(__LINE__, "cuTensorMapEncodeTiled is not available");
+  static std::atomic<unsigned long long> created{0};
   qp_nn* nn = new qp_nn();
   nn->device = device;
+  nn->id = ++created;
   int o = 0;
   for (int l = 0; l < NN_LAYERS; ++l) {
     nn->off[l] = o;
@@ -1679,6 +1683,8 @@ int nn_predict(NNRuntime* r, const void* net, const NNSlicePlanes& p, const Grid
     return -1;
   return 7;
 }
+
+unsigned long long nn_id(const void* net) { return static_cast<const qp_nn*>(net)->id; }
 
 int nn_record_start(NNRuntime* r, void* data, const NNSlicePlanes& p, const GridDims& g,
                     const DevStatus* st, cudaStream_t s) {

@@ -69,6 +69,10 @@ void nn_runtime_destroy(NNRuntime* r);
 constexpr int NN_STATUS_FAILED = -9;
 int nn_predict(NNRuntime* r, const void* net, const NNSlicePlanes& p, const GridDims& g,
                DevStatus* st, cudaStream_t s);
+// A number that no other network of the process has or will have: whoever keeps
+// the launches of nn_predict keeps device pointers of this network, and a later
+// network may be created at the same host address.
+unsigned long long nn_id(const void* net);
 // Recording of training pairs: at the start of slice j (features of the crop,
 // minus the quadratic extrapolation into the target slot; the history moves on),
 // and at its end (plus the converged epw).  Both skip once the set is full.

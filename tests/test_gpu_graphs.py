@@ -12,7 +12,7 @@ L2-reduction deposits (FP32 roundoff, 1e-4 on fields over whole steps as for
 any two runs)."""
 import numpy as np
 import pytest
-from conftest import make_config, rel_l2
+from conftest import BOX, make_config, rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -148,3 +148,41 @@ def test_graph_pass_counts_match_direct(qp):
     for a, b in zip(ig, idir):
         assert abs(a - b) <= 0.02 * b, (ig, idir)
     assert rel_l2(bg, bd) < 1e-4
+
+
+def test_another_predictor_is_captured_anew(qp):
+    """A slice graph holds the network's device pointers.  A network that was
+    destroyed and another one, which may live at the same host address, give
+    the fields of direct launches with that other one."""
+    rng = np.random.default_rng(12)
+
+    def run(graphs):
+        c = qp.Context(7, 7, 4, BOX)
+        sp = qp.Species2d(c, ppc=(2, 2))
+        bm = qp.Beam3d(c, (16, 16, 32), peak_density=2.0, center=(0.0, 0.0, 2.5),
+                       sigma=(0.5, 0.5, 0.5))
+        # one pass: the start is felt in the fields
+        sim = qp.Simulation(c, [sp], [bm], iter=1, predict=3, use_graphs=graphs)
+        out, caps = [], []
+        for params in weights:
+            net = qp.Predictor(seed=1)
+            net.set_params(params)
+            sim.set_predictor(net)
+            sim.step3d()
+            out.append(sim.get_3d("bbxyz"))
+            caps.append(sim.graph_captures)
+            net.close()
+        for h in (sim, bm, sp, c):
+            h.close()
+        return out, caps
+
+    net = qp.Predictor(seed=1)
+    weights = [rng.normal(0, 0.1, net.nparams).astype(np.float32) for _ in range(3)]
+    net.close()
+    (direct, _), (graph, caps) = run(False), run(True)
+    assert caps[0] < caps[1] < caps[2]
+    for d, g in zip(direct, graph):
+        # the run-to-run difference of the deposits' sums moves features across
+        # bfloat16 roundings (2^-8 of a correction of up to a tenth of the field)
+        assert rel_l2(g, d) < 1e-3
+    assert min(rel_l2(direct[0], direct[1]), rel_l2(direct[1], direct[2])) > 5e-3
