@@ -326,7 +326,7 @@ extern "C" int qp_ctx_create(const qp_grid_desc* grid, int device, qp_ctx** out)
   ctx->dy = (float)((float)(grid->box[1][1]) - (float)(grid->box[1][0])) / (float)ctx->g.ny;
   ctx->dxi = (float)((float)(grid->box[2][1]) - (float)(grid->box[2][0])) / (float)ctx->nz;
   CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
-  if (fft_kernels_init() || part_kernels_init() || slice_kernels_init())
+  if (fft_kernels_init() || slice_kernels_init())
     return fail(ctx, __LINE__, "kernel init failed");
   // the fixed scratch array of qp_pmove_static is placed on the device with
   // the context, before a caller's own allocator can take the rest

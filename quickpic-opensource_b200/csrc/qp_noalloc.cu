@@ -13,7 +13,6 @@
 // pass of k_push and the sorted insert, qp_part.cu), with that scratch carved
 // out of one fixed array that lives in this file.  Every GPU on which this
 // module is loaded holds the array until the process exits.
-#include <mutex>
 #include <string>
 
 #include "qp_common.cuh"
@@ -31,11 +30,8 @@ namespace {
 static __device__ __align__(256) unsigned char g_pmove_scratch[QP_PMOVE_STATIC_SCRATCH_BYTES];
 
 constexpr int kMaxDevices = 64;
-constexpr int kMaxInboxCap = 16384;  // the insert kernel sorts at most this many keys per tile
+constexpr int kMaxInboxCap = 16384;  // movers a tile takes in per call; more are an overflow
 constexpr size_t kBytesPerMover = NCOMP * sizeof(float) + sizeof(unsigned long long);
-
-std::mutex g_setup_mutex;
-bool g_attr_done[kMaxDevices] = {};
 
 size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
@@ -55,17 +51,6 @@ int scratch_address(unsigned char** out) {
   if (e != cudaSuccess)
     return reject(__LINE__, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
   *out = static_cast<unsigned char*>(ptr);
-  return 0;
-}
-
-// Once per device, with that device current: the insert kernel's
-// shared-memory limit (a function attribute; it allocates nothing).
-int setup_device(int dev) {
-  std::lock_guard<std::mutex> lock(g_setup_mutex);
-  if (!g_attr_done[dev]) {
-    if (part_kernels_init() != 0) return reject(__LINE__, "insert kernel attribute set-up failed");
-    g_attr_done[dev] = true;
-  }
   return 0;
 }
 
@@ -137,7 +122,7 @@ extern "C" int qp_pmove_static(int indx, int indy, const float* const* part_in,
   if (e != cudaSuccess) return reject(__LINE__, cudaGetErrorString(e));
   if (dev < 0 || dev >= kMaxDevices) return reject(__LINE__, "pmove_static: device index too large");
   unsigned char* base = nullptr;
-  if (setup_device(dev) || scratch_address(&base)) return -1;
+  if (scratch_address(&base)) return -1;
 
   DevStatus* st = reinterpret_cast<DevStatus*>(base);
   Inbox ib{};

@@ -891,16 +891,52 @@ __global__ void __launch_bounds__(256) k_push(PartBuf A, PartBuf B, Inbox ib, Ti
   if (MODE != 0 && threadIdx.x == 0) B.count[t] = written;
 }
 
+// Sorts n (key, index) pairs by key, ascending, with all threads of the CTA:
+// bitonic merges whose comparators all point the same way (the first step of a
+// merge compares with the mirrored element), so that n may be any number:
+// what lies past it would stay there and is not touched.
+template <typename I>
+__device__ __forceinline__ void sort_pairs(unsigned long long* key, I* idx, int n) {
+  int p2 = 1;
+  while (p2 < n) p2 <<= 1;
+  for (int k = 2; k <= p2; k <<= 1) {
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const int o = j == k >> 1 ? i ^ (k - 1) : i ^ j;
+        if (o > i && o < n) {
+          const unsigned long long a = key[i], b = key[o];
+          if (a > b) {
+            key[i] = b;
+            key[o] = a;
+            const I t = idx[i];
+            idx[i] = idx[o];
+            idx[o] = t;
+          }
+        }
+      }
+      __syncthreads();
+    }
+  }
+}
+
 // Insert the movers of tile t after its stayers, sorted by their key so that
 // the particle order does not depend on the order in which the atomics of the
-// push handed out inbox slots.
+// push handed out inbox slots.  One size of shared memory serves any inbox: up
+// to one mover per thread is placed by rank, up to INSERT_SORT are sorted in
+// shared memory, and more in the inbox itself with the movers' slots of the
+// output as the index array (a tile of 8 x 8 particles per cell, 16384 in all,
+// takes in 1000 per cell width that its neighbours' plasma moves in a slice).
 // At most 32 registers: 8 CTAs per SM hold the 1024 tiles of a 512 x 512 grid in
-// one wave (6 left a second one of 136 CTAs).
-__global__ void __launch_bounds__(256, 8) k_insert(PartBuf B, Inbox ib, TileGeom tg, int p2max,
-                                                DevStatus* st, float* dq) {
+// one wave (6 left a second one of 136 CTAs).  The shared memory, 10 KB, is what
+// a CTA keeps from the kernels of other streams: sized by the inbox (24 KB at
+// 2 x 2 particles per cell, 96 KB at 4 x 4) it cost a scan of 64 instances 4 %
+// (6.78 against 7.07e9 particle-slices/s with 8 workers).
+constexpr int INSERT_SORT = 1024;
+__global__ void __launch_bounds__(256, 8) k_insert(PartBuf B, Inbox ib, TileGeom tg, DevStatus* st,
+                                                   float* dq) {
   grid_dep_sync();
-  extern __shared__ unsigned long long skey[];
-  int* sidx = reinterpret_cast<int*>(skey + p2max);
+  __shared__ unsigned long long skey[INSERT_SORT];
+  __shared__ short sidx[INSERT_SORT];
   if (st && st->error) return;
   const int t = blockIdx.x;
   int nin = ib.count[t];
@@ -942,35 +978,25 @@ __global__ void __launch_bounds__(256, 8) k_insert(PartBuf B, Inbox ib, TileGeom
       for (int c = 0; c < NCOMP; ++c) B.c[c][ob + rank] = v[c];
     }
   } else {
-    int p2 = 1;
-    while (p2 < nin) p2 <<= 1;
-    for (int i = threadIdx.x; i < p2; i += blockDim.x) {
-      skey[i] = (i < nin) ? ib.key[ib0 + i] : ~0ull;
-      sidx[i] = i;
-    }
-    __syncthreads();
-    for (int k = 2; k <= p2; k <<= 1) {
-      for (int j = k >> 1; j > 0; j >>= 1) {
-        for (int i = threadIdx.x; i < p2; i += blockDim.x) {
-          const int ixj = i ^ j;
-          if (ixj > i) {
-            const bool up = (i & k) == 0;
-            const unsigned long long a = skey[i], b = skey[ixj];
-            if ((a > b) == up) {
-              skey[i] = b;
-              skey[ixj] = a;
-              const int ti = sidx[i];
-              sidx[i] = sidx[ixj];
-              sidx[ixj] = ti;
-            }
-          }
-        }
-        __syncthreads();
+    const bool shared = nin <= INSERT_SORT;
+    int* gidx = reinterpret_cast<int*>(B.c[0] + ob);
+    for (int i = threadIdx.x; i < nin; i += blockDim.x) {
+      if (shared) {
+        skey[i] = ib.key[ib0 + i];
+        sidx[i] = (short)i;
+      } else {
+        gidx[i] = i;
       }
     }
+    __syncthreads();
+    if (shared)
+      sort_pairs(skey, sidx, nin);
+    else
+      sort_pairs(ib.key + ib0, gidx, nin);
     for (int i = threadIdx.x; i < nin; i += blockDim.x) {
-      const int si = sidx[i];
-      if (si < 0 || si >= nin) {  // the sort must map the first nin keys onto filled slots
+      // slot i of the output is written below, by the thread that reads it here
+      const int si = shared ? sidx[i] : gidx[i];
+      if (si < 0 || si >= nin) {  // the sort must map the keys onto filled slots
         raise_error(st, -8);
         continue;
       }
@@ -1020,20 +1046,9 @@ __global__ void __launch_bounds__(256) k_renew(const __grid_constant__ PartBuf P
 
 }  // namespace
 
-int part_kernels_init() {
-  const int big = 16384 * (int)(sizeof(unsigned long long) + sizeof(int));
-  if (cudaFuncSetAttribute(k_insert, cudaFuncAttributeMaxDynamicSharedMemorySize, big) !=
-      cudaSuccess)
-    return -2;
-  return 0;
-}
-
 void launch_insert(const PartBuf& B, const Inbox& ib, const TileGeom& tg, DevStatus* st,
                    cudaStream_t s, float* deposit_q) {
-  int p2 = 1;
-  while (p2 < ib.cap) p2 <<= 1;
-  const size_t smem = (size_t)p2 * (sizeof(unsigned long long) + sizeof(int));
-  launch_pdl(k_insert, tg.ntiles, 256, smem, s, B, ib, tg, p2, st, deposit_q);
+  launch_pdl(k_insert, tg.ntiles, 256, 0, s, B, ib, tg, st, deposit_q);
 }
 
 void launch_renew(const PartBuf& P0, const PartBuf& A, int ntiles, float qm, cudaStream_t s) {

@@ -55,7 +55,6 @@ struct GatherPlanes {
   int store_planes;
 };
 
-int part_kernels_init();
 // places the static scratch of qp_pmove_static on the current device (qp_noalloc.cu)
 int pmove_static_reserve();
 void launch_deposit_rho(const PartBuf& P, const TileGeom& tg, float* q, const DevStatus* st,

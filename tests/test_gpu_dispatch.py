@@ -4,9 +4,11 @@
   thread up to 222 tiles, one and 4 beyond; tiles with less than one round of
   particles, exactly one, and more.  One 3D step on each side of the line,
   against the FP64 oracle; the bar is that of the whole-step tests (1e-4).
-* Re-bin: up to 256 movers into a tile are placed by rank, more by the sort.
-  Values are only moved, so the tiles must hold exactly the particles they
-  should, the movers in cell order.
+* Re-bin: up to 256 movers into a tile are placed by rank, up to 1024 sorted in
+  shared memory, more in the inbox.  Values are only moved, so the tiles must
+  hold exactly the particles they should, the movers in cell order.
+* A step at 8 x 8 particles per cell, whose inboxes (19661 slots of a tile) are
+  larger than any sort in shared memory.
 """
 import numpy as np
 import pytest
@@ -25,7 +27,7 @@ def qp():
 # 1 tile; 64; 128 tiles (two CTAs each); 256 (one); ppc 1, 4 and 6 per cell:
 # 256, 1024 and 1536 particles per tile
 @pytest.mark.parametrize("ind,ppc", [((4, 4, 4), (2, 2)), ((5, 9, 4), (1, 1)), ((8, 7, 4), (3, 2)),
-                                     ((8, 8, 4), (1, 1)), ((8, 8, 4), (3, 2))])
+                                     ((8, 8, 4), (1, 1)), ((8, 8, 4), (3, 2)), ((5, 5, 4), (8, 8))])
 def test_step_on_both_sides_of_the_tile_count_rule(qp, oracle_mod, ind, ppc):
     cfg = make_config(ind=ind, ppc=ppc, iter=2)
     b = cfg["beams"][0]
@@ -46,7 +48,8 @@ def test_step_on_both_sides_of_the_tile_count_rule(qp, oracle_mod, ind, ppc):
         h.close()
 
 
-@pytest.mark.parametrize("ppc", [(1, 1), (4, 4), (4, 5), (5, 7)])  # 16, 256, 320, 560 movers
+# 16, 256, 320, 560, 1024, 1040, 4608 movers
+@pytest.mark.parametrize("ppc", [(1, 1), (4, 4), (4, 5), (5, 7), (8, 8), (5, 13), (16, 18)])
 def test_rebin_places_any_number_of_movers(qp, ppc):
     c = qp.Context(6, 6, 1, [[-6.0, 6.0], [-6.0, 6.0], [0.0, 1.0]])
     sp = qp.Species2d(c, ppc=ppc)
