@@ -88,6 +88,9 @@ struct qp_species {
   int nppmx0 = 0;          // reference-equivalent capacity
   long long np = 0;
   qp_field2d* q = nullptr;     // species charge (rs + ks, used by cbq)
+  // fused steps of several species: the charge of the slice to come, while q
+  // keeps the last slice's (which the caller may read between slices)
+  float* qx = nullptr;
   qp_field2d* qn = nullptr;    // ion background
   qp_field2d* cusp = nullptr;  // per-species accumulators of the class API
   qp_field2d* dcusp = nullptr;
@@ -95,9 +98,9 @@ struct qp_species {
   float* q3 = nullptr;         // (nz+1) real planes
   float* q3_first = nullptr;   // slice-1 plane after renew (pristine)
   int regrowths = 0;
-  // q holds the charge of A's particles, as the fused step's slices hand it
-  // on; a class-level call that changes either clears it
-  bool q_live = false;
+  // the plane that holds the charge of A's particles, as the fused step's
+  // slices hand it on; a class-level call that changes either clears it
+  const float* q_live = nullptr;
   PlasmaProfile prof;          // the loader's profile, lengths in cells
 };
 
@@ -788,7 +791,7 @@ static int part_copy(qp_ctx* ctx, PartBuf& dst, const PartBuf& src) {
 // passes, x pass back into the species' real-space charge
 static void smooth_charge(qp_species* sp, const float* a, const float* b) {
   qp_ctx* ctx = sp->ctx;
-  sp->q_live = false;
+  sp->q_live = nullptr;
   const GridDims& g = ctx->g;
   XJob xj{};
   YJob yj{};
@@ -871,7 +874,7 @@ static int species_renew_device(qp_species* sp, float s) {
   std::string err;
   if (!plasma_qm(sp->prof, s, &qm, &err)) return fail(ctx, __LINE__, "plasma loader: " + err);
   if (sp->A.cap < sp->P0.cap) return fail(ctx, __LINE__, "renew: capacity shrank");
-  sp->q_live = false;
+  sp->q_live = nullptr;
   launch_renew(sp->P0, sp->A, tg.ntiles, qm, ctx->stream);
   CK(cudaGetLastError());
   return 0;
@@ -981,6 +984,7 @@ extern "C" int qp_species_destroy(qp_species* sp) {
   part_free(&sp->P0);
   inbox_free(&sp->ib);
   field_free(sp->q);
+  if (sp->qx) cudaFree(sp->qx);
   field_free(sp->qn);
   field_free(sp->cusp);
   field_free(sp->dcusp);
@@ -1007,7 +1011,7 @@ extern "C" int qp_species_qdp(qp_species* sp, qp_field2d* qe) {
   if (qe->state != 0) return fail(ctx, __LINE__, "sum: states are different");
   const GridDims& g = ctx->g;
   float* q = sp->q->rs[0];
-  sp->q_live = false;
+  sp->q_live = nullptr;
   launch_lin(g.rplane, q, nullptr, nullptr, 0.f, LIN_FILL, ctx->st, ctx->stream);
   launch_deposit_rho(sp->A, ctx->tg, q, ctx->st, ctx->stream);
   sp->q->state = 0;
@@ -1079,7 +1083,7 @@ extern "C" int qp_species_amjdp(qp_species* sp, qp_field2d* fxy, qp_field2d* bxy
 static int push_rebin(qp_species* sp, int mode, const GatherPlanes& f, float dex) {
   qp_ctx* ctx = sp->ctx;
   const int nt = ctx->tg.ntiles;
-  sp->q_live = false;
+  sp->q_live = nullptr;
   for (int attempt = 0; attempt < 12; ++attempt) {
     if (sp->B.cap < sp->A.cap) {
       part_free(&sp->B);
@@ -1128,7 +1132,7 @@ extern "C" int qp_species_push(qp_species* sp, qp_field2d* fxy, qp_field2d* bxyz
 extern "C" int qp_species_partpush(qp_species* sp, qp_field2d* fxy, qp_field2d* bxyz,
                                    qp_field2d* psit, float dex) {
   qp_ctx* ctx = sp->ctx;
-  sp->q_live = false;
+  sp->q_live = nullptr;
   launch_push(0, sp->A, sp->A, sp->ib, ctx->tg, gplanes(fxy, bxyz, psit, 0), sp->qbm, sp->dt, dex,
               ctx->st, ctx->stream);
   CK(cudaGetLastError());
@@ -1202,7 +1206,7 @@ extern "C" int qp_species_upload(qp_species* sp, const float* ppart, const int* 
   const int nt = ctx->tg.ntiles;
   int mx = 0;
   for (int t = 0; t < nt; ++t) mx = std::max(mx, kpic[t]);
-  sp->q_live = false;
+  sp->q_live = nullptr;
   if (mx > sp->A.cap) {
     part_free(&sp->A);
     if (part_alloc(&sp->A, nt, mx)) return fail(ctx, __LINE__, "out of device memory");

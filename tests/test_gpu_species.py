@@ -109,3 +109,45 @@ def test_field_algebra_runs_components_in_the_lists_order(qp, ind):
         assert np.array_equal(a.get_ks(), ref[id(a)])
     for h in (a, b, c):
         h.close()
+
+
+def test_charge_between_slices_is_the_last_slices(qp):
+    """Between slices() calls get_q() of one of several species is the charge
+    that the last slice ran with, that of the particles as they were before it,
+    after an odd and after an even number of slices."""
+    def run(chunks):
+        c = qp.Context(6, 5, 4, BOX)
+        sp = [qp.Species2d(c, ppc=(2, 2), density=d) for d in (0.75, 0.25)]
+        bm = qp.Beam3d(c, (16, 16, 32), peak_density=2.0, center=(0.0, 0.0, 2.5),
+                       sigma=(0.5, 0.5, 0.5))
+        sim = qp.Simulation(c, sp, [bm], iter=1)
+        sim.begin3d()
+        assert not any(s.get_q().any() for s in sp)
+        seen, done = {}, 0
+        for n in chunks:
+            before = [s.get_particles() for s in sp]
+            sim.slices(n)
+            done += n
+            seen[done] = (before, [s.get_q() for s in sp])
+        sim.end3d()
+        be = sim.get_3d("bexyz")
+        for h in (sim, bm, *sp, c):
+            h.close()
+        return seen, be
+
+    single, be1 = run([1] * 16)
+    several, be2 = run([2, 3, 1, 4, 1, 1, 4])
+    assert rel_l2(be2, be1) < 1e-5
+    c2 = qp.Context(6, 5, 4, BOX)
+    s2, qe = qp.Species2d(c2, ppc=(2, 2)), qp.Field2d(c2, 1)
+    for j in several:
+        for k in range(2):
+            pp, kp = single[j][0][k]
+            s2.set_particles(pp, kp)
+            qe.as_(0.0)
+            s2.qdp(qe)
+            want = s2.get_q()
+            assert rel_l2(single[j][1][k], want) < 1e-6  # FP32 sums in another order
+            assert rel_l2(several[j][1][k], want) < 1e-5  # of another run
+    for h in (s2, qe, c2):
+        h.close()
