@@ -270,7 +270,7 @@ static PackJob rows_job(const GridDims& g, const float* const* p, int dim, long 
   for (int c = 0; c < dim; ++c) j.plane[c] = const_cast<float*>(p[c]);
   j.dim = dim;
   j.n0 = g.nx + 2;
-  j.n1 = j.valid1 = (int)rows;
+  j.n1 = j.valid1 = rows;
   j.stride = 1;
   j.pitch = g.rp;
   j.scale = scale;
@@ -1442,7 +1442,7 @@ extern "C" int qp_beam_download(qp_beam* b, float* part) {
   PackJob j{};
   for (int c = 0; c < BCOMP; ++c) j.plane[c] = b->b.c[c];
   j.dim = BCOMP;
-  j.n0 = (int)b->b.np;
+  j.n0 = b->b.np;
   j.n1 = j.valid1 = 1;
   j.stride = 1;
   j.scale = 1.f;

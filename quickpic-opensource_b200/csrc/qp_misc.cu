@@ -175,28 +175,22 @@ __global__ void k_guard_add(Planes3 pl, GridDims g, const DevStatus* st) {
 __global__ void __launch_bounds__(256) k_pack(const __grid_constant__ PackJob j, long long i0,
                                               long long n, float* out) {
   grid_dep_sync();
-  const long long row = (long long)j.dim * j.n0;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
        k += (long long)gridDim.x * blockDim.x) {
-    const long long i = i0 + k, b = i / row, r = i - b * row, a = r / j.dim;
-    const int c = (int)(r - a * j.dim);
-    float v = 0.f;
-    if (b < j.valid1 && (!j.count || a < j.count[b]))
-      v = j.plane[c][b * j.pitch + a * j.stride] * j.scale;
-    out[k] = v;
+    int c;
+    long long at;
+    out[k] = pack_at(j, i0 + k, &c, &at) ? j.plane[c][at] * j.scale : 0.f;
   }
 }
 
 __global__ void __launch_bounds__(256) k_unpack(const __grid_constant__ PackJob j, long long i0,
                                                 long long n, const float* in) {
   grid_dep_sync();
-  const long long row = (long long)j.dim * j.n0;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
        k += (long long)gridDim.x * blockDim.x) {
-    const long long i = i0 + k, b = i / row, r = i - b * row, a = r / j.dim;
-    const int c = (int)(r - a * j.dim);
-    if (b < j.valid1 && (!j.count || a < j.count[b]))
-      j.plane[c][b * j.pitch + a * j.stride] = in[k];
+    int c;
+    long long at;
+    if (pack_at(j, i0 + k, &c, &at)) j.plane[c][at] = in[k];
   }
 }
 

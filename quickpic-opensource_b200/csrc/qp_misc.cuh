@@ -88,13 +88,25 @@ void launch_guard_add(float* const* p, int count, const GridDims& g, const DevSt
 // for b < n1 (and a < count[b] when count is given), 0 otherwise.
 struct PackJob {
   float* plane[8];
-  int dim, n0, n1;      // host extents: components, fast index, slow index
-  int valid1;           // slow indices that have data
+  int dim;              // host extents: components,
+  long long n0, n1;     //   fast index, slow index
+  long long valid1;     // slow indices that have data
   int stride;           // floats between consecutive fast indices of a plane
   long long pitch;      // floats between consecutive slow indices of a plane
   const int* count;
   float scale;
 };
+// Where element i of the host array lies: component *c and the float of its
+// plane; false for an element without data.
+__host__ __device__ inline bool pack_at(const PackJob& j, long long i, int* c, long long* at) {
+  const long long row = j.dim * j.n0, b = i / row, r = i - b * row, a = r / j.dim;
+  *c = (int)(r - a * j.dim);
+  *at = b * j.pitch + a * j.stride;
+#ifdef __CUDA_ARCH__
+  if (j.count && a >= j.count[b]) return false;
+#endif
+  return b < j.valid1;
+}
 // elements [i0, i0 + n) of the host array; `out` and `in` are pinned host (or
 // device) memory and start at element i0.  No status check: a caller may look at
 // the fields after an error.

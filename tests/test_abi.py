@@ -106,3 +106,44 @@ def test_component_values_may_be_one_number(qp):
     assert seen[-1] == ([1, 3], [2, 1], [2.0, 2.0], 2)
     f.mult(f, [2.0, 3.0], dim=np.array([1, 2]), dim1=[2, 1])
     assert seen[-1] == ([1, 2], [2, 1], [2.0, 3.0], 2)
+
+
+def test_layout_conversion_counts_in_64_bits(tmp_path):
+    """A beam may have more than 2^31 particles: the conversion's extents and
+    indices, compiled for the host from the kernels' header."""
+    src = tmp_path / "pack.cu"
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                        "quickpic-opensource_b200", "csrc")
+    src.write_text("""
+#include "qp_misc.cuh"
+#include <cstdio>
+int main() {
+  qp::PackJob j{};
+  const long long np = 3000000001LL;
+  j.dim = 7;
+  j.n0 = np;
+  j.n1 = j.valid1 = 1;
+  j.stride = 1;
+  int bad = j.n0 != np;
+  for (long long a : {0LL, 1LL, (1LL << 31) - 1, 1LL << 31, np - 1})
+    for (int k = 0; k < 7; ++k) {
+      int c = -1;
+      long long at = -1;
+      bad += !qp::pack_at(j, k + 7 * a, &c, &at) || c != k || at != a;
+    }
+  j.dim = 3;  // and slow indices past 2^31
+  j.n0 = 18;
+  j.n1 = j.valid1 = np;
+  j.pitch = 20;
+  int c;
+  long long at;
+  bad += !qp::pack_at(j, 2 + 3 * (5 + 18 * (np - 1)), &c, &at) || c != 2 || at != 20 * (np - 1) + 5;
+  bad += qp::pack_at(j, 54 * np, &c, &at);
+  return bad;
+}
+""")
+    exe = tmp_path / "pack"
+    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+    subprocess.run([nvcc, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a",
+                    "--expt-relaxed-constexpr", "-I", csrc, "-o", str(exe), str(src)], check=True)
+    assert subprocess.run([str(exe)]).returncode == 0
