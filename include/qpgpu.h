@@ -57,6 +57,11 @@ int qp_ctx_create(const qp_grid_desc* grid, int device, qp_ctx** out);
 int qp_ctx_destroy(qp_ctx* ctx);
 /* Blocks until all work queued on the context has finished. */
 int qp_ctx_sync(qp_ctx* ctx);
+/* Pinned host memory that the library holds now for its transfers, and how
+ * often it has pinned some (each time costs milliseconds): at most 4 buffers of
+ * 512 KB per device beside those of transfers in progress, one buffer while
+ * there is no context.  Either pointer may be null. */
+int qp_host_buffers(long long* bytes, long long* pinned);
 /* Required capacity after a call returned > 0. */
 long long qp_ctx_last_need(const qp_ctx* ctx);
 /* Message of the last failed call (static storage of the context). */

@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -151,10 +152,12 @@ static int ensure_staging(qp_ctx* ctx, size_t bytes) {
 // through two halves: one half crosses PCIe while the host copies the other to
 // or from the caller's pageable array.
 //
-// Pinning costs milliseconds whatever the size, so the halves are kept: a call
-// takes a pair from a pool of the process (its own for the time of the call, so
-// threads and contexts do not share one) and returns it; at most POOL_KEEP
-// pairs stay, and the last context to go frees them.
+// Pinning costs milliseconds whatever the size (1 to 13, now and then more), so
+// the halves are kept: a call takes a pair from a pool of the process (its own
+// for the time of the call, so threads and contexts do not share one) and
+// returns it.  At most POOL_KEEP pairs per device stay while there are contexts,
+// and one pair (512 KB) from the last context to the next, so that a program
+// which makes and closes one context after another pins once.
 static const size_t BOUNCE = 1u << 16;
 static const size_t POOL_KEEP = 4;
 struct Bounce {
@@ -165,11 +168,15 @@ struct Bounce {
 static std::mutex g_pool_mutex;
 static std::vector<Bounce> g_pool;
 static int g_pool_users = 0;  // live contexts
+static std::atomic<long long> g_pairs{0}, g_pins{0};  // pairs that exist; ever pinned
 
 static void bounce_free(Bounce& b) {
   for (cudaEvent_t e : b.ev)
     if (e) cudaEventDestroy(e);
-  if (b.h[0]) cudaFreeHost(b.h[0]);
+  if (b.h[0]) {
+    cudaFreeHost(b.h[0]);
+    --g_pairs;
+  }
   b = Bounce{};
 }
 
@@ -185,6 +192,8 @@ static int bounce_take(qp_ctx* ctx, Bounce* b) {
   }
   b->device = ctx->device;
   CK(cudaMallocHost(&b->h[0], sizeof(float) * 2 * BOUNCE));
+  ++g_pairs;
+  ++g_pins;
   b->h[1] = b->h[0] + BOUNCE;
   for (cudaEvent_t& e : b->ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   return 0;
@@ -192,7 +201,9 @@ static int bounce_take(qp_ctx* ctx, Bounce* b) {
 
 static void bounce_give(Bounce& b) {
   std::lock_guard<std::mutex> lock(g_pool_mutex);
-  if (g_pool_users > 0 && g_pool.size() < POOL_KEEP && b.ev[1])
+  size_t here = 0;
+  for (const Bounce& p : g_pool) here += p.device == b.device;
+  if (here < POOL_KEEP && b.ev[1])
     g_pool.push_back(b);
   else
     bounce_free(b);
@@ -212,8 +223,16 @@ static int pool_enter(qp_ctx* ctx) {
 static void pool_leave() {
   std::lock_guard<std::mutex> lock(g_pool_mutex);
   if (--g_pool_users > 0) return;
-  for (Bounce& b : g_pool) bounce_free(b);
-  g_pool.clear();
+  while (g_pool.size() > 1) {
+    bounce_free(g_pool.back());
+    g_pool.pop_back();
+  }
+}
+
+extern "C" int qp_host_buffers(long long* bytes, long long* pinned) {
+  if (bytes) *bytes = g_pairs * (long long)(sizeof(float) * 2 * BOUNCE);
+  if (pinned) *pinned = g_pins;
+  return 0;
 }
 
 // the whole host array, complete on return

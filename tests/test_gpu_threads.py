@@ -61,3 +61,45 @@ def test_threads_take_turns_on_one_network(qp, shapes):
 
     run_threads([lambda j=j: work(*j) for j in jobs])
     net.close()
+
+
+def host_buffers(qp):
+    import ctypes as C
+
+    bytes_, pinned = C.c_longlong(), C.c_longlong()
+    assert qp.lib().qp_host_buffers(C.byref(bytes_), C.byref(pinned)) == 0
+    return bytes_.value, pinned.value
+
+
+def test_one_context_after_another_pins_once(qp):
+    def cycle():
+        c = qp.Context(5, 5, 2, [[-6.0, 6.0], [-6.0, 6.0], [0.0, 1.0]])
+        f = qp.Field2d(c, 3)
+        f.as_(2.0)
+        assert (f.get_rs()[:, :, : c.ny + 1] == 2.0).all()
+        f.close()
+        c.close()
+
+    cycle()
+    bytes0, pinned0 = host_buffers(qp)
+    for _ in range(5):
+        cycle()
+    assert host_buffers(qp) == (bytes0, pinned0) and bytes0 > 0
+
+
+def test_threads_with_a_context_each_transfer_at_once(qp):
+    """Each transfer has its own pair of host buffers; afterwards no more of
+    them are kept than the bound says.  Values are only moved: exact."""
+    def work(k):
+        c = qp.Context(7, 7, 3, [[-6.0, 6.0], [-6.0, 6.0], [0.0, 1.0]])
+        f = qp.Field2d(c, 3)
+        rng = np.random.default_rng(k)
+        for _ in range(8):
+            a = rng.standard_normal(c.ks_shape(3)).astype(np.float32)
+            f.set_ks(a)
+            assert np.array_equal(f.get_ks(), a)
+        f.close()
+        c.close()
+
+    run_threads([lambda k=k: work(k) for k in range(8)])
+    assert host_buffers(qp)[0] <= 4 * 512 * 1024
