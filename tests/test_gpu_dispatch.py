@@ -24,11 +24,7 @@ def qp():
     return qpgpu
 
 
-# 1 tile; 64; 128 tiles (two CTAs each); 256 (one); ppc 1, 4 and 6 per cell:
-# 256, 1024 and 1536 particles per tile
-@pytest.mark.parametrize("ind,ppc", [((4, 4, 4), (2, 2)), ((5, 9, 4), (1, 1)), ((8, 7, 4), (3, 2)),
-                                     ((8, 8, 4), (1, 1)), ((8, 8, 4), (3, 2)), ((5, 5, 4), (8, 8))])
-def test_step_on_both_sides_of_the_tile_count_rule(qp, oracle_mod, ind, ppc):
+def step_against_oracle(qp, oracle_mod, ind, ppc):
     cfg = make_config(ind=ind, ppc=ppc, iter=2)
     b = cfg["beams"][0]
     c = qp.Context(*ind, cfg["grid"]["box"])
@@ -46,6 +42,21 @@ def test_step_on_both_sides_of_the_tile_count_rule(qp, oracle_mod, ind, ppc):
         assert rel_l2(got, o.get(name).reshape(got.shape, order="F")) < 1e-4, name
     for h in (sim, bm, sp, c):
         h.close()
+
+
+# every length of line in x and in y, where the transforms, their register
+# caps and the staging of the x passes and column solves differ
+@pytest.mark.parametrize("ind", [(10, 5, 4), (5, 10, 4), (11, 4, 4), (4, 11, 4), (7, 8, 4), (8, 7, 4)])
+def test_step_at_every_line_length(qp, oracle_mod, ind):
+    step_against_oracle(qp, oracle_mod, ind, (2, 1))
+
+
+# 1 tile; 64; 128 tiles (two CTAs each); 256 (one); ppc 1, 4 and 6 per cell:
+# 256, 1024 and 1536 particles per tile
+@pytest.mark.parametrize("ind,ppc", [((4, 4, 4), (2, 2)), ((5, 9, 4), (1, 1)), ((8, 7, 4), (3, 2)),
+                                     ((8, 8, 4), (1, 1)), ((8, 8, 4), (3, 2)), ((5, 5, 4), (8, 8))])
+def test_step_on_both_sides_of_the_tile_count_rule(qp, oracle_mod, ind, ppc):
+    step_against_oracle(qp, oracle_mod, ind, ppc)
 
 
 # 16, 256, 320, 560, 1024, 1040, 4608 movers

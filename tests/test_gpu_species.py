@@ -47,6 +47,17 @@ def test_two_half_density_species_are_one_plasma(qp, ind, iter, graphs):
     assert np.isfinite(two["bb"]).all()
 
 
+# the x passes of their cbq ride along up to 4 species and stand alone beyond;
+# more than 8 need launches of their own to clear their currents and sum their
+# charges in two parts (16 planes each), more than 12 smooth in two launches
+@pytest.mark.parametrize("n", [4, 5, 8, 9, 13])
+def test_many_species_are_one_plasma(qp, n):
+    one = step(qp, (6, 5, 4), [1.0], 2, False)
+    many = step(qp, (6, 5, 4), [1.0 / n] * n, 2, n % 2 == 1)
+    for name in ("be", "bb", "epw", "q3"):  # the bar as above
+        assert rel_l2(many[name], one[name]) < 1e-4, name
+
+
 @pytest.mark.parametrize("nspecies", [1, 3])
 def test_particles_restored_between_slices_give_the_same_slices(qp, nspecies):
     """A caller that puts a species' particles back between two slices (here the
