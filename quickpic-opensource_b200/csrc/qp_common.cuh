@@ -109,16 +109,16 @@ __device__ __forceinline__ bool pass_skipped(const DevStatus* st, int pass) {
   return done > 0 && done < pass;
 }
 
-// The words of the device status a slice kernel checks before its work, read
-// with two 16-byte loads (error .. need_inbox, cursor ..) that a
-// kernel issues together with its first data loads.
+// The words of the device status that k_slice_a checks before its work, read
+// with two 16-byte loads (error .. need_inbox, cursor ..) that it issues
+// together with its first data loads.
 struct StatusSnap {
-  int error, cursor, pass_done;
+  int error, cursor;
 };
 __device__ __forceinline__ StatusSnap status_snap(const DevStatus* st) {
   const int4* p = reinterpret_cast<const int4*>(st);
   const int4 a = p[0], b = p[1];
-  return StatusSnap{a.x, b.x, b.y};
+  return StatusSnap{a.x, b.x};
 }
 
 enum { QP_OK = 0, QP_OVERFLOW = 1 };

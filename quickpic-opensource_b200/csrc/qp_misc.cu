@@ -116,11 +116,6 @@ __global__ void __launch_bounds__(256) k_lin(const __grid_constant__ LinJob job,
     if (op == LIN_ADDSC)
       reinterpret_cast<float4*>(p.s)[i] = make_float4(a.x * v, a.y * v, a.z * v, a.w * v);
   }
-  for (long long i = 4 * n4 + i0; i < p.n; i += step) {  // a length that is not a multiple of 4
-    const float a = ra ? p.a[i] : 0.f;
-    p.d[i] = lin1(op, a, rb ? p.b[i] : 0.f, rc ? p.c[i] : 0.f, v);
-    if (op == LIN_ADDSC) p.s[i] = a * v;
-  }
 }
 
 __global__ void __launch_bounds__(256) k_sum(const __grid_constant__ SumJob job, long long n,
@@ -137,11 +132,6 @@ __global__ void __launch_bounds__(256) k_sum(const __grid_constant__ SumJob job,
       v = make_float4(a.x + v.x, a.y + v.y, a.z + v.z, a.w + v.w);
     }
     reinterpret_cast<float4*>(d)[i] = v;
-  }
-  for (long long i = 4 * n4 + i0; i < n; i += step) {
-    float v = job.onto ? d[i] : 0.f;
-    for (int k = 0; k < job.count; ++k) v = job.src[k][i] + v;
-    d[i] = v;
   }
 }
 
@@ -197,7 +187,7 @@ __global__ void __launch_bounds__(256) k_unpack(const __grid_constant__ PackJob 
 __global__ void k_cursor(DevStatus* st, int v) {
   grid_dep_sync();
   if (st->error) return;
-  st->cursor = v < 0 ? st->cursor + 1 : v;
+  st->cursor = v;
 }
 
 }  // namespace

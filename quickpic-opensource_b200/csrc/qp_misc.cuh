@@ -14,8 +14,9 @@ struct Planes3 {
 };
 
 // Element-wise operations on planes, several planes per launch (grid row i =
-// plane i).  Every plane starts on a 16-byte boundary; the planes of one job
-// must not depend on one another (lin_conflict).
+// plane i).  Every plane starts on a 16-byte boundary and holds a multiple of
+// four floats (field pitches and particle capacities are such); the planes of
+// one job must not depend on one another (lin_conflict).
 //   FILL d = v   SCALE d = a v   ADD d = a + b   SUB d = a - b   COPY d = a
 //   ADD3 d = c + (a + b)         ADDSC d = a + b, then s = a v (s may be a)
 enum { LIN_FILL = 0, LIN_SCALE, LIN_ADD, LIN_SUB, LIN_COPY, LIN_ADD3, LIN_ADDSC };

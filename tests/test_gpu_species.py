@@ -94,8 +94,8 @@ def test_particles_restored_between_slices_give_the_same_slices(qp, nspecies):
 def test_field_algebra_runs_components_in_the_lists_order(qp, ind):
     """mult / add / sub over component lists, several of them in one launch: the
     same as one component after another, also where a component reads what an
-    earlier one of the list wrote, and for planes whose length is no multiple of
-    the launch."""
+    earlier one of the list wrote, and for planes that do not fill a launch's CTAs
+    evenly."""
     c = qp.Context(ind[0], ind[1], 1, BOX)
     rng = np.random.default_rng(3)
     a, b = qp.Field2d(c, 3), qp.Field2d(c, 3)
