@@ -235,8 +235,24 @@ extern "C" int qp_host_buffers(long long* bytes, long long* pinned) {
   return 0;
 }
 
+// A context's device is the current one within its scope: kernels are launched
+// and events made there, whichever device the calling thread works on.
+struct DeviceScope {
+  int before = -1;
+  explicit DeviceScope(const qp_ctx* ctx) {
+    int now = -1;
+    if (cudaGetDevice(&now) == cudaSuccess && now != ctx->device &&
+        cudaSetDevice(ctx->device) == cudaSuccess)
+      before = now;
+  }
+  ~DeviceScope() {
+    if (before >= 0) cudaSetDevice(before);
+  }
+};
+
 // the whole host array, complete on return
 static int to_host(qp_ctx* ctx, const PackJob& job, float* out) {
+  DeviceScope scope(ctx);
   const size_t n = (size_t)job.dim * job.n0 * job.n1, parts = (n + BOUNCE - 1) / BOUNCE;
   if (n == 0) return 0;
   Bounce b;
@@ -262,6 +278,7 @@ static int to_host(qp_ctx* ctx, const PackJob& job, float* out) {
 
 // the whole host array; complete on return
 static int to_device(qp_ctx* ctx, const PackJob& job, const float* in) {
+  DeviceScope scope(ctx);
   const size_t n = (size_t)job.dim * job.n0 * job.valid1, parts = (n + BOUNCE - 1) / BOUNCE;
   if (n == 0) return 0;
   Bounce b;
@@ -1222,6 +1239,7 @@ extern "C" int qp_species_download(qp_species* sp, float* ppart, int* kpic, int 
 extern "C" int qp_species_upload(qp_species* sp, const float* ppart, const int* kpic,
                                  int nppmx_ld) {
   qp_ctx* ctx = sp->ctx;
+  DeviceScope scope(ctx);
   const int nt = ctx->tg.ntiles;
   int mx = 0;
   for (int t = 0; t < nt; ++t) mx = std::max(mx, kpic[t]);

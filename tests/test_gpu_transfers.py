@@ -74,3 +74,22 @@ def test_whole_arrays_are_their_planes(qp, ind):
     sim.end3d()
     for h in (sim, bm, sp, c):
         h.close()
+
+
+def test_transfers_run_on_their_contexts_device(qp):
+    """Reading and writing a context's arrays while another device is current."""
+    import torch
+
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two devices")
+    c = qp.Context(5, 5, 1, BOX, device=0)
+    sp, f = qp.Species2d(c, ppc=(2, 2)), qp.Field2d(c, 2)
+    other = qp.Context(5, 5, 1, BOX, device=1)  # makes device 1 the current one
+    a = np.random.default_rng(1).standard_normal(c.ks_shape(2)).astype(np.float32)
+    f.set_ks(a)
+    assert np.array_equal(f.get_ks(), a)
+    pp, kp = sp.get_particles()
+    sp.set_particles(pp, kp)
+    assert np.array_equal(sp.get_particles()[0], pp)
+    for h in (f, sp, c, other):
+        h.close()
