@@ -236,7 +236,7 @@ struct ConvArgs {
   int H, W, NB;               // output images (NB images of H x W)
   int b0;                     // first image of the launch in the input map
   int* err;                   // device error flag (nonzero on a wait that expired)
-  DevStatus* st;              // the step's status, or null outside of a step
+  DevStatus* st;              // EPI_EPW: the step's status
 };
 
 __device__ __forceinline__ void flag_error(int* err, int code) {
@@ -327,9 +327,11 @@ __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtenso
   const int step = (int)gridDim.x;
   bool bad = false;
   // a step whose status holds an error leaves every plane as it is, and so does
-  // a network that has failed before (one decision for the CTA, whose barriers
-  // and tensor-memory loads follow)
-  const bool skip = a.st && __syncthreads_or(a.st->error | *a.err) != 0;
+  // a network that has failed (here in an earlier layer, or in an earlier call):
+  // one decision for the CTA, whose barriers and tensor-memory loads follow.
+  // Only the layer that writes the step's planes looks: the round trip costs a
+  // microsecond per layer.
+  const bool skip = EPI == EPI_EPW && __syncthreads_or(a.st->error | *a.err) != 0;
   if (tid == 0 && !skip && (int)blockIdx.x < ntiles) {
     issue(blockIdx.x, 0);
     pf_k = 0;
@@ -432,7 +434,8 @@ __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtenso
     flag_error(a.err, 1);
   }
   // a step ends with an error once its network has failed
-  if (tid == 0 && a.st && *(volatile int*)a.err) atomicCAS(&a.st->error, 0, NN_STATUS_FAILED);
+  if (EPI == EPI_EPW && tid == 0 && *(volatile int*)a.err)
+    atomicCAS(&a.st->error, 0, NN_STATUS_FAILED);
   // EPI_EPW: the modes outside the conv image (the network's low-mode window)
   // take the quadratic extrapolation alone, spread over every CTA
   if (EPI == EPI_EPW && !failed && !skip) {
