@@ -253,7 +253,8 @@ __global__ void __launch_bounds__(256) k_xinv4(const __grid_constant__ X4Job job
     const int gi = (int)blockIdx.x >= pairs ? 1 : 0;
     const int y0 = 2 * ((int)blockIdx.x - gi * pairs);
     const float4* src = job.src[gi] + y0;
-    // node (kx, row r) -> lines 4 r .. 4 r + 3; every load before the stores
+    // node (kx, row r) -> lines 4 r .. 4 r + 3; every load before the stores (5 a
+    // thread are the 1026 of a 512-point line; longer lines take rounds of 4)
     constexpr int U = P == 8 ? 5 : 4;
     const int total = 2 * (n + 1);
     for (int b0 = threadIdx.x; b0 < total; b0 += U * 256) {
@@ -312,9 +313,16 @@ __global__ void __launch_bounds__(256) k_xinv4(const __grid_constant__ X4Job job
 // 512 (9.4 MB in and out); the planar form took 13.3, the staging through
 // shared memory being the price of the densities' vector reductions (amjdp
 // 2.3 us less per pass).
+// Registers per thread (resident CTAs) by line length: a cap pays where it
+// makes room for one CTA more, 64 at 512 points (4 CTAs: 14.2 us, uncapped
+// 14.4) and 80 at 1024 points (3 CTAs: 34.6 us with 36 bytes spilled, uncapped
+// 35.6).  48 at 512 points (5 CTAs) would suit 64 concurrent instances (7.07 ->
+// 7.15e9 particle-slices/s) but not one (4.48 -> 4.33e9).  Shorter lines take
+// what they need (0): a cap makes the compiler spend registers up to it.  2048
+// points leave one CTA per SM with any cap that does not spill heavily.
 template <int P>
-__global__ void __launch_bounds__(256, P == 8 ? 4 : P == 16 ? 3 : 0) k_xfwd8(const __grid_constant__ X8Job job, GridDims g,
-                                               LineTables tx, const DevStatus* st) {
+__global__ void __launch_bounds__(256, P == 8 ? 4 : P == 16 ? 3 : 0)
+    k_xfwd8(const __grid_constant__ X8Job job, GridDims g, LineTables tx, const DevStatus* st) {
   extern __shared__ __align__(16) float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = g.nx, pitch = line_pitch(n);

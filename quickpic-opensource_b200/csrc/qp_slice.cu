@@ -31,9 +31,12 @@ namespace {
 // one scratch line per warp (line_transform's shared-memory form).
 __host__ __device__ int col_pitch(int n) { return n + 4; }
 
+// Registers capped where that makes room for one CTA more per SM: 64 at 512
+// points (4 CTAs: 16.9 us, uncapped 17.4), 80 at 1024 points (3: 49.8 against
+// 50.3); other lengths take what they need (0).
 template <int P>
-__global__ void __launch_bounds__(256, P == 8 ? 4 : P == 16 ? 3 : 0) k_slice_a(SliceA a, GridDims g, KCoef K, LineTables ty,
-                                                 const DevStatus* st) {
+__global__ void __launch_bounds__(256, P == 8 ? 4 : P == 16 ? 3 : 0)
+    k_slice_a(SliceA a, GridDims g, KCoef K, LineTables ty, const DevStatus* st) {
   extern __shared__ __align__(16) float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = g.ny, pitch = col_pitch(n);
@@ -144,8 +147,8 @@ __global__ void __launch_bounds__(256, P == 8 ? 4 : P == 16 ? 3 : 0) k_slice_a(S
 // CTAs make the launch 100 us instead of 88).  No cap elsewhere (0): a cap makes
 // the compiler spend registers up to it, which slowed the short lines.
 template <int P>
-__global__ void __launch_bounds__(288, P == 16 ? 3 : 0) k_slice_b(SliceB b, GridDims g, KCoef K, LineTables ty,
-                                                 DevStatus* st) {
+__global__ void __launch_bounds__(288, P == 16 ? 3 : 0)
+    k_slice_b(SliceB b, GridDims g, KCoef K, LineTables ty, DevStatus* st) {
   extern __shared__ __align__(16) float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = g.ny, pitch = col_pitch(n);
