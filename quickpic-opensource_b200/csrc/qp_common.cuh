@@ -129,8 +129,9 @@ enum { QP_OK = 0, QP_OVERFLOW = 1 };
 // grid_dep_sync() before it touches device data: griddepcontrol.wait returns
 // once the preceding grid has completed and its writes are visible (at once
 // for a kernel launched without the attribute), and launch_dependents then
-// allows the next grid to be scheduled behind this one.  Data that no kernel
-// writes (the twiddle tables) may be read before the wait.
+// allows the next grid to be scheduled behind this one (a kernel that leaves it
+// out lets the next grid in when it ends).  Data that no kernel writes (the
+// twiddle tables) may be read before the wait.
 __device__ __forceinline__ void grid_dep_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

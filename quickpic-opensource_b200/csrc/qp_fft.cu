@@ -357,8 +357,16 @@ __global__ void __launch_bounds__(256, P == 8 ? 4 : P == 16 ? 3 : 0)
 // inverse is that of the forward transform).  One warp per column and
 // component: a launch is one latency chain (load, transform, store), so the
 // components of a vector run side by side instead of one after another.
+// 1024-point lines: registers capped at 80 (3 CTAs per SM); left alone the
+// compiler takes 64, and a transform pair of one component at 1024 x 1024 takes
+// 40.4 us instead of 24.9 (three components 62.9, 52.2).  Plain transforms of up
+// to 256 points do not let the next grid in early: with several components they
+// are more CTAs than SMs, and the x pass that follows has the long chains (1024
+// x 64, two components: 24.9 -> 19.3 us a pair).  Longer ones gain from it (512 x
+// 512, three components: 22.5 us against 23.5), and so does the smoothing of a
+// step of two species (3.34 ms against 3.41 for 32 slices at 256 x 256).
 template <int P, bool SMOOTH>
-__global__ void __launch_bounds__(256) k_ycol(const __grid_constant__ YJob job, GridDims g,
+__global__ void __launch_bounds__(256, P == 16 ? 3 : 0) k_ycol(const __grid_constant__ YJob job, GridDims g,
                                               KCoef K, LineTables ty, const DevStatus* st) {
   extern __shared__ __align__(16) float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -367,7 +375,8 @@ __global__ void __launch_bounds__(256) k_ycol(const __grid_constant__ YJob job, 
   float* S = smem + (8 + warp) * pitch;
   float* T = smem + line_count(g.indy) * pitch;
   if (P > 0) stage_lane_table(T, ty);  // constant tables: staged before the wait
-  grid_dep_sync();
+  grid_dep_wait();
+  if (SMOOTH || P == 0 || P >= 8) grid_dep_launch();
   if (st && st->error) return;
   if (P > 0) __syncthreads();
   const int kx = blockIdx.x * 8 + warp;
