@@ -44,6 +44,7 @@ struct GatherPlanes {
   int combine;       // 1: the push uses -fxy + (by, -bx), the final slice force
   int ext;           // amjdp only: form p6, p7 from psi first (extpsi); node-major fields
   int pass;          // amjdp only: predictor-corrector pass (pass_skipped), 0 = none
+  int hold;          // amjdp only: 1 = the next grid starts at this one's end
   float* zero_q;     // push only, optional: clear the charge-plane nodes this tile
                      // owns (k_insert then deposits the next slice's charge)
   // push with combine only, optional: the slice's fields go to these planes --
@@ -77,8 +78,9 @@ void launch_push(int mode, const PartBuf& A, const PartBuf& B, const Inbox& ib,
 // A = the particles of P0 (rest of A's slots zero) with charge q P0's times qm
 void launch_renew(const PartBuf& P0, const PartBuf& A, int ntiles, float qm, cudaStream_t s);
 // deposit_q (optional): after the re-bin, deposit the charge of every
-// particle of the tile into deposit_q (zero on entry), as k_deposit_rho does
+// particle of the tile into deposit_q (zero on entry), as k_deposit_rho does;
+// hold = 1: the next grid starts at this one's end
 void launch_insert(const PartBuf& B, const Inbox& ib, const TileGeom& tg, DevStatus* st,
-                   cudaStream_t s, float* deposit_q = nullptr);
+                   cudaStream_t s, float* deposit_q = nullptr, int hold = 0);
 
 }  // namespace qp
