@@ -243,7 +243,8 @@ __global__ void __launch_bounds__(256) k_xinv4(const __grid_constant__ X4Job job
   const int n = g.nx, pitch = line_pitch(n);
   float* T = smem + line_count(g.indx) * pitch;
   if (P > 0) stage_lane_table(T, tx);  // constant tables: staged before the wait
-  grid_dep_sync();
+  grid_dep_wait();
+  if (!job.hold) grid_dep_launch();
   if (st && st->error) return;
   if (pass_skipped(st, job.pass)) return;
   float* L = smem + warp * pitch;

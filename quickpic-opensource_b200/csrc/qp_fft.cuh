@@ -66,6 +66,7 @@ struct X4Job {
   float* zero[16];  // planes that this launch clears
   int nzero;
   int pass;  // predictor-corrector pass of the launch (pass_skipped), 0 = none
+  int hold;  // 1: the next grid starts at this one's end
 };
 void launch_xinv4(const X4Job& job, const GridDims& g, const LineTables& tx, const DevStatus* st,
                   cudaStream_t s);
